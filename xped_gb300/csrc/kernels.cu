@@ -893,85 +893,149 @@ __device__ __forceinline__ double warp_sum(double v) {
 // back to the first value of the first sector when nothing survives, and
 // count kept values per sector.  One CTA; n is the number of singular values
 // of one tensor (thousands at most).
+//
+// Bound by latency (one CTA, a few block barriers).  Everything lives in shared memory up to
+// kTruncSmem values (a global workspace beyond), the ranks count 64-bit integer keys that order like
+// the doubles (a double comparison occupies the narrow FP64 pipe), and the tie groups and the kept list
+// come from block-wide prefix scans.  Measured on GB300 for one tSVD: 45 us with 324 values and 2.0 ms
+// with 1414 when one thread walked the sorted list through global memory; 22 us and 123 us now.
 constexpr double kTieRtol = 1.0e-12;
+constexpr int kTruncThreads = 1024;
+constexpr int64_t kTruncSmem = 8192;  // values held in shared memory: 24 bytes each (196,608 of 227 KB)
 
-__global__ void __launch_bounds__(1024) truncate_kernel(int n_sectors, const int64_t* __restrict__ s_begin,
-                                                        const int32_t* __restrict__ deg, const double* __restrict__ s,
-                                                        int64_t total, int64_t max_keep, double eps, int preserve,
-                                                        int32_t* __restrict__ keep, double* __restrict__ out2,
-                                                        int64_t* __restrict__ ws) {
-  __shared__ double red_w[32], red_e[32];
-  int64_t* exact = ws;                 // exact[r] = index with exact rank r
-  int64_t* gstart = ws + total;        // group start position for each exact position
-  int64_t* order = ws + 2 * total;     // order[f] = index at final position f
-  int64_t* flag = ws + 3 * total;      // flag[i] = 1 kept, 0 dropped; fpos stored in gstart reuse below
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int g = tid; g < n_sectors; g += blockDim.x) keep[g] = 0;
-  // exact ranks under a total order (NaN ranks below every number, ties by
-  // index), so that `exact` is a permutation whatever the values are
-  auto key = [](double v) { return v == v ? v : -INFINITY; };
-  for (int64_t i = tid; i < total; i += blockDim.x) {
-    const double si = key(s[i]);
-    int64_t r = 0;
-    for (int64_t j = 0; j < total; ++j) {
-      const double sj = key(s[j]);
-      r += (sj > si) || (sj == si && j < i);
+// A double as an unsigned integer of the same order; NaN lies below every number, -0.0 equals 0.0.
+__device__ __forceinline__ unsigned long long order_key(double v) {
+  if (v != v) return 0ull;
+  const long long b = __double_as_longlong(v);
+  if (b == (long long)0x8000000000000000ull) return 0x8000000000000000ull;
+  return b < 0 ? ~(unsigned long long)b : (unsigned long long)b | 0x8000000000000000ull;
+}
+
+// Inclusive scans over the CTA's threads (sum / max); `part` holds one int per warp.
+template <bool kMax>
+__device__ __forceinline__ int block_scan(int v, int* part) {
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const int u = __shfl_up_sync(0xffffffffu, v, o);
+    if (lane >= o) v = kMax ? max(v, u) : v + u;
+  }
+  __syncthreads();  // part is free again (an earlier scan's readers are done)
+  if (lane == 31) part[warp] = v;
+  __syncthreads();
+  if (warp == 0) {
+    int w = part[lane];
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, w, o);
+      if (lane >= o) w = kMax ? max(w, u) : w + u;
     }
-    exact[r] = i;
+    part[lane] = w;
+  }
+  __syncthreads();
+  if (warp > 0) v = kMax ? max(v, part[warp - 1]) : v + part[warp - 1];
+  return v;
+}
+
+// `ws`: 3 * total 8-byte words, used when `in_smem` is 0.
+__global__ void __launch_bounds__(kTruncThreads) truncate_kernel(int n_sectors, const int64_t* __restrict__ s_begin,
+                                                                 const int32_t* __restrict__ deg,
+                                                                 const double* __restrict__ s, int total,
+                                                                 int64_t max_keep, double eps, int preserve,
+                                                                 int32_t* __restrict__ keep, double* __restrict__ out2,
+                                                                 unsigned long long* __restrict__ ws, int in_smem) {
+  extern __shared__ unsigned long long trunc_sm[];
+  __shared__ double red_w[32], red_e[32];
+  __shared__ int part[32];
+  __shared__ int kept_n;
+  unsigned long long* base = in_smem ? trunc_sm : ws;
+  unsigned long long* key = base;                     // key[i]: order of value i
+  int* exact = reinterpret_cast<int*>(base + total);  // exact[r] = index with exact rank r; later the kept list
+  int* gstart = exact + total;                        // first position of the tie group of each exact position
+  int* order = gstart + total;                        // order[f] = index at final position f
+  int* flag = order + total;                          // flag[i]: bit 0 kept, bit 1 counts as truncated weight
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, nt = kTruncThreads;
+  for (int g = tid; g < n_sectors; g += nt) keep[g] = 0;
+  for (int i = tid; i < total; i += nt) {
+    key[i] = order_key(s[i]);
     flag[i] = 0;
   }
   __syncthreads();
-  if (tid == 0) {
-    int64_t start = 0;
-    for (int64_t p = 0; p < total; ++p) {
-      if (p > 0) {
-        const double prev = s[exact[p - 1]], cur = s[exact[p]];
-        if (prev - cur > kTieRtol * prev) start = p;
-      }
-      gstart[p] = start;
+  // exact ranks under a total order (ties by index), so that `exact` is a permutation whatever the values are
+  for (int i = tid; i < total; i += nt) {
+    const unsigned long long ki = key[i];
+    int r = 0;
+#pragma unroll 8
+    for (int j = 0; j < total; ++j) {
+      const unsigned long long kj = key[j];
+      r += (kj > ki) || (kj == ki && j < i);
     }
+    exact[r] = i;
   }
   __syncthreads();
-  for (int64_t p = tid; p < total; p += blockDim.x) {
-    const int64_t i = exact[p], g0 = gstart[p];
-    int64_t f = g0;
-    for (int64_t q = g0; q < total && gstart[q] == g0; ++q) f += (exact[q] < i);
+  // tie groups: a value more than kTieRtol below its predecessor opens one (running maximum of the openings)
+  for (int p0 = 0, carry = 0; p0 < total; p0 += nt) {
+    const int p = p0 + tid;
+    int open = 0;
+    if (p < total && p > 0) {
+      const double prev = s[exact[p - 1]], cur = s[exact[p]];
+      if (prev - cur > kTieRtol * prev) open = p;
+    }
+    const int g = max(carry, block_scan<true>(open, part));
+    if (p < total) gstart[p] = g;
+    carry = max(carry, part[31]);
+  }
+  __syncthreads();
+  for (int p = tid; p < total; p += nt) {
+    const int i = exact[p], g0 = gstart[p];
+    int f = g0;
+    for (int q = g0; q < total && gstart[q] == g0; ++q) f += (exact[q] < i);
     order[f] = i;
   }
   __syncthreads();
+  const int lim = total < max_keep ? total : int(max_keep);
+  // kept list in final order, stored compactly at the front of `exact`
+  int nk = 0;
+  for (int f0 = 0; f0 < lim; f0 += nt) {
+    const int f = f0 + tid;
+    const int i = f < lim ? order[f] : 0;
+    const int on = f < lim && !(eps > 0.0 && s[i] < eps);
+    const int at = nk + block_scan<false>(on, part);
+    if (on) exact[at - 1] = i;
+    nk += part[31];
+  }
+  __syncthreads();
   if (tid == 0) {
-    const int64_t lim = total < max_keep ? total : max_keep;
-    // kept list in final order, stored compactly at the front of `exact`
-    int64_t nk = 0;
-    for (int64_t f = 0; f < lim; ++f) {
-      const int64_t i = order[f];
-      if (eps > 0.0 && s[i] < eps) continue;
-      exact[nk++] = i;
-    }
     if (preserve) {
-      int64_t end = -1;
-      for (int64_t k = nk - 1; k > 0; --k) {
+      int end = -1;
+      for (int k = nk - 1; k > 0; --k) {
         const double a = s[exact[k - 1]], b = s[exact[k]];
         if (2.0 * (a - b) / (a + b) > 0.1) { end = k; break; }
       }
       if (end != -1) nk = end;
     }
     if (nk == 0) { exact[0] = 0; nk = 1; }  // first entry: first value of the first sector
-    for (int64_t k = 0; k < nk; ++k) flag[exact[k]] = 1;
-    // positions >= max_keep contribute to the truncated weight
-    for (int64_t f = lim; f < total; ++f) flag[order[f]] |= 2;
+    kept_n = nk;
   }
   __syncthreads();
+  nk = kept_n;
+  for (int k = tid; k < nk; k += nt) flag[exact[k]] = 1;
+  __syncthreads();
+  // positions >= max_keep contribute to the truncated weight
+  for (int f = max(lim, 0) + tid; f < total; f += nt) flag[order[f]] |= 2;
+  __syncthreads();
   double wsum = 0.0, esum = 0.0;
-  for (int64_t i = tid; i < total; i += blockDim.x) {
+  for (int i = tid; i < total; i += nt) {
+    const int fl = flag[i];
+    if (fl == 0) continue;
     int lo = 0, hi = n_sectors - 1;
     while (lo < hi) {
       const int mid = (lo + hi + 1) >> 1;
       if (s_begin[mid] <= i) lo = mid; else hi = mid - 1;
     }
     const double v = s[i];
-    if (flag[i] & 2) wsum += deg[lo] * v * v;
-    if (flag[i] & 1) {
+    if (fl & 2) wsum += deg[lo] * v * v;
+    if (fl & 1) {
       atomicAdd(&keep[lo], 1);
       esum += -deg[lo] * v * v * log(v * v);
     }
@@ -982,7 +1046,7 @@ __global__ void __launch_bounds__(1024) truncate_kernel(int n_sectors, const int
   __syncthreads();
   if (tid == 0) {
     double a = 0, b = 0;
-    for (int w = 0; w < int(blockDim.x + 31) / 32; ++w) { a += red_w[w]; b += red_e[w]; }
+    for (int w = 0; w < nt / 32; ++w) { a += red_w[w]; b += red_e[w]; }
     out2[0] = a;
     out2[1] = b;
   }
@@ -990,10 +1054,18 @@ __global__ void __launch_bounds__(1024) truncate_kernel(int n_sectors, const int
 
 void launch_truncate(int n_sectors, const int64_t* d_s_begin, const int32_t* d_deg, const double* s, int64_t total,
                      int64_t max_keep, double eps, int preserve, int32_t* keep, double* out2, cudaStream_t st) {
-  int64_t* ws = static_cast<int64_t*>(dev_alloc(sizeof(int64_t) * 4 * std::max<int64_t>(total, 1)));
-  truncate_kernel<<<1, 1024, 0, st>>>(n_sectors, d_s_begin, d_deg, s, total, max_keep, eps, preserve, keep, out2, ws);
+  if (total > INT32_MAX / 4) throw std::runtime_error("truncate: too many singular values");
+  static std::once_flag attr;
+  std::call_once(attr, [] {
+    cudaFuncSetAttribute(truncate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTruncSmem) * 24);
+  });
+  const bool in_smem = total <= kTruncSmem;
+  const size_t bytes = size_t(std::max<int64_t>(total, 1)) * 24;
+  auto* ws = in_smem ? nullptr : static_cast<unsigned long long*>(dev_alloc(bytes));
+  truncate_kernel<<<1, kTruncThreads, in_smem ? bytes : 0, st>>>(n_sectors, d_s_begin, d_deg, s, int(total), max_keep,
+                                                                 eps, preserve, keep, out2, ws, in_smem ? 1 : 0);
   count_launch();
-  dev_free(ws);
+  if (ws) dev_free(ws);
 }
 
 // ======================================================================= QR
