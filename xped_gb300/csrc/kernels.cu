@@ -897,7 +897,7 @@ __device__ __forceinline__ double warp_sum(double v) {
 // Bound by latency (one CTA, a few block barriers).  Everything lives in shared memory up to
 // kTruncSmem values (a global workspace beyond), the ranks count 64-bit integer keys that order like
 // the doubles (a double comparison occupies the narrow FP64 pipe), and the tie groups and the kept list
-// come from block-wide prefix scans.  Measured on GB300 for one tSVD: 45 us with 324 values and 2.0 ms
+// come from block-wide prefix scans.  Measured on GB300 for one tSVD: 178 us with 324 values and 2.0 ms
 // with 1414 when one thread walked the sorted list through global memory; 22 us and 123 us now.
 constexpr double kTieRtol = 1.0e-12;
 constexpr int kTruncThreads = 1024;
@@ -1559,7 +1559,7 @@ int xgb_batched_svd(int n, const xgb_svd_desc* descs, const double* A, double* U
   if (n == 0) return XGB_OK;
   auto* dd = upload(descs, size_t(n), s);
   auto* dof = upload(off.data(), off.size(), s);
-  launch_svd(dd, descs, dof, n, maxk, A, U, S, Vt, static_cast<double*>(work), s);
+  launch_svd(dd, descs, dof, n, A, U, S, Vt, static_cast<double*>(work), s);
   dev_free(dd);
   dev_free(dof);
   return check_cuda(cudaGetLastError(), "svd launch");

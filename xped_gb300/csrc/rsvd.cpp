@@ -199,13 +199,12 @@ class OzProducts {
 void batched_svd(const std::vector<xgb_svd_desc>& d, const double* A, double* U, double* S, double* Vt, cudaStream_t s) {
   if (d.empty()) return;
   std::vector<int64_t> woff(d.size());
-  int64_t wt = 0, maxk = 0;
+  int64_t wt = 0;
   double flops = 0;
   for (size_t i = 0; i < d.size(); ++i) {
     woff[i] = wt;
     wt += int64_t(svd_work_elems(d[i].m, d[i].n));
     const double mm = double(std::max(d[i].m, d[i].n)), nn = double(std::min(d[i].m, d[i].n));
-    maxk = std::max(maxk, std::min(d[i].m, d[i].n));
     flops += 6 * mm * nn * nn + 20 * nn * nn * nn;  // thin R-SVD count (U m x n, S, V)
   }
   Staging st;
@@ -213,7 +212,7 @@ void batched_svd(const std::vector<xgb_svd_desc>& d, const double* A, double* U,
   st.upload(s);
   double* W = alloc_d(wt);
   prof_begin(K_SVD, s);
-  launch_svd(st.at<xgb_svd_desc>(od), d.data(), st.at<int64_t>(ow), int(d.size()), maxk, A, U, S, Vt, W, s);
+  launch_svd(st.at<xgb_svd_desc>(od), d.data(), st.at<int64_t>(ow), int(d.size()), A, U, S, Vt, W, s);
   prof_end(K_SVD, s, flops);
   dev_free(W);
 }

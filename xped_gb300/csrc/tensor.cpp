@@ -1099,8 +1099,7 @@ SVDResult tsvd(const Tensor& t0, int64_t max_keep, double eps_svd, bool preserve
   sp.V = static_cast<double*>(dev_alloc(sizeof(double) * std::max<int64_t>(plan->v_total, 1)));
   double* W = static_cast<double*>(dev_alloc(sizeof(double) * std::max<int64_t>(plan->work_total, 1)));
   prof_begin(K_SVD, st);
-  launch_svd(plan->d_descs, plan->h_descs.data(), plan->d_work_off, plan->n, plan->maxk, t.data(), sp.U, sp.S, sp.V, W,
-             st);
+  launch_svd(plan->d_descs, plan->h_descs.data(), plan->d_work_off, plan->n, t.data(), sp.U, sp.S, sp.V, W, st);
   prof_end(K_SVD, st, plan->lapack_flops);
   dev_free(W);
   sp.k = plan->kfull;
