@@ -1068,99 +1068,6 @@ void launch_truncate(int n_sectors, const int64_t* d_s_begin, const int32_t* d_d
   if (ws) dev_free(ws);
 }
 
-// ======================================================================= QR
-// Batched Householder QR in FP64 with LAPACK's dlarfg sign convention
-// (beta = -sign(alpha)*||x||), so Q and R agree with dgeqrf/dorgqr.
-__global__ void __launch_bounds__(256) qr_kernel(const xgb_qr_desc* __restrict__ descs, const int64_t* __restrict__ work_off,
-                                                 const double* __restrict__ A, double* __restrict__ Q,
-                                                 double* __restrict__ R, double* __restrict__ work) {
-  const xgb_qr_desc d = descs[blockIdx.x];
-  const int64_t m = d.m, n = d.n, kk = m < n ? m : n;
-  double* W = work + work_off[blockIdx.x];  // m x n working copy (Householder vectors below diagonal)
-  double* tau = W + m * n;                  // kk
-  double* Qw = tau + kk;                    // m x m accumulation
-  __shared__ double red[8];
-  __shared__ double bcast[2];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int64_t e = tid; e < m * n; e += 256) W[e] = A[d.a_off + e];
-  __syncthreads();
-  auto block_sum = [&](double v) {
-    v = warp_sum(v);
-    if (lane == 0) red[warp] = v;
-    __syncthreads();
-    double r = 0;
-    if (tid == 0) { for (int w = 0; w < 8; ++w) r += red[w]; bcast[0] = r; }
-    __syncthreads();
-    r = bcast[0];
-    __syncthreads();
-    return r;
-  };
-  for (int64_t j = 0; j < kk; ++j) {
-    double* col = W + j * m;
-    double part = 0;
-    for (int64_t i = j + 1 + tid; i < m; i += 256) part = fma(col[i], col[i], part);
-    double xnorm2 = block_sum(part);
-    double alpha = col[j];
-    double t = 0.0, beta = alpha;
-    if (xnorm2 > 0.0) {
-      beta = -copysign(sqrt(alpha * alpha + xnorm2), alpha);
-      t = (beta - alpha) / beta;
-      double scal = 1.0 / (alpha - beta);
-      for (int64_t i = j + 1 + tid; i < m; i += 256) col[i] *= scal;
-    }
-    __syncthreads();
-    if (tid == 0) { tau[j] = t; col[j] = beta; }
-    __syncthreads();
-    if (t != 0.0) {
-      for (int64_t c = j + 1 + warp; c < n; c += 8) {
-        double* cc = W + c * m;
-        double w = (lane == 0) ? cc[j] : 0.0;
-        for (int64_t i = j + 1 + lane; i < m; i += 32) w = fma(col[i], cc[i], w);
-        w = warp_sum(w) * t;
-        if (lane == 0) cc[j] -= w;
-        for (int64_t i = j + 1 + lane; i < m; i += 32) cc[i] -= w * col[i];
-      }
-    }
-    __syncthreads();
-  }
-  // R (r_rows x n): upper triangle of W in the first kk rows
-  for (int64_t e = tid; e < d.r_rows * n; e += 256) {
-    int64_t i = e % d.r_rows, c = e / d.r_rows;
-    R[d.r_off + e] = (i < kk && i <= c) ? W[i + c * m] : 0.0;
-  }
-  // Q = H_0 H_1 ... H_{kk-1} applied to the first q_cols columns of I (backward accumulation)
-  const int64_t qc = d.q_cols < m ? d.q_cols : m;
-  for (int64_t e = tid; e < m * qc; e += 256) Qw[e] = ((e % m) == (e / m)) ? 1.0 : 0.0;
-  __syncthreads();
-  for (int64_t j = kk - 1; j >= 0; --j) {
-    const double t = tau[j];
-    if (t == 0.0) continue;
-    const double* v = W + j * m;
-    for (int64_t c = warp; c < qc; c += 8) {
-      double* cc = Qw + c * m;
-      double w = (lane == 0) ? cc[j] : 0.0;
-      for (int64_t i = j + 1 + lane; i < m; i += 32) w = fma(v[i], cc[i], w);
-      w = warp_sum(w) * t;
-      if (lane == 0) cc[j] -= w;
-      for (int64_t i = j + 1 + lane; i < m; i += 32) cc[i] -= w * v[i];
-    }
-    __syncthreads();
-  }
-  for (int64_t e = tid; e < m * d.q_cols; e += 256) {
-    int64_t c = e / m;
-    Q[d.q_off + e] = (c < qc && c < kk) ? Qw[e] : 0.0;
-  }
-}
-
-size_t qr_work_elems(int64_t m, int64_t n) { return size_t(m * n + std::min(m, n) + m * m); }
-
-void launch_qr(const xgb_qr_desc* d_descs, const int64_t* d_work_off, int n, const double* A, double* Q, double* R,
-               double* work, cudaStream_t s) {
-  if (n <= 0) return;
-  qr_kernel<<<n, 256, 0, s>>>(d_descs, d_work_off, A, Q, R, work);
-  count_launch();
-}
-
 // ======================================================================= elementwise
 __global__ void absmax_kernel(const double* __restrict__ x, int64_t n, unsigned long long* __restrict__ out) {
   double m = 0.0;
@@ -1603,7 +1510,7 @@ int xgb_batched_qr(int n, const xgb_qr_desc* descs, const double* A, double* Q, 
   if (n == 0) return XGB_OK;
   auto* dd = upload(descs, size_t(n), s);
   auto* dof = upload(off.data(), off.size(), s);
-  launch_qr(dd, dof, n, A, Q, R, static_cast<double*>(work), s);
+  launch_qr(dd, descs, dof, n, A, Q, R, static_cast<double*>(work), s);
   dev_free(dd);
   dev_free(dof);
   return check_cuda(cudaGetLastError(), "qr launch");

@@ -98,8 +98,8 @@ void launch_svd(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, const 
                 const double* A, double* U, double* S, double* Vt, double* work, cudaStream_t s);
 void launch_truncate(int n_sectors, const int64_t* d_s_begin, const int32_t* d_deg, const double* sv, int64_t total,
                      int64_t max_keep, double eps, int preserve, int32_t* keep, double* out2, cudaStream_t s);
-void launch_qr(const xgb_qr_desc* d_descs, const int64_t* d_work_off, int n, const double* A, double* Q, double* R,
-               double* work, cudaStream_t s);
+void launch_qr(const xgb_qr_desc* d_descs, const xgb_qr_desc* h_descs, const int64_t* d_work_off, int n,
+               const double* A, double* Q, double* R, double* work, cudaStream_t s);
 void launch_absmax(const double* x, int64_t n, double* out, cudaStream_t s);
 void launch_scale_by_inv(double* x, int64_t n, const double* m, cudaStream_t s);
 void launch_scale(double* x, int64_t n, double alpha, cudaStream_t s);

@@ -1143,7 +1143,7 @@ std::pair<Tensor, Tensor> tqr(const Tensor& t0) {
     double* W = static_cast<double*>(dev_alloc(sizeof(double) * std::max<int64_t>(wt, 1)));
     cuda_ok(cudaMemcpyAsync(dd, descs.data(), sizeof(xgb_qr_desc) * descs.size(), cudaMemcpyHostToDevice, st), "h2d");
     cuda_ok(cudaMemcpyAsync(dw, woff.data(), sizeof(int64_t) * woff.size(), cudaMemcpyHostToDevice, st), "h2d");
-    launch_qr(dd, dw, int(descs.size()), t.data(), Q.data(), R.data(), W, st);
+    launch_qr(dd, descs.data(), dw, int(descs.size()), t.data(), Q.data(), R.data(), W, st);
     dev_free(dd);
     dev_free(dw);
     dev_free(W);
