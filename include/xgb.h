@@ -162,6 +162,11 @@ typedef struct xgb_perm_contrib {
 int xgb_permute(int n_tasks, const xgb_perm_task* tasks, int n_contrib, const xgb_perm_contrib* contribs,
                 const double* src, double* dst, void* stream);
 
+/* The same launch plan walked on the host by the kernel's index arithmetic, for
+   host buffers (no device needed); *transposed: the form that the plan takes. */
+int xgb_permute_walk_host(int n_tasks, const xgb_perm_task* tasks, int n_contrib, const xgb_perm_contrib* contribs,
+                          const double* src, double* dst, int* transposed);
+
 /* -------------------------------------------------------------- batched SVD */
 typedef struct xgb_svd_desc {
   int64_t m, n;           /* block is m x n, k = min(m, n) singular triplets */

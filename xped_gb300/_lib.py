@@ -65,6 +65,8 @@ PROTOS = [
     ("xgb_launch_count", C.c_int64, []),
     ("xgb_grouped_gemm", C.c_int, [C.c_int, C.c_int, C.POINTER(GemmDesc), P, P, P, C.c_double, C.c_double, P]),
     ("xgb_permute", C.c_int, [C.c_int, C.POINTER(PermTask), C.c_int, C.POINTER(PermContrib), P, P, P]),
+    ("xgb_permute_walk_host", C.c_int, [C.c_int, C.POINTER(PermTask), C.c_int, C.POINTER(PermContrib), P, P,
+                                        C.POINTER(C.c_int)]),
     ("xgb_svd_workspace_bytes", C.c_size_t, [C.c_int, C.POINTER(SvdDesc)]),
     ("xgb_batched_svd", C.c_int, [C.c_int, C.POINTER(SvdDesc), P, P, P, P, P, P]),
     ("xgb_truncate", C.c_int, [C.c_int, i64p, i32p, P, C.c_int64, C.c_double, C.c_int, P, P, P]),

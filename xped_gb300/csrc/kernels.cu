@@ -469,413 +469,6 @@ int choose_gemm_tile(const xgb_gemm_desc* descs, int n) {
   return 16;
 }
 
-// ======================================================================= permute
-// Gather-permute with recoupling coefficients, one ROW at a time: a row is the run of a task's
-// output sub-block along output leg 0 (all other leg indices fixed), which is contiguous in the
-// output (leg 0 fastest) and, for the permutations that keep the block's leading leg in front,
-// contiguous in the source too.  A group of G threads (G a power of two up to a warp, chosen on
-// the host from the rows' typical length) takes a chunk of kRowsPerChunk consecutive rows: the
-// first row's multi-index is decoded once (32-bit division), the following rows step it like an
-// odometer (leg 1 fastest, adding the legs' strides), and the lanes walk each row with unit stride,
-// so a warp's loads and stores cover whole 32-byte sectors.  Four rows' loads are issued before
-// their stores.  Tasks with several contributions (SU(2) recoupling) accumulate them in a fixed
-// order.
-constexpr int kRowsPerChunk = 8;
-
-// Row cursor with the current task's extents, strides and coefficient held in registers (loaded
-// once per task, not per row): SI is int32_t when every stride of the plan fits (the host checks),
-// int64_t otherwise.  All per-leg arrays are indexed only inside fully unrolled loops.
-template <typename SI>
-struct RowCursor {
-  int ti = -1;          // task
-  int64_t row_end = 0;  // first row past the task
-  int rank = 0, d0 = 1, n_contrib = 1, contrib0 = 0;
-  double coeff = 0.0;
-  int dims[XGB_MAX_LEGS];
-  SI dstr[XGB_MAX_LEGS], sstr[XGB_MAX_LEGS];  // sstr: strides of the single contribution
-  int idx[XGB_MAX_LEGS];                      // multi-index of legs 1..rank-1
-  int64_t dofs = 0, sofs = 0;
-};
-
-template <typename SI>
-__device__ __forceinline__ void cursor_seek(RowCursor<SI>& c, const xgb_perm_task* __restrict__ tasks,
-                                            const int64_t* __restrict__ row_start, int n_tasks,
-                                            const xgb_perm_contrib* __restrict__ contribs, int64_t r) {
-  int ti = c.ti >= 0 ? c.ti : 0;
-  if (!(r >= row_start[ti] && r < row_start[ti + 1])) {
-    int lo = 0, hi = n_tasks - 1;
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) >> 1;
-      if (row_start[mid] <= r) lo = mid; else hi = mid - 1;
-    }
-    ti = lo;
-  }
-  const xgb_perm_task& t = tasks[ti];
-  if (ti != c.ti) {  // task fields into registers
-    c.ti = ti;
-    c.row_end = row_start[ti + 1];
-    c.rank = t.rank;
-    c.d0 = t.rank > 0 ? t.dims[0] : 1;
-    c.n_contrib = t.n_contrib;
-    c.contrib0 = t.contrib0;
-    const bool single = t.n_contrib == 1;
-    c.coeff = single ? contribs[t.contrib0].coeff : 0.0;
-#pragma unroll
-    for (int k = 0; k < XGB_MAX_LEGS; ++k) {
-      const bool on = k < t.rank;
-      c.dims[k] = on ? t.dims[k] : 1;
-      c.dstr[k] = on ? SI(t.dst_stride[k]) : SI(0);
-      c.sstr[k] = (on && single) ? SI(contribs[t.contrib0].src_stride[k]) : SI(0);
-    }
-  }
-  int64_t rem = r - row_start[ti];
-  c.dofs = t.dst_base;
-  c.sofs = c.n_contrib == 1 ? contribs[c.contrib0].src_base : 0;
-#pragma unroll
-  for (int k = 1; k < XGB_MAX_LEGS; ++k) {
-    c.idx[k] = 0;
-    if (k < c.rank) {
-      const int dk = c.dims[k];
-      int ik;
-      if (rem < (int64_t(1) << 31)) {  // 32-bit division for the common case
-        const uint32_t r32 = uint32_t(rem), q = r32 / uint32_t(dk);
-        ik = int(r32 - q * uint32_t(dk));
-        rem = q;
-      } else {
-        const int64_t q = rem / dk;
-        ik = int(rem - q * dk);
-        rem = q;
-      }
-      c.idx[k] = ik;
-      c.dofs += int64_t(ik) * c.dstr[k];
-      c.sofs += int64_t(ik) * c.sstr[k];
-    }
-  }
-}
-
-// next row of the same task: leg 1 fastest, carrying into the higher legs
-template <typename SI>
-__device__ __forceinline__ void cursor_step(RowCursor<SI>& c) {
-#pragma unroll
-  for (int k = 1; k < XGB_MAX_LEGS; ++k) {
-    if (k >= c.rank) return;
-    c.dofs += c.dstr[k];
-    c.sofs += c.sstr[k];
-    if (++c.idx[k] < c.dims[k]) return;
-    c.idx[k] = 0;
-    c.dofs -= int64_t(c.dims[k]) * c.dstr[k];
-    c.sofs -= int64_t(c.dims[k]) * c.sstr[k];
-  }
-}
-
-template <int G, typename SI>
-__global__ void __launch_bounds__(256) permute_rows_kernel(const xgb_perm_task* __restrict__ tasks,
-                                                           const int64_t* __restrict__ row_start, int n_tasks,
-                                                           int64_t total_rows, const xgb_perm_contrib* __restrict__ contribs,
-                                                           const double* __restrict__ src, double* __restrict__ dst) {
-  constexpr int U = 4;
-  const int lane = int(threadIdx.x) % G;
-  const int64_t group = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) / G;
-  const int64_t ngroups = int64_t(gridDim.x) * blockDim.x / G;
-  const int64_t nchunks = (total_rows + kRowsPerChunk - 1) / kRowsPerChunk;
-  RowCursor<SI> cur;
-  for (int64_t chunk = group; chunk < nchunks; chunk += ngroups) {
-    const int64_t r0 = chunk * kRowsPerChunk;
-    const int64_t r1 = r0 + kRowsPerChunk < total_rows ? r0 + kRowsPerChunk : total_rows;
-    cursor_seek(cur, tasks, row_start, n_tasks, contribs, r0);
-    for (int64_t rb = r0; rb < r1; rb += U) {
-      int64_t doff[U], soff[U];
-      SI ds0[U], ss0[U];
-      double coeff[U];
-      int len[U];
-      int maxlen = 0;
-#pragma unroll
-      for (int u = 0; u < U; ++u) {
-        len[u] = 0;
-        doff[u] = soff[u] = 0;
-        ds0[u] = ss0[u] = 0;
-        coeff[u] = 0.0;
-        const int64_t r = rb + u;
-        if (r >= r1) continue;
-        if (r >= cur.row_end) cursor_seek(cur, tasks, row_start, n_tasks, contribs, r);
-        if (cur.n_contrib == 1) {
-          doff[u] = cur.dofs;
-          soff[u] = cur.sofs;
-          ds0[u] = cur.dstr[0];
-          ss0[u] = cur.sstr[0];
-          coeff[u] = cur.coeff;
-          len[u] = cur.d0;
-          maxlen = max(maxlen, cur.d0);
-          cursor_step(cur);
-          continue;
-        }
-        // several source sub-blocks add into this row (SU(2)): fixed contribution order
-        for (int i = lane; i < cur.d0; i += G) {
-          double v = 0.0;
-          for (int c = 0; c < cur.n_contrib; ++c) {
-            const xgb_perm_contrib& cc = contribs[cur.contrib0 + c];
-            int64_t so = cc.src_base + int64_t(i) * (cur.rank > 0 ? cc.src_stride[0] : 0);
-#pragma unroll
-            for (int k = 1; k < XGB_MAX_LEGS; ++k)
-              if (k < cur.rank) so += cur.idx[k] * cc.src_stride[k];
-            v = fma(cc.coeff, __ldg(src + so), v);
-          }
-          dst[cur.dofs + int64_t(i) * cur.dstr[0]] = v;
-        }
-        cursor_step(cur);
-      }
-      for (int i = lane; i < maxlen; i += G) {
-        double v[U];
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (i < len[u]) v[u] = coeff[u] * __ldg(src + soff[u] + int64_t(i) * ss0[u]);
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-          if (i < len[u]) dst[doff[u] + int64_t(i) * ds0[u]] = v[u];
-      }
-    }
-  }
-}
-
-// Wide-row form (groups of G >= 8 lanes, rows of about G or more elements).  The row cursor above
-// keeps every leg's extent and strides in registers (128 per thread for G = 32: two CTAs per SM),
-// which leaves too few loads in flight to cover HBM latency on large tensors.  Here lane u < 8 of a
-// group decodes row u of the group's 8-row chunk on its own (task by the cached range or a binary
-// search, multi-index by 32-bit division, the per-leg fields read from the L1-resident task table
-// in a loop rather than held in registers), and the row's offsets, strides, length and coefficient
-// reach the other lanes by shuffles.  The loads go through shared memory instead of registers:
-// every lane copies the first 2G elements of each of the chunk's 8 rows (16 elements) with 8-byte
-// cp.async into its own column of the warp's staging buffer, so that in-flight data costs no
-// registers.  Two stages per warp: the next chunk is decoded and its copies issued before the
-// current chunk's copies are awaited, scaled by the coefficient and stored.  Elements past 2G of a
-// long row are copied directly.  It serves plans in which every task has exactly one contribution
-// (every abelian permute); plans with several contributions per task (SU(2) recoupling) take the
-// cursor kernel above.  Loop bounds that contain shuffles are warp-uniform (chunks are taken per
-// warp).
-constexpr int kWideSlots = 2;      // staged elements per row and lane
-constexpr int kWideThreads = 128;  // 4 warps per CTA: 32 KB of staging
-
-__device__ __forceinline__ void find_task(const int64_t* __restrict__ row_start, int n_tasks, int64_t r, int& ti,
-                                          int64_t& lo, int64_t& hi) {
-  if (r >= lo && r < hi) return;
-  int a = 0, b = n_tasks - 1;
-  while (a < b) {
-    const int mid = (a + b + 1) >> 1;
-    if (row_start[mid] <= r) a = mid; else b = mid - 1;
-  }
-  ti = a;
-  lo = row_start[a];
-  hi = row_start[a + 1];
-}
-
-__device__ __forceinline__ int split_index(int64_t& rem, int dk) {
-  if (rem < (int64_t(1) << 31)) {  // 32-bit division for the common case
-    const uint32_t r32 = uint32_t(rem), q = r32 / uint32_t(dk);
-    rem = q;
-    return int(r32 - q * uint32_t(dk));
-  }
-  const int64_t q = rem / dk;
-  const int ik = int(rem - q * dk);
-  rem = q;
-  return ik;
-}
-
-__device__ __forceinline__ void cp_async8(double* smem, const double* gmem) {
-  const unsigned sa = static_cast<unsigned>(__cvta_generic_to_shared(smem));
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(sa), "l"(gmem) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-template <typename SI>
-struct WideRow {  // one decoded row (len 0: no row)
-  long long dofs = 0, sofs = 0;
-  double coeff = 0.0;
-  int len = 0;
-  SI ds0 = 0, ss0 = 0;
-};
-
-template <typename SI>
-__device__ __forceinline__ WideRow<SI> wide_decode(const xgb_perm_task* __restrict__ tasks,
-                                                   const int64_t* __restrict__ row_start, int n_tasks,
-                                                   int64_t total_rows, const xgb_perm_contrib* __restrict__ contribs,
-                                                   int64_t r, bool valid, int& ti, int64_t& lo, int64_t& hi) {
-  WideRow<SI> w;
-  if (!valid || r >= total_rows) return w;
-  find_task(row_start, n_tasks, r, ti, lo, hi);
-  const xgb_perm_task& t = tasks[ti];
-  const xgb_perm_contrib& c = contribs[t.contrib0];  // the only contribution
-  const int rank = t.rank;
-  int64_t rem = r - lo;
-  int64_t dofs = t.dst_base, sofs = c.src_base;
-  for (int k = 1; k < rank; ++k) {
-    const int ik = split_index(rem, t.dims[k]);
-    dofs += int64_t(ik) * t.dst_stride[k];
-    sofs += int64_t(ik) * c.src_stride[k];
-  }
-  w.dofs = dofs;
-  w.sofs = sofs;
-  w.coeff = c.coeff;
-  w.len = rank > 0 ? t.dims[0] : 1;
-  w.ds0 = rank > 0 ? SI(t.dst_stride[0]) : SI(0);
-  w.ss0 = rank > 0 ? SI(c.src_stride[0]) : SI(0);
-  return w;
-}
-
-template <int G, typename SI>
-__global__ void __launch_bounds__(kWideThreads, 6) permute_rows_wide_kernel(const xgb_perm_task* __restrict__ tasks,
-                                                                            const int64_t* __restrict__ row_start,
-                                                                            int n_tasks, int64_t total_rows,
-                                                                            const xgb_perm_contrib* __restrict__ contribs,
-                                                                            const double* __restrict__ src,
-                                                                            double* __restrict__ dst) {
-  static_assert(G >= kRowsPerChunk && G <= 32, "one decoding lane per row of the chunk");
-  constexpr int kGroupsPerWarp = 32 / G;
-  constexpr int kHead = kWideSlots * G;  // staged elements per row
-  constexpr unsigned kFull = 0xffffffffu;
-  __shared__ double stage[kWideThreads / 32][2][kRowsPerChunk * kWideSlots][32];
-  const int lane = int(threadIdx.x) & 31;
-  const int wib = int(threadIdx.x) >> 5;
-  const int gl = lane % G;
-  const bool decoder = gl < kRowsPerChunk;
-  const int64_t warp = (int64_t(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
-  const int64_t nwarps = (int64_t(gridDim.x) * blockDim.x) >> 5;
-  const int64_t nchunks = (total_rows + kRowsPerChunk - 1) / kRowsPerChunk;
-  const int64_t step = nwarps * kGroupsPerWarp;
-  int ti = 0;
-  int64_t lo = 0, hi = 0;  // rows of task ti (empty: the first row searches)
-
-  // copies of the first kHead elements of the chunk's rows into stage st (one commit group)
-  auto issue = [&](const WideRow<SI>& w, int st) {
-#pragma unroll
-    for (int u = 0; u < kRowsPerChunk; ++u) {
-      const long long so = __shfl_sync(kFull, w.sofs, u, G);
-      const SI ss = __shfl_sync(kFull, w.ss0, u, G);
-      const int lu = __shfl_sync(kFull, w.len, u, G);
-#pragma unroll
-      for (int j = 0; j < kWideSlots; ++j) {
-        const int i = j * G + gl;
-        if (i < lu) cp_async8(&stage[wib][st][u * kWideSlots + j][lane], src + so + int64_t(i) * ss);
-      }
-    }
-    cp_async_commit();
-  };
-  // scaled stores of the staged elements, then the elements past kHead of long rows
-  auto drain = [&](const WideRow<SI>& w, int st) {
-#pragma unroll
-    for (int u = 0; u < kRowsPerChunk; ++u) {
-      const long long dof = __shfl_sync(kFull, w.dofs, u, G);
-      const SI ds = __shfl_sync(kFull, w.ds0, u, G);
-      const int lu = __shfl_sync(kFull, w.len, u, G);
-      const double cf = __shfl_sync(kFull, w.coeff, u, G);
-#pragma unroll
-      for (int j = 0; j < kWideSlots; ++j) {
-        const int i = j * G + gl;
-        if (i < lu) dst[dof + int64_t(i) * ds] = cf * stage[wib][st][u * kWideSlots + j][lane];
-      }
-    }
-    if (__reduce_max_sync(kFull, w.len) > kHead) {
-      for (int u = 0; u < kRowsPerChunk; ++u) {
-        const long long so = __shfl_sync(kFull, w.sofs, u, G);
-        const long long dof = __shfl_sync(kFull, w.dofs, u, G);
-        const SI ss = __shfl_sync(kFull, w.ss0, u, G);
-        const SI ds = __shfl_sync(kFull, w.ds0, u, G);
-        const int lu = __shfl_sync(kFull, w.len, u, G);
-        const double cf = __shfl_sync(kFull, w.coeff, u, G);
-        for (int i = kHead + gl; i < lu; i += G) dst[dof + int64_t(i) * ds] = cf * __ldg(src + so + int64_t(i) * ss);
-      }
-    }
-  };
-
-  int64_t cb = warp * kGroupsPerWarp;
-  if (cb >= nchunks) return;  // warp-uniform
-  int64_t chunk = cb + lane / G;
-  WideRow<SI> cur = wide_decode<SI>(tasks, row_start, n_tasks, total_rows, contribs, chunk * kRowsPerChunk + gl,
-                                    decoder && chunk < nchunks, ti, lo, hi);
-  issue(cur, 0);
-  int st = 0;
-  for (; cb < nchunks; cb += step) {
-    const int64_t nb = cb + step;
-    WideRow<SI> nxt;
-    if (nb < nchunks) {  // warp-uniform
-      chunk = nb + lane / G;
-      nxt = wide_decode<SI>(tasks, row_start, n_tasks, total_rows, contribs, chunk * kRowsPerChunk + gl,
-                            decoder && chunk < nchunks, ti, lo, hi);
-      issue(nxt, st ^ 1);
-      cp_async_wait<1>();  // the current chunk's group has landed
-    } else {
-      cp_async_wait<0>();
-    }
-    drain(cur, st);
-    cur = nxt;
-    st ^= 1;
-  }
-}
-
-PermRows perm_rows(const xgb_perm_task* tasks, int n_tasks, const xgb_perm_contrib* contribs, int n_contrib) {
-  PermRows r;
-  r.row_start.assign(size_t(n_tasks) + 1, 0);
-  double elems = 0, weighted = 0;
-  for (int t = 0; t < n_tasks; ++t) {
-    const int64_t d0 = tasks[t].rank > 0 ? std::max<int64_t>(tasks[t].dims[0], 1) : 1;
-    const int64_t rows = d0 > 0 ? tasks[t].nelem / d0 : 0;
-    r.row_start[t + 1] = r.row_start[t] + rows;
-    elems += double(tasks[t].nelem);
-    weighted += double(tasks[t].nelem) * double(d0);
-  }
-  r.total_rows = r.row_start.back();
-  for (int t = 0; t < n_tasks && r.single; ++t) r.single = tasks[t].n_contrib == 1;
-  auto wide = [](int64_t v) { return v > INT32_MAX || v < INT32_MIN; };
-  for (int t = 0; t < n_tasks && r.narrow; ++t)
-    for (int k = 0; k < tasks[t].rank; ++k)
-      if (wide(tasks[t].dst_stride[k])) r.narrow = false;
-  for (int c = 0; c < n_contrib && r.narrow; ++c)
-    for (int k = 0; k < XGB_MAX_LEGS; ++k)
-      if (wide(contribs[c].src_stride[k])) r.narrow = false;
-  const double avg = elems > 0 ? weighted / elems : 1.0;  // element-weighted row length
-  r.group = 1;
-  while (r.group < 32 && 2.0 * r.group <= avg * 1.25) r.group *= 2;
-  return r;
-}
-
-template <typename SI>
-void launch_permute_t(const xgb_perm_task* d_tasks, const int64_t* d_row_start, int n_tasks, int64_t total_rows,
-                      int group, bool single, const xgb_perm_contrib* d_contribs, const double* src, double* dst,
-                      cudaStream_t s) {
-  if (total_rows <= 0 || n_tasks <= 0) return;
-  // one group per chunk of kRowsPerChunk rows; enough CTAs to fill the GPU a few times over
-  const int64_t groups_needed = (total_rows + kRowsPerChunk - 1) / kRowsPerChunk;
-  const int64_t per_block = 256 / group;
-  const int64_t cap = int64_t(num_sms() > 0 ? num_sms() : 152) * 16;
-  const unsigned blocks = unsigned(std::max<int64_t>(1, std::min<int64_t>(cap, (groups_needed + per_block - 1) / per_block)));
-  // wide-row kernel: 128-thread CTAs, about one resident wave (six per SM) looping over the chunks
-  const int64_t wide_per_block = kWideThreads / group;
-  const unsigned wblocks = unsigned(std::max<int64_t>(
-      1, std::min<int64_t>(int64_t(num_sms() > 0 ? num_sms() : 152) * 6, (groups_needed + wide_per_block - 1) / wide_per_block)));
-  // the wide-row kernel for single-contribution plans whose rows fill a group of 8 or more lanes
-  switch (single || group < kRowsPerChunk ? group : -group) {
-    case 32: permute_rows_wide_kernel<32, SI><<<wblocks, kWideThreads, 0, s>>>(d_tasks, d_row_start, n_tasks, total_rows, d_contribs, src, dst); break;
-    case 16: permute_rows_wide_kernel<16, SI><<<wblocks, kWideThreads, 0, s>>>(d_tasks, d_row_start, n_tasks, total_rows, d_contribs, src, dst); break;
-    case 8: permute_rows_wide_kernel<8, SI><<<wblocks, kWideThreads, 0, s>>>(d_tasks, d_row_start, n_tasks, total_rows, d_contribs, src, dst); break;
-    case 4: permute_rows_kernel<4, SI><<<blocks, 256, 0, s>>>(d_tasks, d_row_start, n_tasks, total_rows, d_contribs, src, dst); break;
-    case 2: permute_rows_kernel<2, SI><<<blocks, 256, 0, s>>>(d_tasks, d_row_start, n_tasks, total_rows, d_contribs, src, dst); break;
-    case -32: permute_rows_kernel<32, SI><<<blocks, 256, 0, s>>>(d_tasks, d_row_start, n_tasks, total_rows, d_contribs, src, dst); break;
-    case -16: permute_rows_kernel<16, SI><<<blocks, 256, 0, s>>>(d_tasks, d_row_start, n_tasks, total_rows, d_contribs, src, dst); break;
-    case -8: permute_rows_kernel<8, SI><<<blocks, 256, 0, s>>>(d_tasks, d_row_start, n_tasks, total_rows, d_contribs, src, dst); break;
-    default: permute_rows_kernel<1, SI><<<blocks, 256, 0, s>>>(d_tasks, d_row_start, n_tasks, total_rows, d_contribs, src, dst); break;
-  }
-  count_launch();
-}
-
-void launch_permute(const xgb_perm_task* d_tasks, const int64_t* d_row_start, int n_tasks, int64_t total_rows,
-                    int group, bool narrow, bool single, const xgb_perm_contrib* d_contribs, const double* src,
-                    double* dst, cudaStream_t s) {
-  if (narrow)
-    launch_permute_t<int32_t>(d_tasks, d_row_start, n_tasks, total_rows, group, single, d_contribs, src, dst, s);
-  else launch_permute_t<int64_t>(d_tasks, d_row_start, n_tasks, total_rows, group, single, d_contribs, src, dst, s);
-}
-
 // ======================================================================= shared helpers
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -1413,11 +1006,7 @@ int xgb_gemm_tc_status(void) {
   XGB_GUARD_END
 }
 
-int xgb_permute(int n_tasks, const xgb_perm_task* tasks, int n_contrib, const xgb_perm_contrib* contribs,
-                const double* src, double* dst, void* stream_) {
-  XGB_REQUIRE_INIT();
-  XGB_GUARD_BEGIN
-  cudaStream_t s = pick(stream_);
+static int check_permute(int n_tasks, const xgb_perm_task* tasks, int n_contrib) {
   for (int t = 0; t < n_tasks; ++t) {
     if (tasks[t].rank < 0 || tasks[t].rank > XGB_MAX_LEGS) return set_error(XGB_E_BADPLAN, "task rank out of range");
     if (tasks[t].contrib0 < 0 || tasks[t].contrib0 + tasks[t].n_contrib > n_contrib)
@@ -1429,17 +1018,36 @@ int xgb_permute(int n_tasks, const xgb_perm_task* tasks, int n_contrib, const xg
     }
     if (prod != tasks[t].nelem) return set_error(XGB_E_BADPLAN, "task nelem differs from the product of its extents");
   }
-  if (n_tasks == 0) return XGB_OK;
-  const PermRows rows = perm_rows(tasks, n_tasks, contribs, n_contrib);
-  if (rows.total_rows == 0) return XGB_OK;
-  auto* dt = upload(tasks, size_t(n_tasks), s);
-  auto* ds = upload(rows.row_start.data(), rows.row_start.size(), s);
-  auto* dc = upload(contribs, size_t(n_contrib), s);
-  launch_permute(dt, ds, n_tasks, rows.total_rows, rows.group, rows.narrow, rows.single, dc, src, dst, s);
+  return XGB_OK;
+}
+
+int xgb_permute(int n_tasks, const xgb_perm_task* tasks, int n_contrib, const xgb_perm_contrib* contribs,
+                const double* src, double* dst, void* stream_) {
+  XGB_REQUIRE_INIT();
+  XGB_GUARD_BEGIN
+  cudaStream_t s = pick(stream_);
+  if (const int rc = check_permute(n_tasks, tasks, n_contrib)) return rc;
+  const PlanePlan plan = plan_planes(tasks, n_tasks, contribs);
+  if (plan.start.back() == 0) return XGB_OK;
+  auto* dt = upload(plan.tasks.data(), plan.tasks.size(), s);
+  auto* ds = upload(plan.start.data(), plan.start.size(), s);
+  auto* dc = upload(plan.sources.data(), plan.sources.size(), s);
+  launch_permute(dt, ds, int(plan.tasks.size()), plan.start.back(), plan.form, dc, src, dst, s);
   dev_free(dt);
   dev_free(ds);
   dev_free(dc);
   return check_cuda(cudaGetLastError(), "permute launch");
+  XGB_GUARD_END
+}
+
+int xgb_permute_walk_host(int n_tasks, const xgb_perm_task* tasks, int n_contrib, const xgb_perm_contrib* contribs,
+                          const double* src, double* dst, int* transposed) {
+  XGB_GUARD_BEGIN
+  if (const int rc = check_permute(n_tasks, tasks, n_contrib)) return rc;
+  const PlanePlan plan = plan_planes(tasks, n_tasks, contribs);
+  permute_planes_host(plan, src, dst);
+  if (transposed) *transposed = plan.form.transpose;
+  return XGB_OK;
   XGB_GUARD_END
 }
 

@@ -79,19 +79,43 @@ inline bool gemm_precision_available(int p) {
   return p == XGB_PREC_FP64 || p == XGB_PREC_3XTF32 || p == XGB_PREC_FP32 || p == XGB_PREC_BF16X9 ||
          p == XGB_PREC_F64TC;
 }
-// permute launch shape: rows (runs along output leg 0) per task as prefix sums, and the number of
-// threads that share one row (a power of two up to 32, from the element-weighted row length)
-struct PermRows {
-  std::vector<int64_t> row_start;
-  int64_t total_rows = 0;
-  int group = 1;
-  bool narrow = true;  // every stride fits 32 bits (the kernel keeps them in 32-bit registers)
-  bool single = true;  // every task has exactly one contribution (no SU(2) sums)
+// permute (permute.cu): each task as planes of two legs, chunked, with the other legs decoded per plane
+constexpr int kPlaneOuter = XGB_MAX_LEGS - 2;
+struct PlaneTask {
+  int64_t dst_base, dst_a, dst_b;
+  int32_t na, nb;    // extents of the plane's legs
+  int32_t ci, cj;    // chunk of a plane
+  int32_t nci, ncj;  // chunks along each leg
+  int32_t n_outer, source0, n_source;
+  int32_t ra, rb;          // reciprocals of la, lb (16 bits of fraction)
+  int16_t la, ia, lb, ib;  // lanes along A and rows of them; along B where the transposed form reads
+  int32_t y_is_a, pad;     // a lane has more steps along A than along B
+  int32_t odim[kPlaneOuter];
+  int64_t odst[kPlaneOuter];
 };
-PermRows perm_rows(const xgb_perm_task* tasks, int n_tasks, const xgb_perm_contrib* contribs, int n_contrib);
-void launch_permute(const xgb_perm_task* d_tasks, const int64_t* d_row_start, int n_tasks, int64_t total_rows,
-                    int group, bool narrow, bool single, const xgb_perm_contrib* d_contribs, const double* src,
-                    double* dst, cudaStream_t s);
+struct PlaneSource {
+  int64_t base;
+  double coeff;
+  int64_t a, b, outer[kPlaneOuter];
+};
+struct PlaneForm {
+  int group = 4;           // lanes per chunk
+  int max_source = 0;      // most sources of one task
+  bool transpose = false;  // read along the source's unit-stride leg, through shared memory
+  bool narrow = true;      // offsets within a task and its number of chunks fit 32 bits
+  bool single = true;      // one source per task (no SU(2) sums)
+};
+struct PlanePlan {
+  std::vector<PlaneTask> tasks;
+  std::vector<PlaneSource> sources;
+  std::vector<int64_t> start;  // chunks of planes before each task, and their total
+  PlaneForm form;
+};
+PlanePlan plan_planes(const xgb_perm_task* tasks, int n_tasks, const xgb_perm_contrib* contribs);
+void launch_permute(const PlaneTask* d_tasks, const int64_t* d_start, int n_tasks, int64_t n_planes, PlaneForm form,
+                    const PlaneSource* d_sources, const double* src, double* dst, cudaStream_t s);
+// the plan walked on the host by the kernel's index arithmetic
+void permute_planes_host(const PlanePlan& plan, const double* src, double* dst);
 // h_descs: host copy of the descriptors (blocks at least kSvdGridMin wide run one at a time on a
 // grid-wide Jacobi kernel over all SMs; nullptr keeps every block on the cluster kernel)
 void launch_svd(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, const int64_t* d_work_off, int n,

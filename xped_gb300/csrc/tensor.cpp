@@ -149,13 +149,11 @@ struct PermPlan {
   MetaPtr out;
   bool needs_zero = false;
   int n_tasks = 0;
-  int64_t total_rows = 0;
-  int group = 1;
-  bool narrow = true;
-  bool single = true;
-  xgb_perm_task* d_tasks = nullptr;
-  int64_t* d_row_start = nullptr;
-  xgb_perm_contrib* d_contribs = nullptr;
+  int64_t n_planes = 0;
+  PlaneForm form;
+  PlaneTask* d_tasks = nullptr;
+  int64_t* d_start = nullptr;
+  PlaneSource* d_sources = nullptr;
   double bytes = 0;  // algorithmic: every output written once, every contribution read once
 };
 struct GemmPlan {
@@ -192,16 +190,14 @@ struct GemmPlan {
 std::shared_ptr<PermPlan> upload_tables(const PermTables& t) {
   auto plan = std::make_shared<PermPlan>();
   plan->out = t.out;
-  plan->n_tasks = int(t.tasks.size());
   plan->needs_zero = t.needs_zero;
-  plan->d_tasks = plan->mem.table(t.tasks);
-  const PermRows rows = perm_rows(t.tasks.data(), int(t.tasks.size()), t.contribs.data(), int(t.contribs.size()));
-  plan->total_rows = rows.total_rows;
-  plan->group = rows.group;
-  plan->narrow = rows.narrow;
-  plan->single = rows.single;
-  plan->d_row_start = plan->mem.table(rows.row_start);
-  plan->d_contribs = plan->mem.table(t.contribs);
+  const PlanePlan planes = plan_planes(t.tasks.data(), int(t.tasks.size()), t.contribs.data());
+  plan->n_tasks = int(planes.tasks.size());
+  plan->n_planes = planes.start.back();
+  plan->form = planes.form;
+  plan->d_tasks = plan->mem.table(planes.tasks);
+  plan->d_start = plan->mem.table(planes.start);
+  plan->d_sources = plan->mem.table(planes.sources);
   for (const auto& task : t.tasks) plan->bytes += 8.0 * double(task.nelem) * (1 + task.n_contrib);
   return plan;
 }
@@ -444,8 +440,8 @@ std::shared_ptr<PermPlan> get_perm_plan(const TensorMeta& m, uint32_t mask, int 
 Tensor run_perm_plan(const PermPlan& plan, const Tensor& src) {
   Tensor out = plan.needs_zero ? zeros(plan.out) : empty_like_meta(plan.out);
   prof_begin(K_PERMUTE, stream());
-  launch_permute(plan.d_tasks, plan.d_row_start, plan.n_tasks, plan.total_rows, plan.group, plan.narrow, plan.single,
-                 plan.d_contribs, src.data(), out.data(), stream());
+  launch_permute(plan.d_tasks, plan.d_start, plan.n_tasks, plan.n_planes, plan.form, plan.d_sources,
+                 src.data(), out.data(), stream());
   prof_end(K_PERMUTE, stream(), plan.bytes);
   return out;
 }
