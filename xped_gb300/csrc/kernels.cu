@@ -261,10 +261,55 @@ void prof_end(int kind, cudaStream_t s, double work) {
 // ======================================================================= GEMM
 // Grouped GEMM on the CUDA cores: C_g = alpha*op(A_g)op(B_g) + beta*C_g.  One
 // CTA per TILE x TILE output tile of one group; 256 threads, each owning a
-// (TILE/16)^2 micro-tile.  T = double is the FP64 form (FP64 on GB300 runs on
-// the narrow DFMA pipe, so the host picks the tile edge that spreads the work
-// over the most SMs); T = float is the FP32 form (operands rounded to FP32 as
-// they are staged, FP32 accumulation, alpha/beta and the store in FP64).
+// (TILE/16)^2 micro-tile.  T = double is the FP64 form, bound by GB300's narrow
+// FP64 pipe (two multiply-adds per clock and SM): it reaches 1.0 of that rate on
+// nine blocks 36 to 616 wide (1010 us; 1399 us when edge tiles were multiplied
+// whole and the tiles were 64 wide).  T = float is the FP32 form (operands
+// rounded to FP32 as they are staged, FP32 accumulation, alpha/beta and the
+// store in FP64).
+// A warp owns 8 x 4 outputs of every 16 x 16 sub-block of the tile, and multiplies only the sub-blocks where some of
+// its outputs lie inside the block: a warp's FP64 instruction takes the pipe 64 cycles whatever its active lanes, and
+// predicated off as well, so the count of sub-blocks is a template argument of the inner loop.  An edge tile costs its
+// extents rounded up to 8 x 4 instead of the whole tile (64-wide tiles on blocks 36 to 616 wide: 17 % of the time).
+// Unrolled eight times so that the next operands are read ahead of the pipe: 1089 us without, 1010 with.
+template <int R, int RM, int CM, int LD, typename T>
+__device__ __forceinline__ void multiply(const T (*As)[LD], const T (*Bs)[LD], int kmax, int row, int col, T (*acc)[R]) {
+#pragma unroll 8
+  for (int kk = 0; kk < kmax; ++kk) {
+    T a[RM], b[CM];
+#pragma unroll
+    for (int r = 0; r < RM; ++r) a[r] = As[kk][row + 16 * r];
+#pragma unroll
+    for (int c = 0; c < CM; ++c) b[c] = Bs[kk][col + 16 * c];
+#pragma unroll
+    for (int r = 0; r < RM; ++r)
+#pragma unroll
+      for (int c = 0; c < CM; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+  }
+}
+template <int R, int RM, int LD, typename T>
+__device__ __forceinline__ void multiply_cols(int cm, const T (*As)[LD], const T (*Bs)[LD], int kmax, int row, int col,
+                                              T (*acc)[R]) {
+  if (cm == 1) multiply<R, RM, 1, LD>(As, Bs, kmax, row, col, acc);
+  if constexpr (R >= 2)
+    if (cm == 2) multiply<R, RM, 2, LD>(As, Bs, kmax, row, col, acc);
+  if constexpr (R >= 4) {
+    if (cm == 3) multiply<R, RM, 3, LD>(As, Bs, kmax, row, col, acc);
+    if (cm == 4) multiply<R, RM, 4, LD>(As, Bs, kmax, row, col, acc);
+  }
+}
+template <int R, int LD, typename T>
+__device__ __forceinline__ void multiply_live(int rm, int cm, const T (*As)[LD], const T (*Bs)[LD], int kmax, int row,
+                                              int col, T (*acc)[R]) {
+  if (rm == 1) multiply_cols<R, 1, LD>(cm, As, Bs, kmax, row, col, acc);
+  if constexpr (R >= 2)
+    if (rm == 2) multiply_cols<R, 2, LD>(cm, As, Bs, kmax, row, col, acc);
+  if constexpr (R >= 4) {
+    if (rm == 3) multiply_cols<R, 3, LD>(cm, As, Bs, kmax, row, col, acc);
+    if (rm == 4) multiply_cols<R, 4, LD>(cm, As, Bs, kmax, row, col, acc);
+  }
+}
+
 template <int TILE, typename T>
 __global__ void __launch_bounds__(256) gemm_simt_kernel(const xgb_gemm_desc* __restrict__ descs,
                                                         const GemmTile* __restrict__ tiles, const double* __restrict__ A,
@@ -281,16 +326,26 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const xgb_gemm_desc* __r
   const xgb_gemm_desc d = descs[t.g];
   const int64_t kbeg = t.k0, kend = t.k1 < 0 ? d.k : t.k1;
   const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
   const int64_t row0 = int64_t(t.tm) * TILE, col0 = int64_t(t.tn) * TILE;
-  // a warp whose outputs all lie outside the block (an edge tile of a block narrower than the tile)
-  // skips the multiply-adds: GB300's narrow FP64 pipe takes as long for a warp instruction whatever
-  // its active lanes; its share of the staging loads and the barriers stays
-  bool live = false;
+  // FP64: warps w and w + 4 (one quarter of the SM) hold the two row halves of a column group; the groups rotate with
+  // the tile so that the CTAs of an SM do not all have their fuller warps on the same quarter.  FP32 (not bound by its
+  // pipe): 16 x 2 outputs of every sub-block, and all sub-blocks of a warp with any live output.
+  constexpr bool kNarrowPipe = sizeof(T) == 8;
+  const int warp = tid >> 5, lane = tid & 31;
+  const int wrow = kNarrowPipe ? (warp >> 2) * 8 : 0;
+  const int wcol = kNarrowPipe ? ((warp + int(blockIdx.x)) & 3) * 4 : warp * 2;
+  const int tx = kNarrowPipe ? wrow + (lane & 7) : tid & 15;
+  const int ty = kNarrowPipe ? wcol + (lane >> 3) : tid >> 4;
+  const int64_t rows = d.m - row0 - wrow, cols = d.n - col0 - wcol;
+  const int rm = rows <= 0 ? 0 : int(rows + 15 < TILE ? (rows + 15) / 16 : R);
+  const int cm = cols <= 0 ? 0 : int(cols + 15 < TILE ? (cols + 15) / 16 : R);
+  bool live = kNarrowPipe;
+  if constexpr (!kNarrowPipe) {
 #pragma unroll
-  for (int r = 0; r < R; ++r)
+    for (int r = 0; r < R; ++r)
 #pragma unroll
-    for (int c = 0; c < R; ++c) live |= row0 + tx + 16 * r < d.m && col0 + ty + 16 * c < d.n;
+      for (int c = 0; c < R; ++c) live |= row0 + tx + 16 * r < d.m && col0 + ty + 16 * c < d.n;
+  }
   const bool warp_live = __any_sync(0xffffffffu, live);
   T acc[R][R];
 #pragma unroll
@@ -338,18 +393,20 @@ __global__ void __launch_bounds__(256) gemm_simt_kernel(const xgb_gemm_desc* __r
   for (int64_t k0 = kbeg; k0 < kend; k0 += BK) {
     const bool more = k0 + BK < kend;
     if (more) fetch(k0 + BK);
-    const int kmax = !warp_live ? 0 : (kend - k0) < BK ? int(kend - k0) : BK;
-    for (int kk = 0; kk < kmax; ++kk) {
-      T a[R], b[R];
+    const int kmax = !kNarrowPipe && !warp_live ? 0 : (kend - k0) < BK ? int(kend - k0) : BK;
+    if constexpr (kNarrowPipe) multiply_live<R, TILE + 1>(rm, cm, As[st], Bs[st], kmax, tx, ty, acc);
+    else
+      for (int kk = 0; kk < kmax; ++kk) {
+        T a[R], b[R];
 #pragma unroll
-      for (int r = 0; r < R; ++r) a[r] = As[st][kk][tx + 16 * r];
+        for (int r = 0; r < R; ++r) a[r] = As[st][kk][tx + 16 * r];
 #pragma unroll
-      for (int c = 0; c < R; ++c) b[c] = Bs[st][kk][ty + 16 * c];
+        for (int c = 0; c < R; ++c) b[c] = Bs[st][kk][ty + 16 * c];
 #pragma unroll
-      for (int r = 0; r < R; ++r)
+        for (int r = 0; r < R; ++r)
 #pragma unroll
-        for (int c = 0; c < R; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
-    }
+          for (int c = 0; c < R; ++c) acc[r][c] = fma(a[r], b[c], acc[r][c]);
+      }
     if (more) stash(st ^ 1);
     __syncthreads();
     st ^= 1;
@@ -458,8 +515,7 @@ void order_tiles_by_work(std::vector<GemmTile>& tiles, const xgb_gemm_desc* desc
 }
 
 int choose_gemm_tile(const xgb_gemm_desc* descs, int n) {
-  // Largest tile edge that still yields >= 2 CTAs per SM; FP64 throughput is
-  // per SM, so spreading tiles over SMs beats bigger tiles' reuse here.
+  // FP32 form: the largest tile edge that still yields >= 2 CTAs per SM (operand reuse, then SMs in use)
   const int target = 2 * (g_rt.sms > 0 ? g_rt.sms : 152);
   for (int tile : {64, 32}) {
     int64_t cnt = 0;
@@ -467,6 +523,18 @@ int choose_gemm_tile(const xgb_gemm_desc* descs, int n) {
     if (cnt >= target) return tile;
   }
   return 16;
+}
+
+int choose_f64_tile(const xgb_gemm_desc* descs, int n) {
+  // The FP64 pipe is the bound, so what counts is that the SMs end together and that edges are not rounded up far:
+  // 16-wide tiles are the fastest or within 1 % of it on every list measured from 20 to 1000 wide, with and without
+  // split-K (us, 16 / 32 / 64 wide: nine blocks of 36 to 616 1010 / 1037 / 1159, nine of 9 to 154 31 / 49 / 166, one
+  // of 1000 1657 / 1829 / 2024).  Lists of very many tiles take 32 (nine blocks of 72 to 1232, 18900 tiles: 7907 /
+  // 7864 / 8379), which also keeps their tables short: they are built while the GPU waits.
+  constexpr int64_t kMost = 16384;
+  int64_t cnt = 0;
+  for (int g = 0; g < n; ++g) cnt += ((descs[g].m + 15) / 16) * ((descs[g].n + 15) / 16);
+  return cnt > kMost ? 32 : 16;
 }
 
 // ======================================================================= shared helpers
@@ -970,13 +1038,13 @@ int xgb_grouped_gemm(int precision, int n_groups, const xgb_gemm_desc* descs, co
       dev_free(p);
     return check_cuda(cudaGetLastError(), "tensor-core gemm launch");
   }
-  const int tile = choose_gemm_tile(descs, n_groups);
   if (precision == XGB_PREC_FP64) {
     // FP64: the built-in shape (no split-K) or, with autotuning on, the tuned one of the list's bucket
-    const F64Config cfg = gemm_f64_config(descs, n_groups, A, B, {tile, 0}, s);
+    const F64Config cfg = gemm_f64_config(descs, n_groups, A, B, {choose_f64_tile(descs, n_groups), 0}, s);
     run_gemm_f64_config(descs, n_groups, cfg, A, B, C, alpha, beta, s);
     return check_cuda(cudaGetLastError(), "gemm launch");
   }
+  const int tile = choose_gemm_tile(descs, n_groups);
   std::vector<GemmTile> tiles;
   for (int g = 0; g < n_groups; ++g) {
     int64_t tm = (descs[g].m + tile - 1) / tile, tn = (descs[g].n + tile - 1) / tile;

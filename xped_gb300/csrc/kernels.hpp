@@ -286,6 +286,7 @@ int autotune_mode();
 // helpers
 size_t svd_work_elems(int64_t m, int64_t n);
 size_t qr_work_elems(int64_t m, int64_t n);
-int choose_gemm_tile(const xgb_gemm_desc* descs, int n);  // host-side tile heuristic
+int choose_gemm_tile(const xgb_gemm_desc* descs, int n);  // host-side tile heuristic, FP32 form
+int choose_f64_tile(const xgb_gemm_desc* descs, int n);   // FP64 form
 
 }  // namespace xgb

@@ -62,7 +62,7 @@ void grouped_gemm(const std::vector<xgb_gemm_desc>& d, const double* A, const do
                   double alpha = 1.0, double beta = 0.0, int shape = kGemmDense, bool allow_tc = false) {
   if (d.empty()) return;
   if (allow_tc) {
-    const F64Config tfb{choose_gemm_tile(d.data(), int(d.size())), 2, f64tc_heuristic(d.data(), int(d.size()))};
+    const F64Config tfb{choose_f64_tile(d.data(), int(d.size())), 2, f64tc_heuristic(d.data(), int(d.size()))};
     if (gemm_f64_config(d.data(), int(d.size()), A, B, tfb, s, true).tc) {
       double flops = 0;
       for (const auto& g : d) flops += 2.0 * double(g.m) * double(g.n) * double(g.k);
@@ -72,7 +72,7 @@ void grouped_gemm(const std::vector<xgb_gemm_desc>& d, const double* A, const do
       return;
     }
   }
-  const F64Config fallback{choose_gemm_tile(d.data(), int(d.size())), 2};
+  const F64Config fallback{choose_f64_tile(d.data(), int(d.size())), 2};
   const F64Config cfg = gemm_f64_config(d.data(), int(d.size()), A, B, fallback, s);
   const F64Plan p = plan_gemm_f64(d.data(), int(d.size()), cfg, shape);
   double flops = 0;

@@ -651,9 +651,8 @@ Tensor matmul(const Tensor& a0, const Tensor& b0, bool adj_a, bool adj_b) {
     // both routes are FP64-class: the tensor-core form or the FP64 CUDA-core kernel, whichever the
     // autotuner measures faster for this size bucket (built-in rule: average k >= 64)
     const auto& hd = plan->host_descs;
-    const F64Config rc = gemm_f64_config(hd.data(), int(hd.size()), a.data(), b.data(),
-                                         F64Config{plan->tile, 0, f64tc_heuristic(hd.data(), int(hd.size()))},
-                                         stream(), true);
+    const F64Config rule{choose_f64_tile(hd.data(), int(hd.size())), 0, f64tc_heuristic(hd.data(), int(hd.size()))};
+    const F64Config rc = gemm_f64_config(hd.data(), int(hd.size()), a.data(), b.data(), rule, stream(), true);
     std::lock_guard<std::mutex> lk(g_plan_mu);
     plan->oz_route = rc.tc;
     plan->oz_routed = true;
@@ -742,7 +741,8 @@ Tensor matmul(const Tensor& a0, const Tensor& b0, bool adj_a, bool adj_b) {
     if (!plan->f64_ready) {  // FP64 CUDA-core launch shape: the autotuner's choice or the built-in rule
       const auto& descs = plan->host_descs;
       const F64Config cfg =
-          gemm_f64_config(descs.data(), int(descs.size()), a.data(), b.data(), {plan->tile, 0}, stream());
+          gemm_f64_config(descs.data(), int(descs.size()), a.data(), b.data(),
+                          {choose_f64_tile(descs.data(), int(descs.size())), 0}, stream());
       plan->f64 = plan_gemm_f64(descs.data(), int(descs.size()), cfg);
       plan->d_f64_tiles = plan->mem.table(plan->f64.tiles);
       plan->d_f64_red = plan->mem.table(plan->f64.red);
