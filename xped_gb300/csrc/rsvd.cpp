@@ -51,10 +51,12 @@ class Staging {
 
 double* alloc_d(int64_t n) { return static_cast<double*>(dev_alloc(sizeof(double) * size_t(std::max<int64_t>(n, 1)))); }
 
-// Grouped FP64 GEMM of the sketch pipeline.  When the output tiles cannot fill the SMs
-// (the l x l Gram matrices Y^T Y: few tiles, k = the block's row count) the k range of each
-// tile is split so that about two CTAs per SM run; the partial tiles land in a workspace and
-// one reduce launch adds them in a fixed order (deterministic result).  With autotuning on, the
+// Grouped FP64 GEMM of the sketch pipeline.  The k range of each tile is split so that about eight CTAs
+// per SM run: few tiles (the l x l Gram matrices) would leave SMs idle, and the products' two or three
+// tiles per SM, some with few live columns, end at different times (six blocks of 134 to 1024 times 37
+// columns, ideal 144 us: 230 us at two CTAs per SM, 181 at five, 173 at eight, 168 at twelve).  The
+// partial tiles land in a workspace and one reduce launch adds them in a fixed order (deterministic
+// result).  With autotuning on, the
 // tile edge and the split target are the tuned ones of the list's size bucket.
 // allow_tc (callers running the FP64-accurate tensor-core form): the autotuner may also route the list
 // to that form when it measures it faster (built-in rule: average k >= 64), computing C in full.
@@ -72,7 +74,7 @@ void grouped_gemm(const std::vector<xgb_gemm_desc>& d, const double* A, const do
       return;
     }
   }
-  const F64Config fallback{choose_f64_tile(d.data(), int(d.size())), 2};
+  const F64Config fallback{choose_f64_tile(d.data(), int(d.size())), 8};
   const F64Config cfg = gemm_f64_config(d.data(), int(d.size()), A, B, fallback, s);
   const F64Plan p = plan_gemm_f64(d.data(), int(d.size()), cfg, shape);
   double flops = 0;
@@ -224,7 +226,7 @@ void batched_svd(const std::vector<xgb_svd_desc>& d, const double* A, double* U,
 // between the products of a subspace iteration only have to stay well
 // conditioned; their span is what the iteration carries).  Every pass is two
 // grouped FP64 GEMMs (Gram matrix, Q R^-1) spread over all SMs plus one small
-// Cholesky / triangular-inverse launch (one CTA per block).  The passes alternate
+// launch for the Cholesky factor and its inverse (one CTA or cluster per block).  The passes alternate
 // between Y and Q; returns the buffer holding the basis (Q for 3 passes, Y for
 // 2); the other one holds garbage afterwards.
 double* orthonormalise(const std::vector<int64_t>& rows, const std::vector<int64_t>& cols,

@@ -1,12 +1,17 @@
 // Kernels of the randomized blockwise tSVD: the seeded Gaussian test
 // matrices and the singular-vector sign convention applied after the
 // sketch-space singular vectors are lifted back (U = Q U_B).
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <cstdint>
 #include <mutex>
+#include <stdexcept>
+#include <string>
 
 #include "kernels.hpp"
+
+namespace cg = cooperative_groups;
 
 namespace xgb {
 namespace {
@@ -166,15 +171,42 @@ __global__ void svd_bwd_scale_kernel(const SvdBwdDesc* __restrict__ descs, const
 // below it, so the factor stays finite and well scaled; such pivots are
 // counted in *bad.
 //
-// Both factorisations are right-looking, so every step is a parallel update
-// of a trailing block: Cholesky by columns (scale the column, rank-1 update of
-// the trailing lower triangle), the inverse by forward elimination of the
-// identity (X <- rows of L^-1 as they are finished).  Matrices live in shared
-// memory, row-major with an odd leading dimension, when two of them fit;
-// larger blocks use the same loops on global memory.
-//
-// kInverse = false: the Cholesky factor only; L (lower triangle and diagonal) is
-// left column-major in G for trinv_kernel, which forms L^-1 with many CTAs.
+// Three forms: chol_narrow_kernel, chol_cluster_kernel, and beyond their widths chol_inv_body on global memory (right-
+// looking: Cholesky by columns; the inverse in trinv_kernel by many CTAs, or, kInverse = true for lists wider than its
+// registers allow, by forward elimination of the identity; blocks of such a list that fit shared memory use it,
+// row-major with an odd leading dimension).
+constexpr int kCholNarrow = 48;    // widest list for one CTA per block
+constexpr int kCholCluster = 320;  // widest list for a cluster of eight per block (217 KB of shared memory each)
+constexpr unsigned kFullWarp = 0xffffffffu;
+
+// trace of G by one warp, groups of 32 in order
+template <typename Diag>
+__device__ __forceinline__ double chol_trace(int l, Diag diag) {
+  const int lane = threadIdx.x & 31;
+  double t = 0;
+  for (int g0 = 0; g0 < l; g0 += 32) t += warp_sum_d(g0 + lane < l ? diag(g0 + lane) : 0.0);
+  return t;
+}
+struct CholShift {
+  double shift, floor_v;
+  __device__ __forceinline__ CholShift(const CholDesc& d, double trace, double rel_shift) {
+    const double l = double(d.l);
+    shift = rel_shift * (double(d.m) * l + l * (l + 1)) * trace;
+    floor_v = fmax(2.220446049250313e-16 * (trace > 0.0 ? trace / l : 0.0), 1e-300);
+  }
+};
+struct CholPivot {
+  double r, diag;  // 1 / L_jj, L_jj
+  bool dead;       // at or below the floor, or NaN; tested on the bits
+  __device__ __forceinline__ CholPivot(double x, const CholShift& sh) {
+    const long long bits = __double_as_longlong(x);
+    dead = !(bits > __double_as_longlong(sh.floor_v) && bits <= 0x7ff0000000000000ll);
+    const double v = dead ? sh.floor_v : x;
+    r = rsqrt(v);
+    diag = v * r;
+  }
+};
+
 template <bool kShared, bool kInverse>
 __device__ void chol_inv_body(const CholDesc& d, double* __restrict__ Gg, double* __restrict__ Xg, double rel_shift,
                               int* __restrict__ bad, double* sm) {
@@ -363,53 +395,322 @@ __global__ void __launch_bounds__(1024) chol_inv_kernel(const CholDesc* __restri
     chol_inv_body<false, kInverse>(d, G + d.g_off, Rinv + d.g_off, rel_shift, bad, sm);
 }
 
-// The same shifted Cholesky as chol_inv_body<true, false> for blocks up to kCholWarpL wide, run by one
-// warp per block with no block-wide barriers: the lanes own rows (i = lane + 32 j), every lane forms
-// the pivot itself, and each element sees the same FMAs in the same order as in the 1024-thread
-// kernel (the trace, which sets the shift, is summed in that kernel's order too), so both give the
-// same bits.  For narrow blocks the 1024-thread kernel spends two block barriers per column on a few
-// hundred FMAs; a lane's share grows like l^3 / 192 dependent shared-memory FMAs, so above 48 columns
-// (measured: ~390 us per launch at widths up to 128, against ~110 us) the block kernel is used.
-constexpr int kCholWarpL = 48;
-__global__ void __launch_bounds__(32) chol_warp_kernel(const CholDesc* __restrict__ descs, double* __restrict__ G,
-                                                       double rel_shift, int* __restrict__ bad) {
-  extern __shared__ double wsm[];
+// Narrow blocks: factor and inverse together, in one CTA's shared memory.
+//
+// Iteration j starts with columns <= j of L final and finishes column j + 1 (all of it in warp 0, which forms the
+// pivot between its multiply-add and the scaling), applies column j to the columns behind and row j - 1 of X to the
+// rows behind while warp 1 finishes row j of X; one barrier ends it.  The other warps take a row each, lanes along its
+// columns of X and L: no index is divided.  What bounds it is the chain of warp 0 (on GB300 a dependent FP64 operation
+// takes ~64 cycles and rsqrt ~430, so about 700 cycles a column).  So the warps that share warp 0's quarter of the SM
+// stay out of the updates, and the pivot test is on the bits (a comparison is an FP64 instruction).
+// Measured (two blocks, widths about 16 / 32 / 48, factor and inverse): 63 / 85 / 158 us with one warp per block and a
+// second kernel for the inverse, 25 / 29 / 44 now.
+__global__ void __launch_bounds__(512) chol_narrow_kernel(const CholDesc* __restrict__ descs,
+                                                          const double* __restrict__ G, double* __restrict__ Rinv,
+                                                          double rel_shift, int* __restrict__ bad) {
+  extern __shared__ double sm[];
+  __shared__ double trace_s, pivots[kCholNarrow];  // pivots: 1 / L_jj
+  constexpr int kSlots = (kCholNarrow + 31) / 32;
   const CholDesc d = descs[blockIdx.x];
-  const int l = int(d.l), lane = threadIdx.x, ld = l | 1;
-  double* Gg = G + d.g_off;
-  auto LA = [&](int i, int k) -> double& { return wsm[i * ld + k]; };
-  for (int e = lane; e < l * l; e += 32) {  // upper triangle of G, as in chol_inv_body
-    const int i = e % l, k = e / l;
-    LA(i, k) = Gg[i <= k ? e : k + i * l];
-  }
-  __syncwarp();
-  double t = 0;
-  for (int g0 = 0; g0 < l; g0 += 32) t += warp_sum_d(g0 + lane < l ? LA(g0 + lane, g0 + lane) : 0.0);
-  const double shift = rel_shift * (double(d.m) * l + double(l) * (l + 1)) * t;
-  const double avg = t > 0.0 ? t / l : 0.0;
-  const double dfloor = fmax(2.220446049250313e-16 * avg, 1e-300);
-  for (int i = lane; i < l; i += 32) LA(i, i) += shift;
-  __syncwarp();
-  for (int j = 0; j < l; ++j) {
-    const double dj = LA(j, j);
-    const int dd = !(dj > dfloor);  // also true for NaN
-    const double v = dd ? dfloor : dj;
-    const double inv = rsqrt(v);
-    const double p = v * inv;
-    __syncwarp();
-    if (lane == 0) {
-      LA(j, j) = p;
-      if (dd) atomicAdd(bad, 1);
+  const int l = int(d.l), ld = l | 1, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, warps = blockDim.x >> 5;
+  if (l == 0) return;
+  const double* Gg = G + d.g_off;
+  double* Ls = sm;
+  double* Xs = sm + l * ld;
+  for (int k = warp; k < l; k += warps)  // row k of the lower triangle from column k of G's upper one
+    for (int i = lane; i <= k; i += 32) {
+      Ls[k * ld + i] = Gg[i + k * l];
+      Xs[k * ld + i] = i == k ? 1.0 : 0.0;
     }
-    for (int i = j + 1 + lane; i < l; i += 32) LA(i, j) = dd ? 0.0 : LA(i, j) * inv;
-    __syncwarp();
-    for (int i = j + 1 + lane; i < l; i += 32)
-      for (int k = j + 1; k <= i; ++k) LA(i, k) = fma(-LA(i, j), LA(k, j), LA(i, k));
-    __syncwarp();
+  __syncthreads();
+  if (warp == 0) {
+    const double t = chol_trace(l, [&](int i) { return Ls[i * (ld + 1)]; });
+    if (lane == 0) trace_s = t;
   }
-  for (int e = lane; e < l * l; e += 32) {
-    const int i = e % l, k = e / l;
-    if (i >= k) Gg[e] = LA(i, k);
+  __syncthreads();
+  const CholShift sh(d, trace_s, rel_shift);
+  for (int i = threadIdx.x; i < l; i += blockDim.x) Ls[i * (ld + 1)] += sh.shift;
+  __syncthreads();
+  // warp 0: the pivot of column c and its scaling, lane's rows c + lane + 32 s in x
+  auto finish = [&](int c, const double* x) {
+    const CholPivot p(__shfl_sync(kFullWarp, x[0], 0), sh);
+    if (lane == 0) {
+      Ls[c * (ld + 1)] = p.diag;
+      pivots[c] = p.r;
+      if (p.dead) atomicAdd(bad, 1);
+    }
+#pragma unroll
+    for (int s = 0; s < kSlots; ++s) {
+      const int i = c + lane + 32 * s;
+      if (i > c && i < l) Ls[i * ld + c] = p.dead ? 0.0 : x[s] * p.r;
+    }
+  };
+  if (warp == 0) {
+    double x[kSlots];
+#pragma unroll
+    for (int s = 0; s < kSlots; ++s) x[s] = lane + 32 * s < l ? Ls[(lane + 32 * s) * ld] : 0.0;
+    finish(0, x);
+  }
+  __syncthreads();
+  const int rows = warps - (warps >> 2) - 1, rank = warp - 2 - (warp >> 2);
+  for (int j = 0; j < l; ++j) {
+    if (warp == 0) {
+      const int c = j + 1;
+      if (c < l) {
+        double x[kSlots];
+        const double ljj = Ls[c * ld + j];
+#pragma unroll
+        for (int s = 0; s < kSlots; ++s) {
+          x[s] = 0.0;
+          if (c + 32 * s >= l) break;
+          const int i = min(c + lane + 32 * s, l - 1);
+          x[s] = fma(-Ls[i * ld + j], ljj, Ls[i * ld + c]);
+        }
+        finish(c, x);
+      }
+    } else if (warp == 1) {  // row j of X: the last update and the scaling
+      const double r = pivots[j], a = j > 0 ? Ls[j * ld + j - 1] : 0.0;
+      for (int c = lane; c <= j; c += 32) {
+        double x = Xs[j * ld + c];
+        if (c < j) x = fma(-a, Xs[(j - 1) * ld + c], x);
+        Xs[j * ld + c] = x * r;
+      }
+    } else if (warp & 3) {  // rows behind: X by row j - 1, L (columns j + 2 .. the diagonal) by column j
+      for (int i = j + 1 + rank; i < l; i += rows) {
+        double* Li = Ls + i * ld;
+        const double b = Li[j], a = j > 0 ? Li[j - 1] : 0.0;
+        for (int q = lane; q < i - 1; q += 32) {
+          const int k = q + 2;  // = j + 2 + q - j
+          double* p = q < j ? Xs + i * ld + q : Li + k;
+          const double m = q < j ? Xs[(j - 1) * ld + q] : Ls[k * ld + j];
+          *p = fma(q < j ? -a : -b, m, *p);
+        }
+      }
+    }
+    __syncthreads();
+  }
+  double* Xg = Rinv + d.g_off;  // Rinv = X^T, column-major: Rinv[c + i l] = X[i][c]
+  for (int i = warp; i < l; i += warps)
+    for (int c = lane; c < l; c += 32) Xg[c + i * l] = c <= i ? Xs[i * ld + c] : 0.0;
+}
+
+// Wide blocks: factor and inverse over a cluster, rows of 16 dealt out to its CTAs in turn, everything in their shared
+// memory and in place (a row's columns of L give way to those of Y, with X_i = L_ii^-1 Y_i at the end).  Panel K:
+//   the owner of row block K has factored the diagonal block and sent T = L_KK^-1 and Y_K to every CTA;
+//   each CTA forms P_i = A_iK T^T (= L_iK) and M_i = P_i T of its rows, and sends P to every CTA;
+//   A_iJ -= P_i P_J^T for K < J <= i, Y_iJ -= M_i Y_KJ for J < K, Y_iK = -M_i;
+// where the owner of block K + 1 lets four warps (one per quarter of the SM) update and factor that diagonal block
+// first, beside the update of its other rows.  Two cluster barriers a panel.  The pivots are still a chain, 16 times
+// 700 cycles a panel, but the l^3 / 3 multiply-adds run on the pipes of all CTAs.  The sums' order does not depend on
+// the cluster's size.
+// Measured, against a factorisation on one SM with the inverse in a second kernel: one block about 150 wide 357 ->
+// 180 us, two about 125 wide 214 -> 130, two about 190 wide 894 -> 257; CTMRG D = 6, chi = 128 134 -> 99 us a call.
+// One CTA is the faster up to 48 columns (its chain has no cluster barriers).
+constexpr int kPan = 16;
+__host__ __device__ constexpr int chol_cluster_elems(int l, int cluster) {
+  const int nb = (l + kPan - 1) / kPan, lp = nb * kPan, own = (nb + cluster - 1) / cluster;
+  return own * kPan * (lp + 2) + 2 * kPan * lp + 2 * kPan * kPan + 2 * own * kPan * kPan;
+}
+
+// threads 0..127: D (16 x 16, leading dimension ld, its first bs rows and columns used) -> T = L^-1 (row-major, zeros
+// above the diagonal, the identity in rows behind bs), as in chol_narrow_kernel
+__device__ __forceinline__ void chol_diag(double* D, int ld, int bs, double* T, double* pivots, const CholShift& sh,
+                                          int* bad) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  auto team = [] { asm volatile("bar.sync 1, 128;" ::: "memory"); };
+  for (int e = tid; e < kPan * kPan; e += 128) T[e] = e / kPan == e % kPan ? 1.0 : 0.0;
+  auto finish = [&](int c, double x) {
+    const CholPivot p(__shfl_sync(kFullWarp, x, 0), sh);
+    if (lane == 0) {
+      D[c * (ld + 1)] = p.diag;
+      pivots[c] = p.r;
+      if (p.dead) atomicAdd(bad, 1);
+    }
+    const int i = c + lane;
+    if (i > c && i < bs) D[i * ld + c] = p.dead ? 0.0 : x * p.r;
+  };
+  if (warp == 0) finish(0, lane < bs ? D[lane * ld] : 0.0);
+  team();
+  for (int j = 0; j < bs; ++j) {
+    if (warp == 0) {
+      const int c = j + 1;
+      if (c < bs) {
+        const int i = min(c + lane, bs - 1);
+        finish(c, fma(-D[i * ld + j], D[c * ld + j], D[i * ld + c]));
+      }
+    } else if (warp == 1) {
+      if (lane <= j) {
+        double x = T[j * kPan + lane];
+        if (lane < j) x = fma(-D[j * ld + j - 1], T[(j - 1) * kPan + lane], x);
+        T[j * kPan + lane] = x * pivots[j];
+      }
+    } else {
+      const int q = lane & 15;
+      for (int i = j + 1 + (warp - 2) * 2 + (lane >> 4); i < bs; i += 4)
+        if (q < i - 1) {
+          double* p = q < j ? T + i * kPan + q : D + i * ld + q + 2;
+          const double m = q < j ? T[(j - 1) * kPan + q] : D[(q + 2) * ld + j];
+          *p = fma(-(q < j ? D[i * ld + j - 1] : D[i * ld + j]), m, *p);
+        }
+    }
+    team();
+  }
+}
+
+__global__ void __launch_bounds__(512) chol_cluster_kernel(const CholDesc* __restrict__ descs,
+                                                           const double* __restrict__ G, double* __restrict__ Rinv,
+                                                           double rel_shift, int* __restrict__ bad) {
+  extern __shared__ __align__(16) double chol_sm[];
+  __shared__ double trace_s, pivots[kPan];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int P = int(cluster.num_blocks()), me = int(cluster.block_rank());
+  const CholDesc d = descs[blockIdx.x / P];
+  const int l = int(d.l), nb = (l + kPan - 1) / kPan, lp = nb * kPan, ld = lp + 2, most = (nb + P - 1) / P;
+  if (l == 0) return;  // the whole cluster
+  const int own = me < nb ? (nb - me + P - 1) / P : 0;  // row blocks me, me + P, ...
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
+  double* A = chol_sm;
+  double* Bs = A + most * kPan * ld;            // two of 16 x lp: Y_K left of block K, P^T right of it
+  double* Ts = Bs + 2 * kPan * lp;              // two of 16 x 16
+  double* Pc = Ts + 2 * kPan * kPan;            // P and M of this CTA's rows
+  double* Mc = Pc + most * kPan * kPan;
+  const double* Gg = G + d.g_off;
+  for (int k = warp; k < own * kPan; k += warps) {  // row i of the lower triangle from column i of G's upper one
+    const int gb = me + (k / kPan) * P, i = gb * kPan + k % kPan;
+    for (int c = lane; c < (gb + 1) * kPan; c += 32) A[k * ld + c] = i < l && c <= i ? Gg[c + i * l] : 0.0;
+  }
+  if (warp == 0) {
+    const double t = chol_trace(l, [&](int i) { return Gg[i + i * l]; });
+    if (lane == 0) trace_s = t;
+  }
+  __syncthreads();
+  const CholShift sh(d, trace_s, rel_shift);
+  for (int k = tid; k < own * kPan; k += blockDim.x) {
+    const int i = (me + (k / kPan) * P) * kPan + k % kPan;
+    if (i < l) A[k * ld + i] += sh.shift;
+  }
+  __syncthreads();
+  // factor diagonal block K (this CTA's row block b); T goes to its slot and in place of the block
+  auto diagonal = [&](int K) {
+    double* D = A + (K / P) * kPan * ld + K * kPan;
+    double* T = Ts + (K & 1) * kPan * kPan;
+    chol_diag(D, ld, min(kPan, l - K * kPan), T, pivots, sh, bad);
+    for (int e = tid; e < kPan * kPan; e += 128) D[(e / kPan) * ld + e % kPan] = T[e];
+  };
+  // T and Y of block K to the other CTAs
+  auto send = [&](int K) {
+    double* T = Ts + (K & 1) * kPan * kPan;
+    double* B = Bs + (K & 1) * kPan * lp;
+    const double* Y = A + (K / P) * kPan * ld;
+    const int half = K * kPan / 2;  // pairs of a row
+    for (int p = 0; p < P; ++p) {
+      double* Tp = cluster.map_shared_rank(T, p);
+      double* Bp = cluster.map_shared_rank(B, p);
+      if (p != me)
+        for (int e = tid; e < kPan * kPan; e += blockDim.x) Tp[e] = T[e];
+      for (int r = warp; r < kPan; r += warps)
+        for (int c = lane; c < half; c += 32)
+          reinterpret_cast<double2*>(Bp + r * lp)[c] = reinterpret_cast<const double2*>(Y + r * ld)[c];
+    }
+  };
+  if (me == 0) {
+    if (warp < 4) diagonal(0);
+    __syncthreads();
+    send(0);
+  }
+  cluster.sync();
+  for (int K = 0; K + 1 < nb; ++K) {
+    const double* T = Ts + (K & 1) * kPan * kPan;
+    double* B = Bs + (K & 1) * kPan * lp;
+    for (int e = tid; e < own * kPan * kPan; e += blockDim.x) {
+      const int b = e >> 8, c = (e >> 4) & 15, r = e & 15, gb = me + b * P;
+      if (gb <= K) continue;
+      const double* a = A + (b * kPan + r) * ld + K * kPan;
+      double acc = 0.0;
+      for (int k = 0; k <= c; ++k) acc = fma(a[k], T[c * kPan + k], acc);
+      Pc[(b * kPan + r) * kPan + c] = acc;
+      for (int p = 0; p < P; ++p) cluster.map_shared_rank(B, p)[c * lp + gb * kPan + r] = acc;
+    }
+    __syncthreads();
+    cluster.barrier_arrive();
+    for (int e = tid; e < own * kPan * kPan; e += blockDim.x) {
+      const int b = e >> 8, c = e & 15;
+      if (me + b * P <= K) continue;
+      const double* p = Pc + (e & ~15);
+      double acc = 0.0;
+      for (int k = c; k < kPan; ++k) acc = fma(p[k], T[k * kPan + c], acc);
+      Mc[e] = acc;
+    }
+    cluster.barrier_wait();
+    __syncthreads();
+    const int next = K + 1;
+    const bool mine = next % P == me;
+    if (mine && warp < 4) {
+      const int b = next / P;
+      for (int e = tid; e < kPan * kPan; e += 128) {
+        const int r = e / kPan, c = e % kPan;
+        if (c > r) continue;
+        double* p = A + (b * kPan + r) * ld + next * kPan + c;
+        const double* x = Pc + (b * kPan + r) * kPan;
+        const double* y = Pc + (b * kPan + c) * kPan;
+        double acc = *p;
+#pragma unroll
+        for (int k = 0; k < kPan; ++k) acc = fma(-x[k], y[k], acc);
+        *p = acc;
+      }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      diagonal(next);
+    } else if (!mine || (warp & 3)) {
+      const int team = mine ? warps - 4 - (warps - 4) / 4 : warps;
+      const int rank = mine ? warp - 5 - (warp - 4) / 4 : warp;
+      int at = 0;  // items (row pair, 32 columns) dealt out in turn over all row blocks
+      for (int b = 0; b < own; ++b) {
+        const int gb = me + b * P;
+        if (gb <= K) continue;
+        const int chunks = ((gb + 1) * kPan + 31) / 32, items = chunks * (kPan / 2);
+        for (int w = (rank - at % team + team) % team; w < items; w += team) {
+          const int r = (w / chunks) * 2, c = (w % chunks) * 32 + lane, cb = c / kPan;
+          if (c >= (gb + 1) * kPan || (gb == next && cb == next)) continue;
+          double* a0 = A + (b * kPan + r) * ld + c;
+          const int o = (b * kPan + r) * kPan;
+          if (cb == K) {
+            a0[0] = -Mc[o + c % kPan];
+            a0[ld] = -Mc[o + kPan + c % kPan];
+            continue;
+          }
+          const double* co = (cb < K ? Mc : Pc) + o;
+          double x = a0[0], y = a0[ld];
+#pragma unroll
+          for (int k = 0; k < kPan; ++k) {
+            const double m = B[k * lp + c];
+            x = fma(-co[k], m, x);
+            y = fma(-co[kPan + k], m, y);
+          }
+          a0[0] = x;
+          a0[ld] = y;
+        }
+        at += items;
+      }
+    }
+    __syncthreads();
+    if (mine) send(next);
+    cluster.sync();
+  }
+  // X_i = T_i [Y_i, I]; Rinv = X^T, column-major: Rinv[c + i l] = X[i][c]
+  double* Xg = Rinv + d.g_off;
+  for (int k = warp; k < own * kPan; k += warps) {
+    const int b = k / kPan, r = k % kPan, gb = me + b * P, i = gb * kPan + r;
+    if (i >= l) continue;
+    const double* rows = A + b * kPan * ld;
+    for (int c = lane; c < l; c += 32) {
+      double acc = 0.0;
+      if (c < gb * kPan) {
+        for (int q = 0; q <= r; ++q) acc = fma(rows[r * ld + gb * kPan + q], rows[q * ld + c], acc);
+      } else if (c <= i) {
+        acc = rows[r * ld + c];
+      }
+      Xg[c + i * l] = acc;
+    }
   }
 }
 
@@ -419,8 +720,7 @@ __global__ void __launch_bounds__(32) chol_warp_kernel(const CholDesc* __restric
 // the single-CTA elimination (x_k = r_k * (1 / L_kk), then r_i -= L_ik x_k for i > k), so
 // both give the same bits; lane t keeps r_i for i = t + 32 j in registers (j < T).
 constexpr int kTrinvCols = 8;
-constexpr int kTrinvStageL = 150;  // trailing factor staged in shared memory up to this width (176 KB)
-template <int T, bool kStaged>
+template <int T>
 __global__ void __launch_bounds__(32 * kTrinvCols) trinv_kernel(const CholDesc* __restrict__ descs, int chunks,
                                                                  const double* __restrict__ G,
                                                                  double* __restrict__ Rinv) {
@@ -434,13 +734,6 @@ __global__ void __launch_bounds__(32 * kTrinvCols) trinv_kernel(const CholDesc* 
   const double* L = G + d.g_off;
   double* R = Rinv + d.g_off;
   for (int k = c0 + int(threadIdx.x); k < l; k += blockDim.x) inv_diag[k - c0] = 1.0 / L[k + int64_t(k) * l];
-  // staged: column k of the trailing factor at Ls + (k - c0) * lt, rows c0 .. l-1
-  double* Ls = tsm + lt;
-  if (kStaged)
-    for (int e = threadIdx.x; e < lt * lt; e += blockDim.x) {
-      const int i = e % lt, k = e / lt;
-      Ls[e] = i >= k ? L[(c0 + i) + int64_t(c0 + k) * l] : 0.0;
-    }
   __syncthreads();
   const int lane = threadIdx.x & 31, c = c0 + int(threadIdx.x >> 5);
   if (c >= l) return;
@@ -454,15 +747,13 @@ __global__ void __launch_bounds__(32 * kTrinvCols) trinv_kernel(const CholDesc* 
     for (int j = 0; j < T; ++j)
       if (j == slot) v = r[j];
     const double xk = __shfl_sync(0xffffffffu, v, k & 31) * inv_diag[k - c0];
-    // column k of L: staged rows start at c0, global rows at 0
-    const double* Lk = kStaged ? Ls + int64_t(k - c0) * lt : L + int64_t(k) * l;
-    const int base = kStaged ? c0 : 0;
+    const double* Lk = L + int64_t(k) * l;
 #pragma unroll
     for (int j = 0; j < T; ++j) {
       if (32 * j + 31 < k) continue;  // warp-uniform: rows of this slot are all finished
       const int i = lane + 32 * j;
       if (i == k) r[j] = xk;
-      else if (i > k && i < l) r[j] = fma(-(kStaged ? Lk[i - base] : __ldg(Lk + i)), xk, r[j]);
+      else if (i > k && i < l) r[j] = fma(-__ldg(Lk + i), xk, r[j]);
     }
   }
   // row c of Rinv (= column c of X): Rinv[c + i l] = X[i][c], zero for i < c
@@ -495,46 +786,49 @@ void launch_chol_inv(const CholDesc* d_descs, int n, int64_t max_l, double* G, d
     count_launch();
     return;
   }
-  if (max_l <= kCholWarpL) {
-    static std::once_flag wattr;
-    std::call_once(wattr, [] {
-      cudaFuncSetAttribute(chol_warp_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           kCholWarpL * (kCholWarpL | 1) * int(sizeof(double)));
-    });
+  if (max_l <= kCholNarrow) {
+    constexpr int kBytes = 2 * kCholNarrow * (kCholNarrow | 1) * int(sizeof(double));
+    static_assert(kBytes <= 48 * 1024);
     const int lw = int(max_l);
-    chol_warp_kernel<<<n, 32, lw * (lw | 1) * int(sizeof(double)), s>>>(d_descs, G, rel_shift, bad);
-  } else {
-    // 1024 threads: the rank-1 update of a column is spread thinnest (measured: 128 / 256 threads per block
-    // made the CTM step's factorisations 55 % slower at widths 48-130)
-    const int lc = int(std::min<int64_t>(max_l, kCapChol));
-    chol_inv_kernel<false><<<n, 1024, lc * (lc | 1) * int(sizeof(double)), s>>>(d_descs, G, Rinv, rel_shift, bad,
-                                                                                  kCapChol);
+    chol_narrow_kernel<<<n, lw <= 32 ? 256 : 512, 2 * lw * (lw | 1) * int(sizeof(double)), s>>>(d_descs, G, Rinv,
+                                                                                              rel_shift, bad);
+    count_launch();
+    return;
   }
+  if (max_l <= kCholCluster) {
+    const int cluster = max_l <= 4 * kPan ? 4 : 8;
+    const int bytes = chol_cluster_elems(int(max_l), cluster) * int(sizeof(double));
+    static std::once_flag cattr;
+    std::call_once(cattr, [] {
+      cudaFuncSetAttribute(chol_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           chol_cluster_elems(kCholCluster, 8) * int(sizeof(double)));
+    });
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(unsigned(n) * unsigned(cluster));
+    cfg.blockDim = dim3(512);
+    cfg.dynamicSmemBytes = size_t(bytes);
+    cfg.stream = s;
+    cudaLaunchAttribute at{};
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim = {unsigned(cluster), 1, 1};
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, chol_cluster_kernel, d_descs, static_cast<const double*>(G), Rinv,
+                                             rel_shift, bad);
+    if (e != cudaSuccess) throw std::runtime_error(std::string("Cholesky launch: ") + cudaGetErrorString(e));
+    count_launch();
+    return;
+  }
+  chol_inv_kernel<false><<<n, 1024, kBytesChol, s>>>(d_descs, G, Rinv, rel_shift, bad, kCapChol);
   count_launch();
   const int chunks = int((max_l + kTrinvCols - 1) / kTrinvCols);
-  if (max_l <= kTrinvStageL) {
-    static std::once_flag tattr;
-    std::call_once(tattr, [] {
-      for (auto f : {trinv_kernel<4, true>, trinv_kernel<8, true>})
-        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             int(sizeof(double)) * kTrinvStageL * (kTrinvStageL + 1));
-    });
-    const size_t sm = sizeof(double) * size_t(max_l) * size_t(max_l + 1);
-    if (max_l <= 128)
-      trinv_kernel<4, true><<<n * chunks, 32 * kTrinvCols, sm, s>>>(d_descs, chunks, G, Rinv);
-    else
-      trinv_kernel<8, true><<<n * chunks, 32 * kTrinvCols, sm, s>>>(d_descs, chunks, G, Rinv);
-  } else {
-    const size_t sm = sizeof(double) * size_t(max_l);
-    if (max_l <= 256)
-      trinv_kernel<8, false><<<n * chunks, 32 * kTrinvCols, sm, s>>>(d_descs, chunks, G, Rinv);
-    else if (max_l <= 512)
-      trinv_kernel<16, false><<<n * chunks, 32 * kTrinvCols, sm, s>>>(d_descs, chunks, G, Rinv);
-    else if (max_l <= 1024)
-      trinv_kernel<32, false><<<n * chunks, 32 * kTrinvCols, sm, s>>>(d_descs, chunks, G, Rinv);
-    else
-      trinv_kernel<64, false><<<n * chunks, 32 * kTrinvCols, sm, s>>>(d_descs, chunks, G, Rinv);
-  }
+  const size_t sm = sizeof(double) * size_t(max_l);
+  if (max_l <= 512)
+    trinv_kernel<16><<<n * chunks, 32 * kTrinvCols, sm, s>>>(d_descs, chunks, G, Rinv);
+  else if (max_l <= 1024)
+    trinv_kernel<32><<<n * chunks, 32 * kTrinvCols, sm, s>>>(d_descs, chunks, G, Rinv);
+  else
+    trinv_kernel<64><<<n * chunks, 32 * kTrinvCols, sm, s>>>(d_descs, chunks, G, Rinv);
   count_launch();
 }
 
