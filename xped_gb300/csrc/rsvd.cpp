@@ -51,12 +51,24 @@ class Staging {
 
 double* alloc_d(int64_t n) { return static_cast<double*>(dev_alloc(sizeof(double) * size_t(std::max<int64_t>(n, 1)))); }
 
-// Grouped FP64 GEMM of the sketch pipeline.  The k range of each tile is split so that about eight CTAs
-// per SM run: few tiles (the l x l Gram matrices) would leave SMs idle, and the products' two or three
-// tiles per SM, some with few live columns, end at different times (six blocks of 134 to 1024 times 37
-// columns, ideal 144 us: 230 us at two CTAs per SM, 181 at five, 173 at eight, 168 at twelve).  The
-// partial tiles land in a workspace and one reduce launch adds them in a fixed order (deterministic
-// result).  With autotuning on, the
+// CTAs per SM that the k ranges of a product's tiles are split for.  A tile's time grows with its k, so what the SMs
+// wait for at the end is about half the longest tile: where that is more than an eighth of an SM's share of the work
+// (few tiles, as the l x l Gram matrices; or two or three long ones per SM) the ranges are cut for eight CTAs per SM,
+// else the partial tiles and their reduction cost more than they save.  Measured: six blocks of 134 to 1024 times 37
+// columns (longest tile 0.36 of a share) 230 us unsplit, 181 for five CTAs, 173 for eight, 168 for twelve; four of 300
+// to 2000 times 64 (0.18) 769 and 744; eight products of nine blocks 16 to 281 (0.18) 1000 unsplit and 1068 split.
+int split_waves(const std::vector<xgb_gemm_desc>& d, int tile) {
+  double share = 0, longest = 0;
+  for (const auto& g : d) {
+    share += double((g.m + tile - 1) / tile) * double((g.n + tile - 1) / tile) * double(g.k);
+    if (g.m > 0 && g.n > 0) longest = std::max(longest, double(g.k));
+  }
+  share /= num_sms() > 0 ? num_sms() : 152;
+  return longest > 0.25 * share ? 8 : 0;
+}
+
+// Grouped FP64 GEMM of the sketch pipeline.  The partial tiles of split k ranges land in a workspace
+// and one reduce launch adds them in a fixed order (deterministic result).  With autotuning on, the
 // tile edge and the split target are the tuned ones of the list's size bucket.
 // allow_tc (callers running the FP64-accurate tensor-core form): the autotuner may also route the list
 // to that form when it measures it faster (built-in rule: average k >= 64), computing C in full.
@@ -74,7 +86,8 @@ void grouped_gemm(const std::vector<xgb_gemm_desc>& d, const double* A, const do
       return;
     }
   }
-  const F64Config fallback{choose_f64_tile(d.data(), int(d.size())), 8};
+  const int tile = choose_f64_tile(d.data(), int(d.size()));
+  const F64Config fallback{tile, split_waves(d, tile)};
   const F64Config cfg = gemm_f64_config(d.data(), int(d.size()), A, B, fallback, s);
   const F64Plan p = plan_gemm_f64(d.data(), int(d.size()), cfg, shape);
   double flops = 0;
