@@ -218,8 +218,8 @@ int tune_gemm_f64(const xgb_gemm_desc* d, int n, const double* A, const double* 
           dev_alloc(sizeof(unsigned long long) * size_t(std::max<int64_t>(op.rowmax, 1))));
       auto* ap = static_cast<unsigned char*>(dev_alloc(size_t(std::max<int64_t>(op.a_bytes, 16))));
       auto* bp = static_cast<unsigned char*>(dev_alloc(size_t(std::max<int64_t>(op.b_bytes, 16))));
-      launch_gemm_oz(dd, dg, dk, int(op.tasks.size()), dt, int(op.tiles.size()), dr, int(op.red.size()), op.slots,
-                     A, B, rm, op.rowmax, ap, bp, scratch, 1.0, 0.0, s);
+      launch_gemm_oz(dd, dg, dk, int(op.tasks.size()), op.pack_cluster, dt, int(op.tiles.size()), dr, int(op.red.size()), op.slots,
+                     A, B, rm, ap, bp, scratch, 1.0, 0.0, s);
       dev_free(rm);
       dev_free(ap);
       dev_free(bp);

@@ -6,7 +6,7 @@
 // integers |m_1| <= 128 and |m_s| <= 64 for s >= 2; every column of op(B) likewise (2^f_j).  A slice
 // m_s 2^(-7 s) is exact in BF16, the product of two slices is exact in FP32, and all products of a
 // "level" L = s + t share the unit 2^(-7 L).  Per k value a level adds at most 2 x 128 x 64 + 5 x 64 x 64
-// = 36864 units, so a sum over 448 k values (14 K slices) stays below 2^24 and is exact in the FP32
+// = 36864 units, so a sum over 448 k values (28 K slices) stays below 2^24 and is exact in the FP32
 // tensor-memory accumulator whatever order the tensor core adds in.  The row and column scales
 // 2^(e_i + f_j) go into the exponent field when the tile is stored.  This is the slicing scheme of
 // Ozaki, Ogita, Oishi and Rump ("Error-free transformations of matrix multiplication by using fast
@@ -18,50 +18,57 @@
 // maxima, scales and slices are integer operations on the IEEE bits.
 //
 // Kernels (one launch each, all groups of the list):
-//  * oz_rowmax_kernel: per 128-row (A) / 64-row (B) x 32-K chunk, the largest |entry| of every row
-//    into a max over the whole k range (atomicMax on the IEEE bits of a non-negative double);
-//  * oz_pack_kernel: the seven slices of every chunk as BF16 in the K-major, unswizzled canonical
-//    layout the MMA reads (8-row x 16-byte core matrices), zero padded past the block edges; the
-//    slices come from integer arithmetic on the FP64 significand (|x| rounded to 49 bits below the
-//    row's scale, balanced digits, every slice with the sign of its entry);
-//  * oz_gemm_kernel: one CTA (10 warps) per 128 x 64 output tile and K range.  Warp 8 streams the
-//    slices of each 32-wide K slice of the tile's rows and columns into a 2-stage shared-memory ring
-//    (84 KB per stage, bulk copies counted on mbarriers); warp 9 issues, per 16-deep k step, the 28
+//  * oz_pack_kernel: the row scales, and the seven slices of every entry as BF16 in the K-major,
+//    unswizzled canonical layout the MMA reads (8-row x 16-byte core matrices), zero padded past the
+//    block edges; the slices come from integer arithmetic on the FP64 significand (|x| rounded to 49
+//    bits below the row's scale, balanced digits, every slice with the sign of its entry);
+//  * oz_gemm_kernel: one CTA (18 warps) per 128 x 64 output tile and K range.  Warp 16 streams the
+//    slices of each 16-wide K slice of the tile's rows and columns into a 5-stage shared-memory ring
+//    (42 KB per stage, bulk copies counted on mbarriers); warp 17 issues, per K slice, the 28
 //    BF16 MMAs of the slice pairs with s + t <= 8 into seven 64-column TMEM accumulators (one per
-//    level, 448 of 512 columns); after every fourteen K slices (the exactness bound) and at the end
-//    of the range warps 0-7 read the seven levels and add them into double-FP32 (hi + lo) register
-//    sums, then the next chunk starts from zero.  The slice rounding (2^-50 of the row / column
-//    scale), the dropped pairs (s + t > 8) and the double-FP32 sums bound the error of an element by
-//    a small multiple of 2^-49 k max_k |a_ik| max_k |b_kj|: about 5e-14 of ||C|| for Gaussian blocks,
-//    against ~1e-15 for an FP64 dot product and ~3e-7 for 3xTF32.
+//    level, 448 of 512 columns); after every 28 K slices (the exactness bound) and at the end of the
+//    range warps 0-15 read the seven levels and add them into double-FP32 (hi + lo) register sums, two
+//    values per instruction, and the next chunk starts from zero on the levels that have been read.
+//    The slice rounding (2^-50 of the row / column scale), the dropped pairs (s + t > 8) and the
+//    double-FP32 sums bound the error of an element by a small multiple of
+//    2^-49 k max_k |a_ik| max_k |b_kj|: about 5e-14 of ||C|| for Gaussian blocks, against ~1e-15 for
+//    an FP64 dot product and ~3e-7 for 3xTF32.
+// Bound by the MMA rate: nine blocks of 144 to 2464 take 2042 us with 8 draining warps, a 2-stage ring
+// and MMAs in the order in which they open the levels, 1640 now (1.16 ms at the rate of a plain BF16
+// product of 28 times the size; slicing 0.24, drains and epilogues about 0.15).
 //
 // Every mbarrier wait is bounded; on timeout the CTA records an error flag (shared with the 3xTF32
 // kernel, xgb_gemm_tc_status), skips the epilogue and still frees its TMEM.
-#include <cuda_bf16.h>
+#include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
 #include <cstdint>
 #include <mutex>
+#include <stdexcept>
+#include <string>
 
 #include "kernels.hpp"
+
+namespace cg = cooperative_groups;
 
 namespace xgb {
 namespace {
 
-constexpr int OM = 128, ON = 64, OK = 32;          // output tile rows / columns, K per slice
+constexpr int OM = 128, ON = 64, OK = 16;          // output tile rows / columns, K per slice
 constexpr int kPieces = 7, kBits = 7;               // seven 7-bit slices per entry
 constexpr int kLevels = kPieces;                    // levels s + t = 2 .. 8 (1-based slices)
-constexpr int kChunk = 14;                          // K slices per exact TMEM accumulation (448 x 36864 < 2^24)
-constexpr int kMinSplit = 4;                        // smallest K range of a split-K CTA, in K slices
-constexpr int kAPieceBytes = OM * OK * 2;           // 8 KB
-constexpr int kBPieceBytes = ON * OK * 2;           // 4 KB
-constexpr int kOzStageBytes = kPieces * (kAPieceBytes + kBPieceBytes);  // 84 KB
-constexpr int kOzStages = 2;
+constexpr int kChunk = 28;                          // K slices per exact TMEM accumulation (448 x 36864 < 2^24)
+constexpr int kMinSplit = 8;                        // smallest K range of a split-K CTA, in K slices
+constexpr int kAPieceBytes = OM * OK * 2;           // 4 KB
+constexpr int kBPieceBytes = ON * OK * 2;           // 2 KB
+constexpr int kOzStageBytes = kPieces * (kAPieceBytes + kBPieceBytes);  // 42 KB
+constexpr int kOzStages = 5;
 constexpr int kOzSmem = kOzStages * kOzStageBytes + 1024;
 constexpr uint32_t kOzTmemCols = 512;               // 7 levels x 64 columns used
-constexpr int kOzWarps = 10, kOzThreads = kOzWarps * 32;
-constexpr int kOzProducer = 8, kOzMma = 9, kOzDrainWarps = 8;
+constexpr int kOzDrainWarps = 16, kOzProducer = kOzDrainWarps, kOzMma = kOzDrainWarps + 1;
+constexpr int kOzWarps = kOzDrainWarps + 2, kOzThreads = kOzWarps * 32;
+constexpr int kDrainCols = ON / (kOzDrainWarps / 4);  // columns of a drain warp
 constexpr long long kOzSpin = 1ll << 26;
 constexpr uint32_t kSboBytes = 128;                 // next 8-row group
 // A: seven separate 128-row pieces.  B: the seven 64-row pieces stacked into one 448-row operand (row
@@ -126,48 +133,45 @@ __device__ __forceinline__ void mma_bf16_oz(uint32_t tmem_d, uint64_t adesc, uin
       "l"(adesc), "l"(bdesc), "r"(oz_idesc<NC>()), "r"(acc));
 }
 
+// 16 columns of this warp's 32 lanes; the registers hold them after tcgen05.wait::ld
+__device__ __forceinline__ void tmem_load16(uint32_t addr, uint32_t* v) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]), "=r"(v[8]),
+        "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
+      : "r"(addr));
+}
+
+// waits for the loads; the values pass through so that no use moves ahead of it
+__device__ __forceinline__ void tmem_wait16(uint32_t* v) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
+               :
+               : "memory");
+}
+
+// two FP32 additions at once, each rounded as __fadd_rn
+__device__ __forceinline__ unsigned long long pair(uint32_t a, uint32_t b) {
+  return uint64_t(a) | uint64_t(b) << 32;
+}
+__device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ unsigned long long sub2(unsigned long long a, unsigned long long b) {
+  unsigned long long d;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+
 __device__ __forceinline__ void commit_to(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(s_u32(bar))
                : "memory");
 }
 
-// ----------------------------------------------------------------------------- row scales
-// task: (group, tile of OM rows of op(A) or ON rows of op(B)^T, K slice, which)
-__global__ void __launch_bounds__(256) oz_rowmax_kernel(const xgb_gemm_desc* __restrict__ descs,
-                                                         const OzGroup* __restrict__ groups,
-                                                         const TcPackTask* __restrict__ tasks,
-                                                         const double* __restrict__ A, const double* __restrict__ B,
-                                                         unsigned long long* __restrict__ rowmax) {
-  // |x| as IEEE bits: for non-negative doubles the integer order is the numeric order
-  __shared__ unsigned long long X[OM][OK + 1];
-  const TcPackTask t = tasks[blockIdx.x];
-  const xgb_gemm_desc d = descs[t.g];
-  const OzGroup gr = groups[t.g];
-  const bool isB = t.which != 0;
-  const bool sb = isB != (gr.swap != 0);  // the rows of this role are op(B)^T's (columns of op(B))
-  const double* src = sb ? B : A;
-  const int64_t off = sb ? d.b_off : d.a_off, ld = sb ? d.ldb : d.lda;
-  const int64_t rows = sb ? d.n : d.m;
-  const int tr = isB ? ON : OM;
-  const bool rowfast = sb ? d.trans_b != 0 : d.trans_a == 0;
-  const int64_t r0 = int64_t(t.tile) * tr, k0 = int64_t(t.slice) * OK;
-  for (int e = threadIdx.x; e < tr * OK; e += 256) {
-    int r, k;
-    if (rowfast) { r = e % tr; k = e / tr; } else { k = e % OK; r = e / OK; }
-    const int64_t gr_ = r0 + r, gk = k0 + k;
-    double x = 0.0;
-    if (gr_ < rows && gk < d.k) x = rowfast ? src[off + gr_ + gk * ld] : src[off + gk + gr_ * ld];
-    X[r][k] = static_cast<unsigned long long>(__double_as_longlong(x)) & 0x7FFFFFFFFFFFFFFFull;
-  }
-  __syncthreads();
-  for (int r = threadIdx.x; r < tr; r += 256) {
-    if (r0 + r >= rows) continue;
-    unsigned long long m = 0;
-    for (int k = 0; k < OK; ++k) m = m > X[r][k] ? m : X[r][k];
-    if (m) atomicMax(rowmax + (isB ? gr.b_rowmax : gr.a_rowmax) + r0 + r, m);
-  }
-}
-
+// ----------------------------------------------------------------------------- row scales and slices
 // exponent e with |x| < 2^e for every entry of the row, from the bits of its largest |entry|
 // m = f 2^e, f in [0.5, 1): the biased exponent less 1022.  A zero row, or one whose largest entry
 // is subnormal (its slices are all zero), gets 0.
@@ -176,89 +180,139 @@ __device__ __forceinline__ int row_scale(unsigned long long bits) {
   return be == 0 ? 0 : be - 1022;
 }
 
-// seven balanced base-128 digits of x relative to 2^e (|x| < 2^e):
-// x = 2^e sum_s m_s 2^(-7 s) + O(2^(e - 50)), |m_1| <= 128, |m_s| <= 64 for s >= 2
-__device__ __forceinline__ void slice7(double x, int e, float* out) {
-  const long long bits = __double_as_longlong(x);
+// Seven balanced base-128 digits of x relative to 2^e (|x| < 2^e): x = 2^e sum_s m_s 2^(-7 s) + O(2^(e - 50)),
+// |m_1| <= 128, |m_s| <= 64 for s >= 2.  Adding 64 at each of the six lower digits turns the balanced digits of |x| into
+// the plain 7-bit fields of one integer: lo holds fields 7, 6, 5, 4 (four of 7 bits), hi fields 3, 2 and the leading one.
+__device__ __forceinline__ void digits7(double x, int e, uint32_t& lo, uint32_t& hi) {
+  const unsigned long long bits = static_cast<unsigned long long>(__double_as_longlong(x));
   const int ex = int((bits >> 52) & 0x7FF);
-  const bool neg = bits < 0;
-  long long q = 0;
+  unsigned long long q = 64ull * (1 + (1ull << 7) + (1ull << 14) + (1ull << 21) + (1ull << 28) + (1ull << 35));
   if (ex != 0) {  // normal numbers (subnormals are below every slice of any realistic row)
-    const unsigned long long mant = (static_cast<unsigned long long>(bits) & ((1ull << 52) - 1)) | (1ull << 52);
+    const unsigned long long mant = (bits & ((1ull << 52) - 1)) | (1ull << 52);
     // x = mant 2^(ex - 1075); |x| rounded to the nearest multiple of 2^(e - 49) (ties up): shift right
-    // by sh = e - 49 - (ex - 1075) >= 4 (|x| < 2^e) with one guard bit; q <= 2^49
+    // by sh = e - 49 - (ex - 1075) >= 4 (|x| < 2^e) with one guard bit; at most 2^49
     const int sh = e - 49 - (ex - 1075);
-    q = sh >= 64 ? 0ll : static_cast<long long>(((mant >> (sh - 1)) + 1ull) >> 1);
+    if (sh < 64) q += ((mant >> (sh - 1)) + 1ull) >> 1;
   }
-  // lowest digit first: m in [-64, 63] and the carry moves into q; what is left after six digits is
-  // the leading digit, round(q / 2^42) <= 128
-  int m[kPieces];
-#pragma unroll
-  for (int s = kPieces; s >= 2; --s) {
-    int dg = int(q & ((1ll << kBits) - 1));
-    if (dg >= 64) dg -= 128;
-    m[s - 1] = dg;
-    q = (q - dg) >> kBits;
-  }
-  m[0] = int(q);
-#pragma unroll
-  for (int s = 1; s <= kPieces; ++s) {
-    const float v = __fmul_rn(float(neg ? -m[s - 1] : m[s - 1]), __int_as_float((127 - kBits * s) << 23));  // x 2^(-7 s)
-    out[s - 1] = v;
-  }
+  lo = uint32_t(q);
+  hi = uint32_t(q >> 28);
 }
 
+// digit s (1-based) times 2^(-7 s) as a float, from its 7-bit (leading: 8-bit) field: the field below 2^23 in a
+// significand, and one exact multiply-add that takes the offset off and scales
+template <int S>
+__device__ __forceinline__ uint32_t digit_float(uint32_t lo, uint32_t hi) {
+  constexpr float k = 1.0f / float(1ull << (7 * S));
+  constexpr float c = -(8388608.0f + (S == 1 ? 0.0f : 64.0f)) * k;
+  const uint32_t f = S == 1 ? hi >> 14 : S <= 3 ? (hi >> (7 * (3 - S))) & 127u : (lo >> (7 * (7 - S))) & 127u;
+  return __float_as_uint(fmaf(__uint_as_float(0x4B000000u | f), k, c));
+}
+
+// slice S of eight consecutive entries as BF16 (exact: at most 8 significant bits, the upper half of the float), with
+// the entries' signs
+template <int S>
+__device__ __forceinline__ void store_slice(unsigned char* at, int stride, const uint32_t* lo, const uint32_t* hi,
+                                            const uint32_t* sign) {
+  uint32_t w[4];
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    w[j] = __byte_perm(digit_float<S>(lo[2 * j], hi[2 * j]), digit_float<S>(lo[2 * j + 1], hi[2 * j + 1]), 0x7632) ^ sign[j];
+  *reinterpret_cast<uint4*>(at + (S - 1) * stride) = make_uint4(w[0], w[1], w[2], w[3]);
+  if constexpr (S < kPieces) store_slice<S + 1>(at, stride, lo, hi, sign);
+}
+
+// One cluster per (group, tile of OM rows of op(A) or ON rows of op(B)^T): its CTAs share the K range in groups of
+// eight, a thread a row and every second or fourth group.  The row maxima (on the IEEE bits: integer order is numeric
+// order) meet in distributed shared memory; then the same entries are read again, from L2, and sliced.  Bound by the
+// 14 bytes written per entry for large operands, by the reads' latency for small ones.
+// Measured (nine blocks of 100 to 1729 squared, both operands): 233 us as a maximum kernel (with atomics) and a slicing
+// kernel with 64-bit digit arithmetic, 114 now.
 __global__ void __launch_bounds__(256) oz_pack_kernel(const xgb_gemm_desc* __restrict__ descs,
                                                        const OzGroup* __restrict__ groups,
                                                        const TcPackTask* __restrict__ tasks,
                                                        const double* __restrict__ A, const double* __restrict__ B,
-                                                       const unsigned long long* __restrict__ rowmax,
+                                                       unsigned long long* __restrict__ rowmax,
                                                        unsigned char* __restrict__ apack,
                                                        unsigned char* __restrict__ bpack) {
-  __shared__ double X[OM][OK + 1];
-  __shared__ int E[OM];
-  const TcPackTask t = tasks[blockIdx.x];
+  __shared__ unsigned long long part[256], own[OM];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int P = int(cluster.num_blocks()), me = int(cluster.block_rank());
+  const TcPackTask t = tasks[blockIdx.x / unsigned(P)];
   const xgb_gemm_desc d = descs[t.g];
   const OzGroup gr = groups[t.g];
   const bool isB = t.which != 0;
   const bool sb = isB != (gr.swap != 0);  // the rows of this role are op(B)^T's (columns of op(B))
-  const double* src = sb ? B : A;
-  const int64_t off = sb ? d.b_off : d.a_off, ld = sb ? d.ldb : d.lda;
-  const int64_t rows = sb ? d.n : d.m;
-  const int tr = isB ? ON : OM;
+  const int64_t ld = sb ? d.ldb : d.lda, rows = sb ? d.n : d.m;
   const bool rowfast = sb ? d.trans_b != 0 : d.trans_a == 0;
-  const int64_t r0 = int64_t(t.tile) * tr, k0 = int64_t(t.slice) * OK;
-  for (int e = threadIdx.x; e < tr * OK; e += 256) {
-    int r, k;
-    if (rowfast) { r = e % tr; k = e / tr; } else { k = e % OK; r = e / OK; }
-    const int64_t gr_ = r0 + r, gk = k0 + k;
-    double x = 0.0;
-    if (gr_ < rows && gk < d.k) x = rowfast ? src[off + gr_ + gk * ld] : src[off + gk + gr_ * ld];
-    X[r][k] = x;
+  const int tr = isB ? ON : OM, r = int(threadIdx.x) % tr, q = int(threadIdx.x) / tr, nq = 256 / tr;
+  const int64_t row = int64_t(t.tile) * tr + r;
+  const bool live = row < rows;
+  const double* src = (sb ? B + d.b_off : A + d.a_off) + (live ? (rowfast ? row : row * ld) : 0);
+  const int64_t step = rowfast ? ld : 1;
+  const int n8 = gr.slices * (OK / 8), per = (n8 + P - 1) / P, first = min(n8, me * per) + q, last = min(n8, (me + 1) * per);
+  auto load8 = [&](int g, double* x) {
+    const int64_t k = int64_t(g) * 8;
+    const double* at = src + k * step;
+    if (live && k + 8 <= d.k) {
+      if (!rowfast && (reinterpret_cast<uintptr_t>(at) & 15) == 0) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const double2 v = __ldg(reinterpret_cast<const double2*>(at) + j);
+          x[2 * j] = v.x;
+          x[2 * j + 1] = v.y;
+        }
+        return;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = __ldg(at + j * step);
+      return;
+    }
+#pragma unroll
+    for (int j = 0; j < 8; ++j) x[j] = live && k + j < d.k ? __ldg(at + j * step) : 0.0;
+  };
+  unsigned long long m = 0;
+  for (int g = first; g < last; g += nq) {
+    double x[8];
+    load8(g, x);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      const unsigned long long b = static_cast<unsigned long long>(__double_as_longlong(x[j])) & 0x7FFFFFFFFFFFFFFFull;
+      m = m > b ? m : b;
+    }
   }
-  for (int r = threadIdx.x; r < tr; r += 256)
-    E[r] = (r0 + r < rows) ? row_scale(rowmax[(isB ? gr.b_rowmax : gr.a_rowmax) + r0 + r]) : 0;
+  part[threadIdx.x] = m;
   __syncthreads();
-  // slice block of this (tile, K slice): kPieces pieces of tr x OK BF16, each in canonical layout
+  if (int(threadIdx.x) < tr) {
+    for (int p = 1; p < nq; ++p) m = m > part[p * tr + r] ? m : part[p * tr + r];
+    own[r] = m;
+  }
+  cluster.sync();
+  if (int(threadIdx.x) < tr) {
+    for (int p = 0; p < P; ++p) {
+      const unsigned long long o = cluster.map_shared_rank(own, p)[r];
+      m = m > o ? m : o;
+    }
+    part[r] = m;
+    if (me == 0 && live) rowmax[(isB ? gr.b_rowmax : gr.a_rowmax) + row] = m;
+  }
+  cluster.sync();  // `own` of every CTA has been read
+  const int e = row_scale(part[r]);
+  // block of one (tile, K slice): kPieces pieces of tr x OK BF16, each in canonical layout
   const int piece_bytes = isB ? kBPieceBytes : kAPieceBytes;
   const int piece_stride = isB ? int(kBPieceStride) : kAPieceBytes;
   const uint32_t lbo = isB ? kLboB : kLboA;
-  unsigned char* base = (isB ? bpack + gr.b_pack : apack + gr.a_pack) +
-                        (int64_t(t.tile) * gr.slices + t.slice) * int64_t(kPieces) * piece_bytes;
-  for (int e = threadIdx.x; e < tr * (OK / 8); e += 256) {
-    const int r = e % tr, kq = e / tr;  // one 16-byte core-matrix row: 8 consecutive K of row r
-    __nv_bfloat16 pc[kPieces][8];
+  unsigned char* base = (isB ? bpack + gr.b_pack : apack + gr.a_pack) + int64_t(t.tile) * gr.slices * (kPieces * piece_bytes);
+  for (int g = first; g < last; g += nq) {
+    double x[8];
+    load8(g, x);
+    uint32_t lo[8], hi[8], sign[4];
 #pragma unroll
-    for (int kk = 0; kk < 8; ++kk) {
-      float v[kPieces];
-      slice7(X[r][kq * 8 + kk], E[r], v);
+    for (int j = 0; j < 8; ++j) digits7(x[j], e, lo[j], hi[j]);
 #pragma unroll
-      for (int s = 0; s < kPieces; ++s) pc[s][kk] = __float2bfloat16_rn(v[s]);  // exact: <= 7 significant bits
-    }
-    const uint32_t bo = uint32_t(kq) * lbo + uint32_t(r >> 3) * kSboBytes + uint32_t(r & 7) * 16;
-#pragma unroll
-    for (int s = 0; s < kPieces; ++s)
-      *reinterpret_cast<uint4*>(base + int64_t(s) * piece_stride + bo) = *reinterpret_cast<const uint4*>(pc[s]);
+    for (int j = 0; j < 4; ++j)
+      sign[j] = (uint32_t(__double2hiint(x[2 * j])) & 0x80000000u) >> 16 | (uint32_t(__double2hiint(x[2 * j + 1])) & 0x80000000u);
+    store_slice<1>(base + int64_t(g / (OK / 8)) * (kPieces * piece_bytes) + (g % (OK / 8)) * lbo + r * 16, piece_stride, lo,
+                   hi, sign);
   }
 }
 
@@ -286,7 +340,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
                    double* __restrict__ C, double alpha, double beta, double* __restrict__ ws,
                    int* __restrict__ err) {
   extern __shared__ unsigned char smem_raw[];
-  __shared__ uint64_t full[kOzStages], empty[kOzStages], accf, acce, done;
+  __shared__ uint64_t full[kOzStages], empty[kOzStages], accf, acce[2], done;
   __shared__ uint32_t tmem_slot;
   __shared__ int fail, issued, consumed;
   __shared__ int rsc[OM], csc[ON];  // row and column scale exponents of the tile
@@ -319,7 +373,7 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       bar_init(&empty[s], 1);
     }
     bar_init(&accf, 1);
-    bar_init(&acce, kOzDrainWarps);
+    for (int h = 0; h < 2; ++h) bar_init(&acce[h], kOzDrainWarps);
     bar_init(&done, 1);
     fail = 0;
     issued = 0;
@@ -331,11 +385,11 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
 
-  // drain-warp state: TMEM lane quarter (rows) and 32-column group; double-FP32 sums of 32 columns
+  // drain-warp state: TMEM lane quarter (rows) and column group; double-FP32 sums of 16 columns
   const int quarter = warp & 3, colg = warp >> 2;
-  float hi[32], lo[32];
+  unsigned long long hi2[kDrainCols / 2], lo2[kDrainCols / 2];  // two floats each
 #pragma unroll
-  for (int j = 0; j < 32; ++j) { hi[j] = 0.f; lo[j] = 0.f; }
+  for (int j = 0; j < kDrainCols / 2; ++j) { hi2[j] = 0; lo2[j] = 0; }
 
   if (nk > 0 && warp == kOzProducer) {
     if (lane == 0) {
@@ -343,13 +397,9 @@ __global__ void __launch_bounds__(kOzThreads, 1)
           apack + gr.a_pack + (int64_t(t.tm) * gr.slices + ks) * kPieces * kAPieceBytes;
       const unsigned char* b_base =
           bpack + gr.b_pack + (int64_t(t.tn) * gr.slices + ks) * kPieces * kBPieceBytes;
-      uint32_t ph[kOzStages] = {0, 0};
       for (int kc = 0; kc < nk; ++kc) {
-        const int s = kc % kOzStages;
-        if (kc >= kOzStages) {
-          if (!bar_wait(&empty[s], ph[s])) { atomicExch(&fail, 1); break; }
-          ph[s] ^= 1u;
-        }
+        const int s = kc % kOzStages, round = kc / kOzStages;
+        if (round > 0 && !bar_wait(&empty[s], uint32_t((round - 1) & 1))) { atomicExch(&fail, 1); break; }
         unsigned char* st = smem + s * kOzStageBytes;
         bar_expect_tx(&full[s], kOzStageBytes);
         bulk_g2s(st, a_base + int64_t(kc) * kPieces * kAPieceBytes, kPieces * kAPieceBytes, &full[s]);
@@ -360,40 +410,48 @@ __global__ void __launch_bounds__(kOzThreads, 1)
     }
   } else if (nk > 0 && warp == kOzMma) {
     if (lane == 0) {
-      uint32_t ph[kOzStages] = {0, 0};
       for (int kc = 0; kc < nk; ++kc) {
         const int s = kc % kOzStages, cs = kc % kChunk, ch = kc / kChunk;
-        // a new chunk overwrites the level accumulators: the previous chunk must be drained
-        if (cs == 0 && ch > 0 && !bar_wait(&acce, uint32_t((ch - 1) & 1))) { atomicExch(&fail, 1); break; }
-        if (!bar_wait(&full[s], ph[s])) { atomicExch(&fail, 1); break; }
-        ph[s] ^= 1u;
+        if (!bar_wait(&full[s], uint32_t((kc / kOzStages) & 1))) { atomicExch(&fail, 1); break; }
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         const uint32_t abase = s_u32(smem + s * kOzStageBytes);
         const uint32_t bbase = abase + kPieces * kAPieceBytes;
-#pragma unroll
-        for (int kk = 0; kk < OK / 16; ++kk) {
-          // slice pairs (i, j), j <= 6 - i, in MMAs of up to four stacked B pieces: the product of A piece
-          // i with B pieces j0 .. j0 + c - 1 lands in levels i + j0 .. i + j0 + c - 1, the adjacent
-          // 64-column accumulators from column 64 (i + j0); ten MMAs cover the 28 pairs
-          const uint64_t ad[kPieces] = {
-              oz_desc(abase + 0 * kAPieceBytes + kk * 2 * kLboA, kLboA), oz_desc(abase + 1 * kAPieceBytes + kk * 2 * kLboA, kLboA),
-              oz_desc(abase + 2 * kAPieceBytes + kk * 2 * kLboA, kLboA), oz_desc(abase + 3 * kAPieceBytes + kk * 2 * kLboA, kLboA),
-              oz_desc(abase + 4 * kAPieceBytes + kk * 2 * kLboA, kLboA), oz_desc(abase + 5 * kAPieceBytes + kk * 2 * kLboA, kLboA),
-              oz_desc(abase + 6 * kAPieceBytes + kk * 2 * kLboA, kLboA)};
-          auto bd = [&](int j0) { return oz_desc(bbase + j0 * kBPieceStride + kk * 2 * kLboB, kLboB); };
-          const uint32_t a0 = (cs == 0 && kk == 0) ? 0u : 1u;  // the i = 0 MMAs open every level of a chunk
-          auto col = [&](int lvl) { return tmem + uint32_t(lvl * ON); };
-          mma_bf16_oz<4>(col(0), ad[0], bd(0), a0);
-          mma_bf16_oz<3>(col(4), ad[0], bd(4), a0);
-          mma_bf16_oz<4>(col(1), ad[1], bd(0), 1u);
-          mma_bf16_oz<2>(col(5), ad[1], bd(4), 1u);
-          mma_bf16_oz<4>(col(2), ad[2], bd(0), 1u);
-          mma_bf16_oz<1>(col(6), ad[2], bd(4), 1u);
-          mma_bf16_oz<4>(col(3), ad[3], bd(0), 1u);
-          mma_bf16_oz<3>(col(4), ad[4], bd(0), 1u);
-          mma_bf16_oz<2>(col(5), ad[5], bd(0), 1u);
-          mma_bf16_oz<1>(col(6), ad[6], bd(0), 1u);
+        // slice pairs (i, j), j <= 6 - i, in MMAs of up to four stacked B pieces: the product of A piece
+        // i with B pieces j0 .. j0 + c - 1 lands in levels i + j0 .. i + j0 + c - 1, the adjacent
+        // 64-column accumulators from column 64 (i + j0); ten MMAs cover the 28 pairs.  Narrow ones first:
+        // an MMA of N = 64 or 128 waits for its operands, and the wide ones behind hide that (k = 144 to
+        // 2464, without the drains: 1.66 ms as the levels are opened, 1.73 from wide to narrow, 1.49 so)
+        const uint64_t ad[kPieces] = {
+            oz_desc(abase + 0 * kAPieceBytes, kLboA), oz_desc(abase + 1 * kAPieceBytes, kLboA),
+            oz_desc(abase + 2 * kAPieceBytes, kLboA), oz_desc(abase + 3 * kAPieceBytes, kLboA),
+            oz_desc(abase + 4 * kAPieceBytes, kLboA), oz_desc(abase + 5 * kAPieceBytes, kLboA),
+            oz_desc(abase + 6 * kAPieceBytes, kLboA)};
+        auto bd = [&](int j0) { return oz_desc(bbase + j0 * kBPieceStride, kLboB); };
+        auto col = [&](int lvl) { return tmem + uint32_t(lvl * ON); };
+        // The first slice of a chunk opens the levels with its i = 0 MMAs, each once the previous chunk has
+        // been drained from it: the levels 4-6 are drained first and multiplied while 0-3 are read.
+        const uint32_t drained = uint32_t((ch - 1) & 1);
+        if (cs == 0) {
+          if (ch > 0 && !bar_wait(&acce[0], drained)) { atomicExch(&fail, 1); break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          mma_bf16_oz<3>(col(4), ad[0], bd(4), 0u);
         }
+        mma_bf16_oz<1>(col(6), ad[6], bd(0), 1u);
+        mma_bf16_oz<1>(col(6), ad[2], bd(4), 1u);
+        mma_bf16_oz<2>(col(5), ad[5], bd(0), 1u);
+        mma_bf16_oz<2>(col(5), ad[1], bd(4), 1u);
+        mma_bf16_oz<3>(col(4), ad[4], bd(0), 1u);
+        if (cs == 0) {
+          if (ch > 0 && !bar_wait(&acce[1], drained)) { atomicExch(&fail, 1); break; }
+          asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          mma_bf16_oz<4>(col(0), ad[0], bd(0), 0u);
+        } else {
+          mma_bf16_oz<3>(col(4), ad[0], bd(4), 1u);
+        }
+        mma_bf16_oz<4>(col(3), ad[3], bd(0), 1u);
+        mma_bf16_oz<4>(col(2), ad[2], bd(0), 1u);
+        mma_bf16_oz<4>(col(1), ad[1], bd(0), 1u);
+        if (cs != 0) mma_bf16_oz<4>(col(0), ad[0], bd(0), 1u);
         commit_to(&empty[s]);
         if (cs == kChunk - 1 || kc == nk - 1) commit_to(&accf);
         consumed = kc + 1;
@@ -408,39 +466,39 @@ __global__ void __launch_bounds__(kOzThreads, 1)
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll 1
-      for (int level = kLevels - 1; level >= 0; --level) {  // smallest contributions first
-        uint32_t v[32];
-        const uint32_t taddr = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(level * ON + colg * 32);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,"
-            "%16,%17,%18,%19,%20,%21,%22,%23,%24,%25,%26,%27,%28,%29,%30,%31}, [%32];"
-            : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-              "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-              "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-              "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-            : "r"(taddr));
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      // smallest contributions first; the next level's load is in flight while one is added
+      static_assert(kDrainCols == 16, "the loads below");
+      uint32_t next[kDrainCols];
+      const uint32_t tcol = tmem + (uint32_t(quarter * 32) << 16) + uint32_t(colg * kDrainCols);
+      tmem_load16(tcol + uint32_t((kLevels - 1) * ON), next);
 #pragma unroll
-        for (int j = 0; j < 32; ++j) {
+      for (int level = kLevels - 1; level >= 0; --level) {
+        uint32_t v[kDrainCols];
+        tmem_wait16(next);
+#pragma unroll
+        for (int j = 0; j < kDrainCols; ++j) v[j] = next[j];
+        if (level == 4 || level == 0) {  // levels 4-6, then 0-3 have been read
+          asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+          __syncwarp();
+          if (lane == 0)
+            asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s_u32(&acce[level == 0])) : "memory");
+        }
+        if (level > 0) tmem_load16(tcol + uint32_t((level - 1) * ON), next);
+#pragma unroll
+        for (int j = 0; j < kDrainCols / 2; ++j) {
           // two-sum of hi and the exact level partial; the rounding error goes to lo
-          const float x = __uint_as_float(v[j]);
-          const float s = __fadd_rn(hi[j], x);
-          const float bb = __fsub_rn(s, hi[j]);
-          const float e = __fadd_rn(__fsub_rn(hi[j], __fsub_rn(s, bb)), __fsub_rn(x, bb));
-          hi[j] = s;
-          lo[j] = __fadd_rn(lo[j], e);
+          const unsigned long long x = pair(v[2 * j], v[2 * j + 1]);
+          const unsigned long long t = add2(hi2[j], x), bb = sub2(t, hi2[j]);
+          lo2[j] = add2(lo2[j], add2(sub2(hi2[j], sub2(t, bb)), sub2(x, bb)));
+          hi2[j] = t;
         }
       }
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {  // renormalise: |lo| stays below one unit of hi
-        const float s = __fadd_rn(hi[j], lo[j]);
-        lo[j] = __fsub_rn(lo[j], __fsub_rn(s, hi[j]));
-        hi[j] = s;
+      for (int j = 0; j < kDrainCols / 2; ++j) {  // renormalise: |lo| stays below one unit of hi
+        const unsigned long long t = add2(hi2[j], lo2[j]);
+        lo2[j] = sub2(lo2[j], sub2(t, hi2[j]));
+        hi2[j] = t;
       }
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(s_u32(&acce)) : "memory");
     }
   }
   bool ok = true;
@@ -450,18 +508,24 @@ __global__ void __launch_bounds__(kOzThreads, 1)
   ok = __syncthreads_and(ok);
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
 
+  float hi[kDrainCols], lo[kDrainCols];
+#pragma unroll
+  for (int j = 0; j < kDrainCols; ++j) {
+    hi[j] = __uint_as_float(uint32_t(hi2[j / 2] >> (32 * (j % 2))));
+    lo[j] = __uint_as_float(uint32_t(lo2[j / 2] >> (32 * (j % 2))));
+  }
   // 0: partial tile to the workspace, 1: C = acc, 2: C = alpha acc, 3: C = alpha acc + beta C
   const int mode = t.slot >= 0 ? 0 : beta != 0.0 ? 3 : alpha != 1.0 ? 2 : 1;
   if (ok && nk > 0 && warp < kOzDrainWarps) {
     const int64_t row = m0 + quarter * 32 + lane;
     const int ei = rsc[quarter * 32 + lane];
     if (mode != 0 && swp) {
-      // transposed store through shared memory (the stages are idle now): thread (r, 32 columns) puts
+      // transposed store through shared memory (the stages are idle now): thread (r, its columns) puts
       // its values at T[c][r] (row pitch 129 doubles), then each warp writes 32 consecutive rows of C
       double* T = reinterpret_cast<double*>(smem);
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int c = colg * 32 + j;
+      for (int j = 0; j < kDrainCols; ++j) {
+        const int c = colg * kDrainCols + j;
         const int sc = ei + csc[c];
         T[c * (OM + 1) + quarter * 32 + lane] = scaled_double(hi[j], sc) + scaled_double(lo[j], sc);
       }
@@ -478,13 +542,13 @@ __global__ void __launch_bounds__(kOzThreads, 1)
       }
     } else if (row < pm) {
 #pragma unroll
-      for (int j = 0; j < 32; ++j) {
-        const int64_t col = n0 + colg * 32 + j;
+      for (int j = 0; j < kDrainCols; ++j) {
+        const int64_t col = n0 + colg * kDrainCols + j;
         if (col < pn) {
-          const int sc = ei + csc[colg * 32 + j];
+          const int sc = ei + csc[colg * kDrainCols + j];
           const double acc = scaled_double(hi[j], sc) + scaled_double(lo[j], sc);
           if (mode == 0) {  // split-K partial: raw sum, tile-local column-major OM x ON
-            ws[int64_t(t.slot) * OM * ON + (quarter * 32 + lane) + int64_t(colg * 32 + j) * OM] = acc;
+            ws[int64_t(t.slot) * OM * ON + (quarter * 32 + lane) + int64_t(colg * kDrainCols + j) * OM] = acc;
           } else {
             double* cp = C + d.c_off + row + col * d.ldc;
             if (mode == 1) *cp = acc;
@@ -550,11 +614,10 @@ OzPlanHost build_oz_plan(const xgb_gemm_desc* descs, int n, bool allow_swap) {
   if (allow_swap)
     for (int g = 0; g < n; ++g) swap[g] = 4 * tiles_of(descs[g].n, descs[g].m) <= 3 * tiles_of(descs[g].m, descs[g].n);
   // rowmax layout: every group's rows of the "A" role first, then every group's rows of the "B" role
-  // (columns of the product), so that the B part can be cleared and recomputed alone when only B
-  // changes between products
+  // (columns of the product)
   OzPlanHost p;
-  for (int g = 0; g < n; ++g) p.rowmax_a += swap[g] ? descs[g].n : descs[g].m;
-  int64_t ra = 0, rb = p.rowmax_a;
+  int64_t ra = 0, rb = 0;
+  for (int g = 0; g < n; ++g) rb += swap[g] ? descs[g].n : descs[g].m;
   for (int g = 0; g < n; ++g) {
     const xgb_gemm_desc& d = descs[g];
     const int64_t pm = swap[g] ? d.n : d.m, pn = swap[g] ? d.m : d.n;  // extents of the computed product
@@ -571,10 +634,10 @@ OzPlanHost build_oz_plan(const xgb_gemm_desc* descs, int n, bool allow_swap) {
     rb += pn;
     p.a_bytes += int64_t(gr.a_tiles) * gr.slices * kPieces * kAPieceBytes;
     p.b_bytes += int64_t(gr.b_tiles) * gr.slices * kPieces * kBPieceBytes;
-    for (int32_t s = 0; s < gr.slices; ++s) {
-      for (int32_t t = 0; t < gr.a_tiles; ++t) p.tasks_a.push_back({g, t, s, 0});
-      for (int32_t t = 0; t < gr.b_tiles; ++t) p.tasks_b.push_back({g, t, s, 1});
-    }
+    // clusters that slice the operands: at most 128 k values per CTA, eight CTAs
+    while (p.pack_cluster < 8 && gr.slices * OK > 128 * p.pack_cluster) p.pack_cluster *= 2;
+    for (int32_t t = 0; t < gr.a_tiles; ++t) p.tasks_a.push_back({g, t, 0, 0});
+    for (int32_t t = 0; t < gr.b_tiles; ++t) p.tasks_b.push_back({g, t, 0, 1});
     p.groups.push_back(gr);
   }
   // output tiles and their K ranges.  One CTA runs per SM (its stages and TMEM fill one), so the K
@@ -622,13 +685,20 @@ OzPlanHost build_oz_plan(const xgb_gemm_desc* descs, int n, bool allow_swap) {
 }
 
 void launch_oz_pack(const xgb_gemm_desc* d_descs, const OzGroup* d_groups, const TcPackTask* d_tasks, int n_tasks,
-                    const double* A, const double* B, unsigned long long* rowmax, int64_t clear_from,
-                    int64_t clear_count, unsigned char* apack, unsigned char* bpack, cudaStream_t s) {
+                    int cluster, const double* A, const double* B, unsigned long long* rowmax, unsigned char* apack,
+                    unsigned char* bpack, cudaStream_t s) {
   if (n_tasks <= 0) return;
-  if (clear_count > 0) cudaMemsetAsync(rowmax + clear_from, 0, sizeof(unsigned long long) * size_t(clear_count), s);
-  oz_rowmax_kernel<<<n_tasks, 256, 0, s>>>(d_descs, d_groups, d_tasks, A, B, rowmax);
-  count_launch();
-  oz_pack_kernel<<<n_tasks, 256, 0, s>>>(d_descs, d_groups, d_tasks, A, B, rowmax, apack, bpack);
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3(unsigned(n_tasks) * unsigned(cluster));
+  cfg.blockDim = dim3(256);
+  cfg.stream = s;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim = {unsigned(cluster), 1, 1};
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  const cudaError_t e = cudaLaunchKernelEx(&cfg, oz_pack_kernel, d_descs, d_groups, d_tasks, A, B, rowmax, apack, bpack);
+  if (e != cudaSuccess) throw std::runtime_error(std::string("slicing launch: ") + cudaGetErrorString(e));
   count_launch();
 }
 
@@ -679,19 +749,18 @@ void run_gemm_oz_host(const xgb_gemm_desc* h_descs, int n, const double* A, cons
   auto* rm = static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long) * size_t(std::max<int64_t>(op.rowmax, 1))));
   auto* ap = static_cast<unsigned char*>(dev_alloc(size_t(std::max<int64_t>(op.a_bytes, 16))));
   auto* bp = static_cast<unsigned char*>(dev_alloc(size_t(std::max<int64_t>(op.b_bytes, 16))));
-  launch_gemm_oz(dd, dg, dk, int(op.tasks.size()), dt, int(op.tiles.size()), dr, int(op.red.size()), op.slots, A, B,
-                 rm, op.rowmax, ap, bp, C, alpha, beta, s);
+  launch_gemm_oz(dd, dg, dk, int(op.tasks.size()), op.pack_cluster, dt, int(op.tiles.size()), dr, int(op.red.size()), op.slots, A, B,
+                 rm, ap, bp, C, alpha, beta, s);
   for (void* p : {static_cast<void*>(dd), static_cast<void*>(dg), static_cast<void*>(dk), static_cast<void*>(dt),
                   static_cast<void*>(dr), static_cast<void*>(rm), static_cast<void*>(ap), static_cast<void*>(bp)})
     dev_free(p);
 }
 
 void launch_gemm_oz(const xgb_gemm_desc* d_descs, const OzGroup* d_groups, const TcPackTask* d_tasks, int n_tasks,
-                    const GemmTile* d_tiles, int n_tiles, const SplitReduce* d_red, int n_red, int slots,
-                    const double* A, const double* B, unsigned long long* rowmax, int64_t n_rowmax,
-                    unsigned char* apack, unsigned char* bpack, double* C, double alpha, double beta, cudaStream_t s) {
+                    int cluster, const GemmTile* d_tiles, int n_tiles, const SplitReduce* d_red, int n_red, int slots,
+                    const double* A, const double* B, unsigned long long* rowmax, unsigned char* apack, unsigned char* bpack, double* C, double alpha, double beta, cudaStream_t s) {
   if (n_tiles <= 0) return;
-  launch_oz_pack(d_descs, d_groups, d_tasks, n_tasks, A, B, rowmax, 0, n_rowmax, apack, bpack, s);
+  launch_oz_pack(d_descs, d_groups, d_tasks, n_tasks, cluster, A, B, rowmax, apack, bpack, s);
   launch_oz_gemm(d_descs, d_groups, d_tiles, n_tiles, d_red, n_red, slots, apack, bpack, rowmax, C, alpha, beta, s);
 }
 

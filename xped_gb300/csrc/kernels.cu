@@ -1010,8 +1010,8 @@ int xgb_grouped_gemm(int precision, int n_groups, const xgb_gemm_desc* descs, co
     auto* ap = static_cast<unsigned char*>(dev_alloc(size_t(std::max<int64_t>(op.a_bytes, 16))));
     auto* bp = static_cast<unsigned char*>(dev_alloc(size_t(std::max<int64_t>(op.b_bytes, 16))));
     prof_begin(K_GEMM_OZ, s);
-    launch_gemm_oz(dd, dg, dk, int(op.tasks.size()), dt, int(op.tiles.size()), dr, int(op.red.size()), op.slots, A, B,
-                   rm, op.rowmax, ap, bp, C, alpha, beta, s);
+    launch_gemm_oz(dd, dg, dk, int(op.tasks.size()), op.pack_cluster, dt, int(op.tiles.size()), dr, int(op.red.size()), op.slots, A, B,
+                   rm, ap, bp, C, alpha, beta, s);
     prof_end(K_GEMM_OZ, s, flops);
     for (void* p : {static_cast<void*>(dd), static_cast<void*>(dg), static_cast<void*>(dk), static_cast<void*>(dt),
                     static_cast<void*>(dr), static_cast<void*>(rm), static_cast<void*>(ap), static_cast<void*>(bp)})

@@ -171,29 +171,30 @@ struct OzGroup {
 struct OzPlanHost {
   std::vector<OzGroup> groups;
   std::vector<TcPackTask> tasks;            // tasks_a then tasks_b
-  std::vector<TcPackTask> tasks_a, tasks_b;  // the op(A) and op(B) chunks alone
+  std::vector<TcPackTask> tasks_a, tasks_b;  // the op(A) and op(B) tiles alone
+  int pack_cluster = 1;                      // CTAs per task
   std::vector<GemmTile> tiles;               // k0 / k1 in K slices; slot >= 0: split-K partial
   std::vector<SplitReduce> red;              // fixed-order sums of the split tiles
   int32_t slots = 0;                         // partial tiles (workspace slots x 128 x 64 doubles)
   int64_t a_bytes = 0, b_bytes = 0;
-  int64_t rowmax = 0, rowmax_a = 0;  // entries in all; the op(A) rows come first
+  int64_t rowmax = 0;  // entries; the op(A) rows come first
 };
 // allow_swap: groups with few rows and many columns may be computed transposed (not for callers that
 // keep one operand's slices across products, whose roles must stay fixed)
 OzPlanHost build_oz_plan(const xgb_gemm_desc* descs, int n, bool allow_swap = true);
-// the row scales and slices of the given chunks (rowmax[clear_from .. + clear_count) zeroed first)
+// the row scales and slices of the given tiles (pack_cluster CTAs each)
 void launch_oz_pack(const xgb_gemm_desc* d_descs, const OzGroup* d_groups, const TcPackTask* d_tasks, int n_tasks,
-                    const double* A, const double* B, unsigned long long* rowmax, int64_t clear_from,
-                    int64_t clear_count, unsigned char* apack, unsigned char* bpack, cudaStream_t s);
+                    int cluster, const double* A, const double* B, unsigned long long* rowmax, unsigned char* apack,
+                    unsigned char* bpack, cudaStream_t s);
 // the product kernel (and, for split tiles, the fixed-order reduce; workspace allocated stream-ordered)
 void launch_oz_gemm(const xgb_gemm_desc* d_descs, const OzGroup* d_groups, const GemmTile* d_tiles, int n_tiles,
                     const SplitReduce* d_red, int n_red, int slots, const unsigned char* apack,
                     const unsigned char* bpack, const unsigned long long* rowmax, double* C, double alpha, double beta,
                     cudaStream_t s);
 void launch_gemm_oz(const xgb_gemm_desc* d_descs, const OzGroup* d_groups, const TcPackTask* d_tasks, int n_tasks,
-                    const GemmTile* d_tiles, int n_tiles, const SplitReduce* d_red, int n_red, int slots,
-                    const double* A, const double* B, unsigned long long* rowmax, int64_t n_rowmax,
-                    unsigned char* apack, unsigned char* bpack, double* C, double alpha, double beta, cudaStream_t s);
+                    int cluster, const GemmTile* d_tiles, int n_tiles, const SplitReduce* d_red, int n_red, int slots,
+                    const double* A, const double* B, unsigned long long* rowmax, unsigned char* apack,
+                    unsigned char* bpack, double* C, double alpha, double beta, cudaStream_t s);
 
 // randomized tSVD helpers (rsvd.cu)
 struct GaussBlock { int64_t offset, count, stream; };       // fill out[offset .. offset+count) from stream

@@ -162,8 +162,7 @@ class OzProducts {
     n_red_ = int(op.red.size());
     slots_ = op.slots;
     n_b_ = int(op.tasks_b.size());
-    rowmax_a_ = op.rowmax_a;
-    rowmax_ = op.rowmax;
+    cluster_ = op.pack_cluster;
     for (const auto& g : d) flops_ += 2.0 * double(g.m) * double(g.n) * double(g.k);
     od_ = st_.add(d);
     og_ = st_.add(op.groups);
@@ -172,12 +171,12 @@ class OzProducts {
     ot_ = st_.add(op.tiles);
     or_ = st_.add(op.red);
     st_.upload(s);
-    rm_ = static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long) * size_t(std::max<int64_t>(rowmax_, 1))));
+    rm_ = static_cast<unsigned long long*>(dev_alloc(sizeof(unsigned long long) * size_t(std::max<int64_t>(op.rowmax, 1))));
     ap_ = static_cast<unsigned char*>(dev_alloc(size_t(std::max<int64_t>(op.a_bytes, 16))));
     bp_ = static_cast<unsigned char*>(dev_alloc(size_t(std::max<int64_t>(op.b_bytes, 16))));
     prof_begin(K_GEMM_OZ, s);
-    launch_oz_pack(st_.at<xgb_gemm_desc>(od_), st_.at<OzGroup>(og_), st_.at<TcPackTask>(oa_), int(op.tasks_a.size()), A,
-                   nullptr, rm_, 0, rowmax_a_, ap_, bp_, s);
+    launch_oz_pack(st_.at<xgb_gemm_desc>(od_), st_.at<OzGroup>(og_), st_.at<TcPackTask>(oa_), int(op.tasks_a.size()),
+                   cluster_, A, nullptr, rm_, ap_, bp_, s);
     prof_end(K_GEMM_OZ, s, 0.0);
   }
   OzProducts(const OzProducts&) = delete;
@@ -191,8 +190,8 @@ class OzProducts {
   void apply(const double* A, const double* X, double* C, cudaStream_t s) {
     if (n_tiles_ == 0) return;
     prof_begin(K_GEMM_OZ, s);
-    launch_oz_pack(st_.at<xgb_gemm_desc>(od_), st_.at<OzGroup>(og_), st_.at<TcPackTask>(ob_), n_b_, A, X, rm_,
-                   rowmax_a_, rowmax_ - rowmax_a_, ap_, bp_, s);
+    launch_oz_pack(st_.at<xgb_gemm_desc>(od_), st_.at<OzGroup>(og_), st_.at<TcPackTask>(ob_), n_b_, cluster_, A, X,
+                   rm_, ap_, bp_, s);
     launch_oz_gemm(st_.at<xgb_gemm_desc>(od_), st_.at<OzGroup>(og_), st_.at<GemmTile>(ot_), n_tiles_,
                    st_.at<SplitReduce>(or_), n_red_, slots_, ap_, bp_, rm_, C, 1.0, 0.0, s);
     prof_end(K_GEMM_OZ, s, flops_);
@@ -201,8 +200,7 @@ class OzProducts {
  private:
   Staging st_;
   size_t od_ = 0, og_ = 0, oa_ = 0, ob_ = 0, ot_ = 0, or_ = 0;
-  int n_tiles_ = 0, n_b_ = 0, n_red_ = 0, slots_ = 0;
-  int64_t rowmax_a_ = 0, rowmax_ = 0;
+  int n_tiles_ = 0, n_b_ = 0, n_red_ = 0, slots_ = 0, cluster_ = 1;
   double flops_ = 0;
   unsigned long long* rm_ = nullptr;
   unsigned char* ap_ = nullptr;

@@ -174,7 +174,7 @@ struct GemmPlan {
   // FP64-accurate tensor-core form from exact BF16 slices (built on first use); oz_route: whether
   // this product takes it (k too short to amortise the per-tile cost: the FP64 CUDA-core kernel)
   bool oz_ready = false, oz_route = true, oz_routed = false;
-  int n_oz_tiles = 0, n_oz_tasks = 0, n_oz_red = 0, oz_slots = 0;
+  int n_oz_tiles = 0, n_oz_tasks = 0, n_oz_red = 0, oz_slots = 0, oz_cluster = 1;
   SplitReduce* d_oz_red = nullptr;
   int64_t oz_a_bytes = 0, oz_b_bytes = 0, oz_rowmax = 0;
   OzGroup* d_oz_groups = nullptr;
@@ -673,6 +673,7 @@ Tensor matmul(const Tensor& a0, const Tensor& b0, bool adj_a, bool adj_b) {
         plan->d_oz_red = plan->mem.table(op.red);
         plan->n_oz_red = int(op.red.size());
         plan->oz_slots = op.slots;
+        plan->oz_cluster = op.pack_cluster;
         plan->oz_ready = true;
       }
     }
@@ -682,9 +683,9 @@ Tensor matmul(const Tensor& a0, const Tensor& b0, bool adj_a, bool adj_b) {
     auto* ap = static_cast<unsigned char*>(dev_alloc(size_t(std::max<int64_t>(plan->oz_a_bytes, 16))));
     auto* bp = static_cast<unsigned char*>(dev_alloc(size_t(std::max<int64_t>(plan->oz_b_bytes, 16))));
     prof_begin(K_GEMM_OZ, st);
-    launch_gemm_oz(plan->d_descs, plan->d_oz_groups, plan->d_oz_tasks, plan->n_oz_tasks, plan->d_oz_tiles,
-                   plan->n_oz_tiles, plan->d_oz_red, plan->n_oz_red, plan->oz_slots, a.data(), b.data(), rm,
-                   plan->oz_rowmax, ap, bp, out.data(), 1.0, 0.0, st);
+    launch_gemm_oz(plan->d_descs, plan->d_oz_groups, plan->d_oz_tasks, plan->n_oz_tasks, plan->oz_cluster,
+                   plan->d_oz_tiles, plan->n_oz_tiles, plan->d_oz_red, plan->n_oz_red, plan->oz_slots, a.data(),
+                   b.data(), rm, ap, bp, out.data(), 1.0, 0.0, st);
     prof_end(K_GEMM_OZ, st, plan->flops);
     dev_free(rm);
     dev_free(ap);
