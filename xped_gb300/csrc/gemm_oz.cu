@@ -70,6 +70,7 @@ constexpr int kOzDrainWarps = 16, kOzProducer = kOzDrainWarps, kOzMma = kOzDrain
 constexpr int kOzWarps = kOzDrainWarps + 2, kOzThreads = kOzWarps * 32;
 constexpr int kDrainCols = ON / (kOzDrainWarps / 4);  // columns of a drain warp
 constexpr long long kOzSpin = 1ll << 26;
+constexpr int kPackRows = 32;                       // rows of a slicing cluster
 constexpr uint32_t kSboBytes = 128;                 // next 8-row group
 // A: seven separate 128-row pieces.  B: the seven 64-row pieces stacked into one 448-row operand (row
 // group g of piece s is row group 8 s + g), so that pieces t .. t + c - 1 form one N = 64 c operand
@@ -221,8 +222,8 @@ __device__ __forceinline__ void store_slice(unsigned char* at, int stride, const
   if constexpr (S < kPieces) store_slice<S + 1>(at, stride, lo, hi, sign);
 }
 
-// One cluster per (group, tile of OM rows of op(A) or ON rows of op(B)^T): its CTAs share the K range in groups of
-// eight, a thread a row and every second or fourth group.  The row maxima (on the IEEE bits: integer order is numeric
+// One cluster per (group, 32 rows of op(A) or of op(B)^T): its CTAs share the K range in groups of eight, a thread a row
+// and every eighth group.  The row maxima (on the IEEE bits: integer order is numeric
 // order) meet in distributed shared memory; then the same entries are read again, from L2, and sliced.  Bound by the
 // 14 bytes written per entry for large operands, by the reads' latency for small ones.
 // Measured (nine blocks of 100 to 1729 squared, both operands): 233 us as a maximum kernel (with atomics) and a slicing
@@ -234,7 +235,7 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const xgb_gemm_desc* __res
                                                        unsigned long long* __restrict__ rowmax,
                                                        unsigned char* __restrict__ apack,
                                                        unsigned char* __restrict__ bpack) {
-  __shared__ unsigned long long part[256], own[OM];
+  __shared__ unsigned long long part[256], own[kPackRows];
   cg::cluster_group cluster = cg::this_cluster();
   const int P = int(cluster.num_blocks()), me = int(cluster.block_rank());
   const TcPackTask t = tasks[blockIdx.x / unsigned(P)];
@@ -244,7 +245,8 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const xgb_gemm_desc* __res
   const bool sb = isB != (gr.swap != 0);  // the rows of this role are op(B)^T's (columns of op(B))
   const int64_t ld = sb ? d.ldb : d.lda, rows = sb ? d.n : d.m;
   const bool rowfast = sb ? d.trans_b != 0 : d.trans_a == 0;
-  const int tr = isB ? ON : OM, r = int(threadIdx.x) % tr, q = int(threadIdx.x) / tr, nq = 256 / tr;
+  constexpr int tr = kPackRows, nq = 256 / kPackRows;
+  const int r = int(threadIdx.x) % tr, q = int(threadIdx.x) / tr;
   const int64_t row = int64_t(t.tile) * tr + r;
   const bool live = row < rows;
   const double* src = (sb ? B + d.b_off : A + d.a_off) + (live ? (rowfast ? row : row * ld) : 0);
@@ -301,7 +303,9 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const xgb_gemm_desc* __res
   const int piece_bytes = isB ? kBPieceBytes : kAPieceBytes;
   const int piece_stride = isB ? int(kBPieceStride) : kAPieceBytes;
   const uint32_t lbo = isB ? kLboB : kLboA;
-  unsigned char* base = (isB ? bpack + gr.b_pack : apack + gr.a_pack) + int64_t(t.tile) * gr.slices * (kPieces * piece_bytes);
+  const int per_tile = (isB ? ON : OM) / tr, in_tile = (t.tile % per_tile) * tr + r;  // row of the output tile
+  unsigned char* base = (isB ? bpack + gr.b_pack : apack + gr.a_pack) +
+                        int64_t(t.tile / per_tile) * gr.slices * (kPieces * piece_bytes) + in_tile * 16;
   for (int g = first; g < last; g += nq) {
     double x[8];
     load8(g, x);
@@ -311,7 +315,7 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const xgb_gemm_desc* __res
 #pragma unroll
     for (int j = 0; j < 4; ++j)
       sign[j] = (uint32_t(__double2hiint(x[2 * j])) & 0x80000000u) >> 16 | (uint32_t(__double2hiint(x[2 * j + 1])) & 0x80000000u);
-    store_slice<1>(base + int64_t(g / (OK / 8)) * (kPieces * piece_bytes) + (g % (OK / 8)) * lbo + r * 16, piece_stride, lo,
+    store_slice<1>(base + int64_t(g / (OK / 8)) * (kPieces * piece_bytes) + (g % (OK / 8)) * lbo, piece_stride, lo,
                    hi, sign);
   }
 }
@@ -595,8 +599,18 @@ __global__ void __launch_bounds__(256) oz_splitk_reduce_kernel(const xgb_gemm_de
     const int64_t i = int64_t(r.tm) * OM + li, j = int64_t(r.tn) * ON + lj;
     if (i >= pm || j >= pn) continue;
     const int64_t w = li + int64_t(lj) * OM;
-    double acc = ws[int64_t(r.first) * OM * ON + w];
-    for (int p = 1; p < r.count; ++p) acc += ws[(int64_t(r.first) + p) * OM * ON + w];
+    const double* part = ws + int64_t(r.first) * OM * ON + w;
+    double acc = part[0];
+    // eight loads in flight: one after the other a tile cut nineteen ways took 12 us
+    for (int p = 1; p < r.count; p += 8) {
+      double x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (p + u < r.count) x[u] = __ldg(part + int64_t(p + u) * OM * ON);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (p + u < r.count) acc += x[u];
+    }
     double* c = C + d.c_off + (swp ? j + i * d.ldc : i + j * d.ldc);
     *c = beta != 0.0 ? fma(alpha, acc, beta * *c) : alpha == 1.0 ? acc : alpha * acc;
   }
@@ -636,8 +650,8 @@ OzPlanHost build_oz_plan(const xgb_gemm_desc* descs, int n, bool allow_swap) {
     p.b_bytes += int64_t(gr.b_tiles) * gr.slices * kPieces * kBPieceBytes;
     // clusters that slice the operands: at most 128 k values per CTA, eight CTAs
     while (p.pack_cluster < 8 && gr.slices * OK > 128 * p.pack_cluster) p.pack_cluster *= 2;
-    for (int32_t t = 0; t < gr.a_tiles; ++t) p.tasks_a.push_back({g, t, 0, 0});
-    for (int32_t t = 0; t < gr.b_tiles; ++t) p.tasks_b.push_back({g, t, 0, 1});
+    for (int32_t t = 0; t < gr.a_tiles * (OM / kPackRows); ++t) p.tasks_a.push_back({g, t, 0, 0});
+    for (int32_t t = 0; t < gr.b_tiles * (ON / kPackRows); ++t) p.tasks_b.push_back({g, t, 0, 1});
     p.groups.push_back(gr);
   }
   // output tiles and their K ranges.  One CTA runs per SM (its stages and TMEM fill one), so the K

@@ -456,8 +456,17 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const xgb_gemm_desc*
   for (int64_t e = threadIdx.x; e < tt; e += blockDim.x) {
     const int64_t i = int64_t(r.tm) * tile + e % tile, j = int64_t(r.tn) * tile + e / tile;
     if (i >= d.m || j >= d.n) continue;
-    double acc = ws[int64_t(r.first) * tt + e];
-    for (int p = 1; p < r.count; ++p) acc += ws[(int64_t(r.first) + p) * tt + e];
+    const double* part = ws + int64_t(r.first) * tt + e;
+    double acc = part[0];
+    for (int p = 1; p < r.count; p += 8) {  // eight loads in flight
+      double x[8];
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (p + u < r.count) x[u] = __ldg(part + int64_t(p + u) * tt);
+#pragma unroll
+      for (int u = 0; u < 8; ++u)
+        if (p + u < r.count) acc += x[u];
+    }
     double* c = C + d.c_off + i + j * d.ldc;
     double v = alpha == 1.0 ? acc : alpha * acc;
     if (beta != 0.0) v += beta * (*c);
