@@ -500,11 +500,12 @@ __global__ void __launch_bounds__(512) chol_narrow_kernel(const CholDesc* __rest
 //   each CTA forms P_i = A_iK T^T (= L_iK) and M_i = P_i T of its rows, and sends P to every CTA;
 //   A_iJ -= P_i P_J^T for K < J <= i, Y_iJ -= M_i Y_KJ for J < K, Y_iK = -M_i;
 // where the owner of block K + 1 lets four warps (one per quarter of the SM) update and factor that diagonal block
-// first, beside the update of its other rows.  Two cluster barriers a panel.  The pivots are still a chain, 16 times
-// 700 cycles a panel, but the l^3 / 3 multiply-adds run on the pipes of all CTAs.  The sums' order does not depend on
-// the cluster's size.
+// first, beside the update of its other rows; the owner of K stores X_K = T Y_K meanwhile.  Two cluster barriers a panel.
+// The pivots are still a chain, 16 times 880 cycles a panel (1300 beside the updates), but the l^3 / 3 multiply-adds run
+// on the pipes of all CTAs.  The sums' order does not depend on the cluster's size.  (Two rows of every block per CTA
+// balance the updates, but need a third barrier and send more: as fast at 150 columns, 5 % slower at 125.)
 // Measured, against a factorisation on one SM with the inverse in a second kernel: one block about 150 wide 357 ->
-// 180 us, two about 125 wide 214 -> 130, two about 190 wide 894 -> 257; CTMRG D = 6, chi = 128 134 -> 99 us a call.
+// 171 us, two about 125 wide 214 -> 119, two about 190 wide 894 -> 256; CTMRG D = 6, chi = 128 134 -> 89 us a call.
 // One CTA is the faster up to 48 columns (its chain has no cluster barriers).
 constexpr int kPan = 16;
 __host__ __device__ constexpr int chol_cluster_elems(int l, int cluster) {
@@ -561,7 +562,7 @@ __global__ void __launch_bounds__(512) chol_cluster_kernel(const CholDesc* __res
                                                            const double* __restrict__ G, double* __restrict__ Rinv,
                                                            double rel_shift, int* __restrict__ bad) {
   extern __shared__ __align__(16) double chol_sm[];
-  __shared__ double trace_s, pivots[kPan];
+  __shared__ double pivots[kPan], partial[(kCholCluster + 31) / 32];
   cg::cluster_group cluster = cg::this_cluster();
   const int P = int(cluster.num_blocks()), me = int(cluster.block_rank());
   const CholDesc d = descs[blockIdx.x / P];
@@ -577,46 +578,74 @@ __global__ void __launch_bounds__(512) chol_cluster_kernel(const CholDesc* __res
   const double* Gg = G + d.g_off;
   for (int k = warp; k < own * kPan; k += warps) {  // row i of the lower triangle from column i of G's upper one
     const int gb = me + (k / kPan) * P, i = gb * kPan + k % kPan;
-    for (int c = lane; c < (gb + 1) * kPan; c += 32) A[k * ld + c] = i < l && c <= i ? Gg[c + i * l] : 0.0;
+#pragma unroll 5
+    for (int c = lane; c < (gb + 1) * kPan; c += 32) A[k * ld + c] = i < l && c <= i ? __ldg(Gg + c + i * l) : 0.0;
   }
-  if (warp == 0) {
-    const double t = chol_trace(l, [&](int i) { return Gg[i + i * l]; });
-    if (lane == 0) trace_s = t;
+  const int groups = (l + 31) / 32;
+  for (int g = warp; g < groups; g += warps) {
+    const int i = g * 32 + lane;
+    const double t = warp_sum_d(i < l ? Gg[i + i * l] : 0.0);
+    if (lane == 0) partial[g] = t;
   }
   __syncthreads();
-  const CholShift sh(d, trace_s, rel_shift);
+  double trace = 0.0;
+  for (int g = 0; g < groups; ++g) trace += partial[g];
+  const CholShift sh(d, trace, rel_shift);
   for (int k = tid; k < own * kPan; k += blockDim.x) {
     const int i = (me + (k / kPan) * P) * kPan + k % kPan;
     if (i < l) A[k * ld + i] += sh.shift;
   }
   __syncthreads();
-  // factor diagonal block K (this CTA's row block b); T goes to its slot and in place of the block
+  // factor diagonal block K (this CTA's): T goes to its slot
   auto diagonal = [&](int K) {
     double* D = A + (K / P) * kPan * ld + K * kPan;
     double* T = Ts + (K & 1) * kPan * kPan;
     chol_diag(D, ld, min(kPan, l - K * kPan), T, pivots, sh, bad);
-    for (int e = tid; e < kPan * kPan; e += 128) D[(e / kPan) * ld + e % kPan] = T[e];
   };
-  // T and Y of block K to the other CTAs
-  auto send = [&](int K) {
+  // T of block K, and its Y (by `count` warps), to the other CTAs
+  auto send_t = [&](int K) {
     double* T = Ts + (K & 1) * kPan * kPan;
+    for (int p = 0; p < P; ++p)
+      if (p != me && tid < kPan * kPan) cluster.map_shared_rank(T, p)[tid] = T[tid];
+  };
+  auto send_y = [&](int K, int rank, int count) {
     double* B = Bs + (K & 1) * kPan * lp;
     const double* Y = A + (K / P) * kPan * ld;
     const int half = K * kPan / 2;  // pairs of a row
     for (int p = 0; p < P; ++p) {
-      double* Tp = cluster.map_shared_rank(T, p);
       double* Bp = cluster.map_shared_rank(B, p);
-      if (p != me)
-        for (int e = tid; e < kPan * kPan; e += blockDim.x) Tp[e] = T[e];
-      for (int r = warp; r < kPan; r += warps)
+      for (int r = rank; r < kPan; r += count)
         for (int c = lane; c < half; c += 32)
           reinterpret_cast<double2*>(Bp + r * lp)[c] = reinterpret_cast<const double2*>(Y + r * ld)[c];
+    }
+  };
+  // X_K = T [Y_K, I] by `count` warps of its CTA; Rinv = X^T, column-major: Rinv[c + i l] = X[i][c]
+  double* Xg = Rinv + d.g_off;
+  auto store_x = [&](int K, int rank, int count) {
+    const double* T = Ts + (K & 1) * kPan * kPan;
+    const double* Y = A + (K / P) * kPan * ld;
+    const int chunks = (l + 31) / 32;
+    for (int w = rank; w < kPan * chunks; w += count) {
+      const int r = w / chunks, c = (w % chunks) * 32 + lane, i = K * kPan + r;
+      if (i >= l || c >= l) continue;
+      const double* t = T + r * kPan;
+      double even = 0.0, odd = 0.0;  // T is zero behind r
+      if (c < K * kPan) {
+        for (int q = 0; q <= r; q += 2) {
+          even = fma(t[q], Y[q * ld + c], even);
+          odd = fma(t[q + 1], Y[(q + 1) * ld + c], odd);
+        }
+        even += odd;
+      } else if (c <= i) {
+        even = t[c - K * kPan];
+      }
+      Xg[c + i * l] = even;
     }
   };
   if (me == 0) {
     if (warp < 4) diagonal(0);
     __syncthreads();
-    send(0);
+    send_t(0);
   }
   cluster.sync();
   for (int K = 0; K + 1 < nb; ++K) {
@@ -626,8 +655,12 @@ __global__ void __launch_bounds__(512) chol_cluster_kernel(const CholDesc* __res
       const int b = e >> 8, c = (e >> 4) & 15, r = e & 15, gb = me + b * P;
       if (gb <= K) continue;
       const double* a = A + (b * kPan + r) * ld + K * kPan;
-      double acc = 0.0;
-      for (int k = 0; k <= c; ++k) acc = fma(a[k], T[c * kPan + k], acc);
+      double even = 0.0, odd = 0.0;  // two chains: T is zero behind c
+      for (int k = 0; k <= c; k += 2) {
+        even = fma(a[k], T[c * kPan + k], even);
+        odd = fma(a[k + 1], T[c * kPan + k + 1], odd);
+      }
+      const double acc = even + odd;
       Pc[(b * kPan + r) * kPan + c] = acc;
       for (int p = 0; p < P; ++p) cluster.map_shared_rank(B, p)[c * lp + gb * kPan + r] = acc;
     }
@@ -645,20 +678,25 @@ __global__ void __launch_bounds__(512) chol_cluster_kernel(const CholDesc* __res
     __syncthreads();
     const int next = K + 1;
     const bool mine = next % P == me;
-    if (mine && warp < 4) {
+    if (mine) {  // the next diagonal block first, all warps
       const int b = next / P;
-      for (int e = tid; e < kPan * kPan; e += 128) {
+      for (int e = tid; e < kPan * kPan; e += blockDim.x) {
         const int r = e / kPan, c = e % kPan;
         if (c > r) continue;
         double* p = A + (b * kPan + r) * ld + next * kPan + c;
         const double* x = Pc + (b * kPan + r) * kPan;
         const double* y = Pc + (b * kPan + c) * kPan;
-        double acc = *p;
+        double even = *p, odd = 0.0;
 #pragma unroll
-        for (int k = 0; k < kPan; ++k) acc = fma(-x[k], y[k], acc);
-        *p = acc;
+        for (int k = 0; k < kPan; k += 2) {
+          even = fma(-x[k], y[k], even);
+          odd = fma(-x[k + 1], y[k + 1], odd);
+        }
+        *p = even + odd;
       }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
+      __syncthreads();
+    }
+    if (mine && warp < 4) {
       diagonal(next);
     } else if (!mine || (warp & 3)) {
       const int team = mine ? warps - 4 - (warps - 4) / 4 : warps;
@@ -690,28 +728,18 @@ __global__ void __launch_bounds__(512) chol_cluster_kernel(const CholDesc* __res
           a0[ld] = y;
         }
         at += items;
+        if (mine && gb == next) {  // its Y is final: to the other CTAs, beside the factorisation
+          asm volatile("bar.sync 2, %0;" ::"r"(team * 32) : "memory");
+          send_y(next, rank, team);
+        }
       }
+      if (K % P == me) store_x(K, rank, team);
     }
     __syncthreads();
-    if (mine) send(next);
+    if (mine) send_t(next);
     cluster.sync();
   }
-  // X_i = T_i [Y_i, I]; Rinv = X^T, column-major: Rinv[c + i l] = X[i][c]
-  double* Xg = Rinv + d.g_off;
-  for (int k = warp; k < own * kPan; k += warps) {
-    const int b = k / kPan, r = k % kPan, gb = me + b * P, i = gb * kPan + r;
-    if (i >= l) continue;
-    const double* rows = A + b * kPan * ld;
-    for (int c = lane; c < l; c += 32) {
-      double acc = 0.0;
-      if (c < gb * kPan) {
-        for (int q = 0; q <= r; ++q) acc = fma(rows[r * ld + gb * kPan + q], rows[q * ld + c], acc);
-      } else if (c <= i) {
-        acc = rows[r * ld + c];
-      }
-      Xg[c + i * l] = acc;
-    }
-  }
+  if ((nb - 1) % P == me) store_x(nb - 1, warp, warps);
 }
 
 // Rinv = L^-T from the Cholesky factor L (column-major, lower triangle, in G): one warp per
