@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cmath>
 #include <cstring>
 #include <map>
@@ -201,9 +202,19 @@ std::shared_ptr<PermPlan> upload_tables(const PermTables& t) {
   for (const auto& task : t.tasks) plan->bytes += 8.0 * double(task.nelem) * (1 + task.n_contrib);
   return plan;
 }
+// diagonal weights on the legs of a site tensor
+struct WeightPlan {
+  PlanMem mem;
+  MetaPtr out;
+  bool needs_zero = false;
+  int n_tasks = 0;
+  LegWeightTask* d_tasks = nullptr;
+  double bytes = 0;
+};
 std::mutex g_plan_mu;
 std::unordered_map<std::string, std::shared_ptr<PermPlan>> g_perm_plans;
 std::unordered_map<std::string, std::shared_ptr<GemmPlan>> g_gemm_plans;
+std::unordered_map<std::string, std::shared_ptr<WeightPlan>> g_weight_plans;
 CacheStats g_stats;
 
 struct TaskBuilder {
@@ -454,6 +465,7 @@ void clear_plan_caches() {
   std::lock_guard<std::mutex> lk(g_plan_mu);
   g_perm_plans.clear();
   g_gemm_plans.clear();
+  g_weight_plans.clear();
 }
 
 Tensor materialize(const Tensor& t) {
@@ -1229,11 +1241,81 @@ void sector_features(const TensorMeta& m, const History& last, int64_t chi, std:
 }
 
 // ======================================================================= simple update
+namespace {
+// sub-blocks of A (any charges on its legs) with the diagonals of the weights' blocks of those charges
+std::shared_ptr<WeightPlan> build_weight_plan(const TensorMeta& m, const std::array<const TensorMeta*, 4>& w) {
+  auto plan = std::make_shared<WeightPlan>();
+  plan->out = make_meta(m.sym, {w[0]->dom[0], w[1]->dom[0]}, {w[2]->cod[0], w[3]->cod[0], m.cod[2]});
+  const TensorMeta& o = *plan->out;
+  std::vector<LegWeightTask> tasks;
+  int64_t written = 0;
+  for (size_t si = 0; si < m.sectors.size(); ++si) {
+    const int q = m.sectors[si], oq = o.index(q);
+    if (oq < 0) throw std::runtime_error("weights: output sector missing");
+    for (const auto& f1 : m.cdom->trees[m.cdom->index(q)])
+      for (const auto& f2 : m.ccod->trees[m.ccod->index(q)]) {
+        LegWeightTask k{};
+        int64_t n = 1;
+        bool present = true;
+        for (int leg = 0; leg < 5; ++leg) {
+          k.dims[leg] = leg < 2 ? f1.dims[leg] : f2.dims[leg - 2];
+          n *= k.dims[leg];
+          if (leg == 4) break;
+          const int wi = w[leg]->index(leg < 2 ? f1.qu[leg] : f2.qu[leg - 2]);
+          present = present && wi >= 0;
+          if (wi < 0) continue;
+          if (w[leg]->rows[wi] != k.dims[leg] || w[leg]->cols[wi] != k.dims[leg])
+            throw std::runtime_error("weights: a weight does not match its leg");
+          k.weight[leg] = w[leg]->offset[wi];
+          k.weight_step[leg] = w[leg]->rows[wi] + 1;
+        }
+        if (!present || n == 0) continue;  // a charge that a weight does not carry: zero
+        k.src = m.offset[si] + m.cdom->left_offset(f1) + m.ccod->left_offset(f2) * m.rows[si];
+        k.dst = o.offset[oq] + o.cdom->left_offset(f1) + o.ccod->left_offset(f2) * o.rows[oq];
+        sub_strides(f1, f2, m.rows[si], k.src_stride);
+        sub_strides(f1, f2, o.rows[oq], k.dst_stride);
+        for (k.first = 0; k.first < n; k.first += 256) {
+          k.last = std::min<int64_t>(n, k.first + 256);
+          tasks.push_back(k);
+        }
+        written += n;
+      }
+  }
+  plan->n_tasks = int(tasks.size());
+  plan->needs_zero = written != o.size;
+  plan->bytes = 16.0 * double(written);
+  plan->d_tasks = plan->mem.table(tasks);
+  return plan;
+}
+}  // namespace
+
+// The weights are diagonal (identities, singular values and their square roots or inverses), so contracting
+// them (TimePropagator.cpp:112-186) multiplies every entry by one diagonal entry per leg.
 Tensor apply_weights(const Tensor& A, const Tensor& wL, const Tensor& wT, const Tensor& wR, const Tensor& wB) {
-  Tensor t = contract(A, twist(wL, 1), {1, -2, -3, -4, -5}, {-1, 1}, 2);
-  t = contract(t, twist(wT, 1), {-1, 1, -3, -4, -5}, {-2, 1}, 2);
-  t = contract(t, wR, {-1, -2, 1, -4, -5}, {1, -3}, 2);
-  return contract(t, wB, {-1, -2, -3, 1, -5}, {1, -4}, 2);
+  const Tensor t = materialize(A);
+  const std::array<Tensor, 4> w{materialize(wL), materialize(wT), materialize(wR), materialize(wB)};
+  std::ostringstream os;
+  os << t.meta->id;
+  for (const Tensor& x : w) os << '|' << x.meta->id;
+  const std::string key = os.str();
+  std::shared_ptr<WeightPlan> plan;
+  {
+    std::lock_guard<std::mutex> lk(g_plan_mu);
+    auto it = g_weight_plans.find(key);
+    if (it != g_weight_plans.end()) plan = it->second;
+  }
+  if (!plan) {
+    plan = build_weight_plan(*t.meta, {w[0].meta.get(), w[1].meta.get(), w[2].meta.get(), w[3].meta.get()});
+    std::lock_guard<std::mutex> lk(g_plan_mu);
+    if (g_weight_plans.size() >= kPlanCacheCap) g_weight_plans.clear();
+    g_weight_plans[key] = plan;
+  }
+  Tensor out = plan->needs_zero ? zeros(plan->out) : empty_like_meta(plan->out);
+  prof_begin(K_DIAG, stream());
+  launch_leg_weights(plan->d_tasks, plan->n_tasks, {{w[0].data(), w[1].data(), w[2].data(), w[3].data()}}, t.data(),
+                     out.data(), stream());
+  prof_end(K_DIAG, stream(), plan->bytes);
+  return out;
 }
 
 namespace {
