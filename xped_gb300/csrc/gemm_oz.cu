@@ -70,6 +70,7 @@ constexpr int kOzDrainWarps = 16, kOzProducer = kOzDrainWarps, kOzMma = kOzDrain
 constexpr int kOzWarps = kOzDrainWarps + 2, kOzThreads = kOzWarps * 32;
 constexpr int kDrainCols = ON / (kOzDrainWarps / 4);  // columns of a drain warp
 constexpr long long kOzSpin = 1ll << 26;
+constexpr int kReduceThreads = 256;
 constexpr int kPackRows = 32;                       // rows of a slicing cluster
 constexpr uint32_t kSboBytes = 128;                 // next 8-row group
 // A: seven separate 128-row pieces.  B: the seven 64-row pieces stacked into one 448-row operand (row
@@ -591,29 +592,29 @@ __global__ void __launch_bounds__(256) oz_splitk_reduce_kernel(const xgb_gemm_de
   const xgb_gemm_desc d = descs[r.g];
   const bool swp = groups[r.g].swap != 0;
   const int64_t pm = swp ? d.n : d.m, pn = swp ? d.m : d.n;
-  // blockIdx.y: a 1024-element part of the tile (eight CTAs per tile keep the sums spread over the SMs);
-  // consecutive threads take consecutive rows of C (tile rows, or tile columns of a swapped group)
-  const int e0 = int(blockIdx.y) * 1024, e1 = e0 + 1024 < OM * ON ? e0 + 1024 : OM * ON;
-  for (int e = e0 + threadIdx.x; e < e1; e += blockDim.x) {
-    const int li = swp ? e / ON : e % OM, lj = swp ? e % ON : e / OM;  // tile-local row / column
-    const int64_t i = int64_t(r.tm) * OM + li, j = int64_t(r.tn) * ON + lj;
-    if (i >= pm || j >= pn) continue;
-    const int64_t w = li + int64_t(lj) * OM;
-    const double* part = ws + int64_t(r.first) * OM * ON + w;
-    double acc = part[0];
-    // eight loads in flight: one after the other a tile cut nineteen ways took 12 us
-    for (int p = 1; p < r.count; p += 8) {
-      double x[8];
+  // blockIdx.y: 256 elements of the tile, one per thread (the sums are chains of dependent loads: four per thread took
+  // 12 us on tiles cut nineteen ways); consecutive threads take consecutive rows of C (tile rows, or tile columns of a
+  // swapped group)
+  static_assert(OM * ON % kReduceThreads == 0);
+  const int e = int(blockIdx.y) * kReduceThreads + int(threadIdx.x);
+  const int li = swp ? e / ON : e % OM, lj = swp ? e % ON : e / OM;  // tile-local row / column
+  const int64_t i = int64_t(r.tm) * OM + li, j = int64_t(r.tn) * ON + lj;
+  if (i >= pm || j >= pn) return;
+  const int64_t w = li + int64_t(lj) * OM;
+  const double* part = ws + int64_t(r.first) * OM * ON + w;
+  double acc = part[0];
+  // eight loads in flight
+  for (int p = 1; p < r.count; p += 8) {
+    double x[8];
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (p + u < r.count) x[u] = __ldg(part + int64_t(p + u) * OM * ON);
+    for (int u = 0; u < 8; ++u)
+      if (p + u < r.count) x[u] = __ldg(part + int64_t(p + u) * OM * ON);
 #pragma unroll
-      for (int u = 0; u < 8; ++u)
-        if (p + u < r.count) acc += x[u];
-    }
-    double* c = C + d.c_off + (swp ? j + i * d.ldc : i + j * d.ldc);
-    *c = beta != 0.0 ? fma(alpha, acc, beta * *c) : alpha == 1.0 ? acc : alpha * acc;
+    for (int u = 0; u < 8; ++u)
+      if (p + u < r.count) acc += x[u];
   }
+  double* c = C + d.c_off + (swp ? j + i * d.ldc : i + j * d.ldc);
+  *c = beta != 0.0 ? fma(alpha, acc, beta * *c) : alpha == 1.0 ? acc : alpha * acc;
 }
 
 std::once_flag g_oz_attr;
@@ -729,7 +730,7 @@ void launch_oz_gemm(const xgb_gemm_desc* d_descs, const OzGroup* d_groups, const
                                                      beta, ws, gemm_tc_error_flag());
   count_launch();
   if (n_red > 0) {
-    oz_splitk_reduce_kernel<<<dim3(unsigned(n_red), (OM * ON + 1023) / 1024), 256, 0, s>>>(d_descs, d_groups, d_red,
+    oz_splitk_reduce_kernel<<<dim3(unsigned(n_red), OM * ON / kReduceThreads), kReduceThreads, 0, s>>>(d_descs, d_groups, d_red,
                                                                                             ws, C, alpha, beta);
     count_launch();
   }
