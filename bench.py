@@ -492,8 +492,8 @@ def permute_roofline(degs=(20, 40, 60, 40, 20), reps=5):
     # DRAM read + write of one launch from an ncu capture of the [14, 28, 42, 28, 14] case (42.5 M
     # doubles: 344.7 MB read, 294.2 MB written, the rest of the output still in L2 at the kernel's end),
     # scaled by the element count (the traffic grows in proportion)
-    traffic = (344.672e6 + 294.158e6) * (algorithmic / 16.0) / 42526512.0
-    return {"kernel": "permute_rows_wide_kernel", "elements": int(algorithmic // 16),
+    traffic = (357.380e6 + 307.415e6) * (algorithmic / 16.0) / 42526512.0
+    return {"kernel": "permute_planes_kernel", "elements": int(algorithmic // 16),
             "gbytes_moved": algorithmic / 1e9, "launches": int(n), "ms_per_launch": per_launch, "achieved": gbs,
             "peak": hbm, "unit": "GB/s", "frac": gbs / hbm, "bound": "hbm", "traffic": traffic,
             "traffic_source": "ncu capture of the deg [14, 28, 42, 28, 14] case scaled by elements",
@@ -1087,9 +1087,7 @@ def roofline(prof, steps, fp64_peak=None):
     out["frac"] = out["achieved"] / out["peak"]
     # DRAM bytes per launch of the dominant kernel from one ncu capture (profiles/): the chosen
     # step's working sets are L2-resident
-    traffic = {"svd_jacobi": (0.355e6, "ncu capture of one svd_cluster_kernel launch of the projected l x l "
-                                       "factors, U(1) D=6 chi=128 (dram__bytes_read.sum 322 KB + write 33 KB)"),
-               "gemm_tc": (7.025e9, "ncu capture, SU(2) Tensor<2,2> product (6.613 GB read + 0.412 GB written)"),
+    traffic = {"gemm_tc": (7.025e9, "ncu capture, SU(2) Tensor<2,2> product (6.613 GB read + 0.412 GB written)"),
                "gemm_f64tc": (68.27e6, "ncu one-pass capture of the 76 oz_gemm_kernel launches of one chosen U(1) D=6 "
                                        "chi=128 step (bench.py --profile-step): 67.44 MB read + 0.83 MB written per "
                                        "launch, average (the packed slices of the sector blocks)"),
