@@ -104,6 +104,7 @@ struct PlaneForm {
   bool transpose = false;  // read along the source's unit-stride leg, through shared memory
   bool narrow = true;      // offsets within a task and its number of chunks fit 32 bits
   bool single = true;      // one source per task (no SU(2) sums)
+  int64_t elems = 0;       // output elements
 };
 struct PlanePlan {
   std::vector<PlaneTask> tasks;

@@ -17,7 +17,7 @@
 // pipe 64 cycles, predicated off or not, and multiplying made the 1.4 GB permutes 1.2 ms instead of 0.54.
 // Bound by HBM where the tensor is large, by the number of warp instructions for sums over short legs, and for the
 // smallest by the dependent loads of one batch (6.5 us under the profiler).  Measured, before -> now (U(1), 5 sectors,
-// legs up to 60, 2.8 GB moved): (0,2,1,3) 803 -> 540 us, (2,3,0,1) 3440 -> 517, (2,0,3,1) 1475 -> 629; SU(2) 2.6 M
+// legs up to 60, 2.8 GB moved): (0,2,1,3) 803 -> 540 us, (2,3,0,1) 3440 -> 438, (2,0,3,1) 1475 -> 499; SU(2) 2.6 M
 // elements: (2,0,3,1) with 270 sources of 158 sub-blocks 48 -> 35 us, (1,0,3,2) 27 -> 17.
 #include <cuda_runtime.h>
 
@@ -321,7 +321,14 @@ void launch_permute(const PlaneTask* d_tasks, const int64_t* d_start, int n_task
   if (n_planes <= 0 || n_tasks <= 0) return;
   auto pick = [&](auto single) {
     constexpr bool kSingle = decltype(single)::value;
-    if (form.transpose) return form.narrow ? launch_form<32, true, kSingle, int32_t> : launch_form<32, true, kSingle, int64_t>;
+    // Tiles copied from a single source: 64-bit offsets make the copy loop plain pointer additions, and are the faster
+    // from 4 M elements on (us, 32- / 64-bit offsets: 2.7 M elements 17.1 / 18.3, 7.3 M 40.4 / 35.9, 23 M 94 / 80,
+    // 177 M 638 / 499); below, and for sums (34.5 / 37.8 at 2.6 M), decoding in 32 bits is.
+    constexpr int64_t kWideFrom = 4 << 20;
+    if (form.transpose) {
+      if (form.narrow && (!kSingle || form.elems < kWideFrom)) return launch_form<32, true, kSingle, int32_t>;
+      return launch_form<32, true, kSingle, int64_t>;
+    }
     if (!form.narrow) return launch_form<32, false, kSingle, int64_t>;
     switch (form.group) {
       case 32: return launch_form<32, false, kSingle, int32_t>;
@@ -418,8 +425,8 @@ PlanePlan plan_planes(const xgb_perm_task* tasks, int n_tasks, const xgb_perm_co
       int64_t span = 0;
       for (int i = 0; i < k.rank; ++i) {
         if (k.dims[i] == 1) continue;  // such a leg is not walked
-        if (std::abs(stride[i]) > INT32_MAX / 2048) return false;
-        span += std::abs(stride[i]) * (int64_t(k.dims[i]) + 32 * kUnroll);
+        if (std::abs(stride[i]) > INT32_MAX) return false;
+        span += std::abs(stride[i]) * (int64_t(k.dims[i]) + 32 * kFlight);
       }
       return span <= INT32_MAX;
     };
@@ -471,6 +478,7 @@ PlanePlan plan_planes(const xgb_perm_task* tasks, int n_tasks, const xgb_perm_co
     plan.tasks.push_back(p);
     plan.start.push_back(plan.start.back() + planes);
   }
+  plan.form.elems = int64_t(elems);
   // lanes per chunk: about four elements each or more
   const double avg = elems > 0 ? weighted / elems : 1.0;
   plan.form.group = plan.form.transpose || !plan.form.narrow || avg >= 96 ? 32 : avg >= 48 ? 16 : avg >= 24 ? 8 : 4;
