@@ -568,6 +568,7 @@ __global__ void __launch_bounds__(512) chol_cluster_kernel(const CholDesc* __res
   const CholDesc d = descs[blockIdx.x / P];
   const int l = int(d.l), nb = (l + kPan - 1) / kPan, lp = nb * kPan, ld = lp + 2, most = (nb + P - 1) / P;
   if (l == 0) return;  // the whole cluster
+  cluster.barrier_arrive();  // completed before the first store to another CTA, which has to be running by then
   const int own = me < nb ? (nb - me + P - 1) / P : 0;  // row blocks me, me + P, ...
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, warps = blockDim.x >> 5;
   double* A = chol_sm;
@@ -642,11 +643,10 @@ __global__ void __launch_bounds__(512) chol_cluster_kernel(const CholDesc* __res
       Xg[c + i * l] = even;
     }
   };
-  if (me == 0) {
-    if (warp < 4) diagonal(0);
-    __syncthreads();
-    send_t(0);
-  }
+  if (me == 0 && warp < 4) diagonal(0);
+  cluster.barrier_wait();
+  __syncthreads();
+  if (me == 0) send_t(0);
   cluster.sync();
   for (int K = 0; K + 1 < nb; ++K) {
     const double* T = Ts + (K & 1) * kPan * kPan;
