@@ -374,8 +374,9 @@ int xgb_grouped_gemm_f64_config(int tile, int split_waves, int n, const xgb_gemm
   try {
     for (int g = 0; g < n; ++g)
       if (descs[g].m < 0 || descs[g].n < 0 || descs[g].k < 0) return set_error(XGB_E_BADPLAN, "negative GEMM extent");
-    run_gemm_f64_config(descs, n, {tile, split_waves}, A, B, C, alpha, beta,
-                        stream_ ? static_cast<cudaStream_t>(stream_) : stream());
+    cudaStream_t s = stream_ ? static_cast<cudaStream_t>(stream_) : stream();
+    AllocScope alloc(s);
+    run_gemm_f64_config(descs, n, {tile, split_waves}, A, B, C, alpha, beta, s);
     return check_cuda(cudaGetLastError(), "gemm launch");
   } catch (const std::bad_alloc&) {
     return XGB_E_OOM;

@@ -45,6 +45,7 @@ std::atomic<int64_t> g_launches{0};
 std::atomic<bool> g_lanes_used{false};
 thread_local std::string g_err;
 thread_local int t_lane = 0;
+thread_local cudaStream_t t_alloc = nullptr;  // stream of an AllocScope
 
 // The worker host thread of lane 1: runs one task at a time, handed over under a mutex.
 class LaneWorker {
@@ -179,10 +180,13 @@ int check_cuda(cudaError_t e, const char* what) {
                    std::string(what) + ": " + cudaGetErrorString(e));
 }
 
+AllocScope::AllocScope(cudaStream_t s) : saved(t_alloc) { t_alloc = s; }
+AllocScope::~AllocScope() { t_alloc = saved; }
+
 void* dev_alloc(size_t bytes) {
   if (bytes == 0) bytes = 8;
   void* p = nullptr;
-  cudaError_t e = cudaMallocAsync(&p, bytes, stream());
+  cudaError_t e = cudaMallocAsync(&p, bytes, t_alloc ? t_alloc : stream());
   if (e != cudaSuccess) {
     (void)cudaGetLastError();
     set_error(XGB_E_OOM, std::string("cudaMallocAsync: ") + cudaGetErrorString(e));
@@ -192,7 +196,7 @@ void* dev_alloc(size_t bytes) {
 }
 
 void dev_free(void* p) {
-  if (p && g_rt.ready) cudaFreeAsync(p, stream());
+  if (p && g_rt.ready) cudaFreeAsync(p, t_alloc ? t_alloc : stream());
 }
 
 // ======================================================================= instrumentation
@@ -1046,6 +1050,7 @@ int xgb_grouped_gemm(int precision, int n_groups, const xgb_gemm_desc* descs, co
   if (n_groups < 0) return set_error(XGB_E_BADPLAN, "n_groups < 0");
   XGB_GUARD_BEGIN
   cudaStream_t s = pick(stream_);
+  AllocScope alloc(s);
   for (int g = 0; g < n_groups; ++g)
     if (descs[g].m < 0 || descs[g].n < 0 || descs[g].k < 0) return set_error(XGB_E_BADPLAN, "negative GEMM extent");
   if (precision == XGB_PREC_F64TC) {
@@ -1146,6 +1151,7 @@ int xgb_permute(int n_tasks, const xgb_perm_task* tasks, int n_contrib, const xg
   XGB_REQUIRE_INIT();
   XGB_GUARD_BEGIN
   cudaStream_t s = pick(stream_);
+  AllocScope alloc(s);
   if (const int rc = check_permute(n_tasks, tasks, n_contrib)) return rc;
   const PlanePlan plan = plan_planes(tasks, n_tasks, contribs);
   if (plan.start.back() == 0) return XGB_OK;
@@ -1182,6 +1188,7 @@ int xgb_batched_svd(int n, const xgb_svd_desc* descs, const double* A, double* U
   XGB_REQUIRE_INIT();
   XGB_GUARD_BEGIN
   cudaStream_t s = pick(stream_);
+  AllocScope alloc(s);
   std::vector<int64_t> off(size_t(std::max(n, 0)), 0);
   int64_t acc = 0, maxk = 0;
   for (int i = 0; i < n; ++i) {
@@ -1208,6 +1215,7 @@ int xgb_truncate(int n_sectors, const int64_t* s_begin_host, const int32_t* dege
   XGB_GUARD_BEGIN
   if (n_sectors <= 0) return set_error(XGB_E_BADPLAN, "truncation needs at least one sector");
   cudaStream_t st = pick(stream_);
+  AllocScope alloc(st);
   const int64_t total = s_begin_host[n_sectors];
   if (total <= 0) return set_error(XGB_E_BADPLAN, "no singular values");
   auto* db = upload(s_begin_host, size_t(n_sectors) + 1, st);
@@ -1229,6 +1237,7 @@ int xgb_batched_qr(int n, const xgb_qr_desc* descs, const double* A, double* Q, 
   XGB_REQUIRE_INIT();
   XGB_GUARD_BEGIN
   cudaStream_t s = pick(stream_);
+  AllocScope alloc(s);
   std::vector<int64_t> off(size_t(std::max(n, 0)), 0);
   int64_t acc = 0;
   for (int i = 0; i < n; ++i) {
@@ -1270,6 +1279,7 @@ int xgb_copy2d_batched(int n, const xgb_copy2d_desc* descs, const double* src, d
   XGB_GUARD_BEGIN
   if (n <= 0) return XGB_OK;
   cudaStream_t s = pick(stream_);
+  AllocScope alloc(s);
   int64_t mx = 0;
   for (int i = 0; i < n; ++i) mx = std::max(mx, descs[i].rows * descs[i].cols);
   auto* dd = upload(descs, size_t(n), s);
@@ -1284,6 +1294,7 @@ int xgb_diag_from_vec(int n, const xgb_copy2d_desc* descs, int fn, const double*
   XGB_GUARD_BEGIN
   if (n <= 0) return XGB_OK;
   cudaStream_t s = pick(stream_);
+  AllocScope alloc(s);
   int64_t mx = 0;
   for (int i = 0; i < n; ++i) mx = std::max(mx, descs[i].rows);
   auto* dd = upload(descs, size_t(n), s);
@@ -1298,6 +1309,7 @@ int xgb_diag_apply(int n, const xgb_copy2d_desc* descs, int fn, double* x, void*
   XGB_GUARD_BEGIN
   if (n <= 0) return XGB_OK;
   cudaStream_t s = pick(stream_);
+  AllocScope alloc(s);
   int64_t mx = 0;
   for (int i = 0; i < n; ++i) mx = std::max(mx, std::max(descs[i].rows, descs[i].cols));
   auto* dd = upload(descs, size_t(n), s);

@@ -55,8 +55,19 @@ void order_after_lanes(cudaStream_t s);
 bool runtime_ready();  // xgb_init has run
 int set_error(int code, const std::string& msg);
 int check_cuda(cudaError_t e, const char* what);
-void* dev_alloc(size_t bytes);          // stream-ordered; throws std::bad_alloc on failure
+// stream-ordered on this host thread's stream() or, inside an AllocScope, on the scope's stream; throws
+// std::bad_alloc on failure
+void* dev_alloc(size_t bytes);
 void dev_free(void* p);
+// For entries that take the caller's stream: their temporaries are allocated and freed in the order of that
+// stream, so that none is handed to another allocation while the caller's kernels still read it.
+struct AllocScope {
+  cudaStream_t saved;
+  explicit AllocScope(cudaStream_t s);
+  ~AllocScope();
+  AllocScope(const AllocScope&) = delete;
+  AllocScope& operator=(const AllocScope&) = delete;
+};
 void count_launch(int n = 1);
 int num_sms();
 
