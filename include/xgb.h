@@ -187,8 +187,9 @@ int xgb_batched_svd(int n, const xgb_svd_desc* descs, const double* A, double* U
    whose host framework owns all device allocations, or a service with a
    fixed device-memory budget).  No counterpart in the reference: it exists
    only for embedders of this library.  Same descriptors, outputs and kernels
-   as xgb_batched_svd (cooperative sweeps for blocks wider than 512, clusters
-   or single CTAs for the others), but the workspace comes from
+   as xgb_batched_svd (cooperative grids for blocks wider than 512 and for those
+   from 512 on that no cluster holds, clusters or single CTAs for the others),
+   but the workspace comes from
    one fixed 16 MiB device array per GPU
    (xgb_batched_svd_noalloc_capacity_bytes()) that the library holds until
    exit; batches needing more return XGB_E_UNSUPPORTED (one square block of
@@ -204,7 +205,8 @@ int xgb_batched_svd_noalloc(int n, const xgb_svd_desc* descs, const double* A, d
 size_t xgb_batched_svd_noalloc_capacity_bytes(void);
 
 /* Diagnostics of the last batched SVD, 6 ints per block: FP32 sweeps, FP64
-   sweeps, cycles/1024 spent in the FP32 sweeps, FP64 refinement iterations,
+   sweeps, cycles/1024 spent in the FP32 sweeps (in the QR factor of the blocks
+   that no cluster holds), FP64 refinement iterations,
    then the cycles/1024 spent in the FP64 sweeps and in the last stage
    (FP64 sweeps of the narrower blocks and output); returns the number of
    blocks written */

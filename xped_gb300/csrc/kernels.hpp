@@ -128,8 +128,7 @@ void launch_permute(const PlaneTask* d_tasks, const int64_t* d_start, int n_task
                     const PlaneSource* d_sources, const double* src, double* dst, cudaStream_t s);
 // the plan walked on the host by the kernel's index arithmetic
 void permute_planes_host(const PlanePlan& plan, const double* src, double* dst);
-// h_descs: host copy of the descriptors (the FP32 sweeps and the polish of the widest blocks run one block at a
-// time on a cooperative grid; nullptr keeps every block on clusters)
+// h_descs: host copy of the descriptors (on lane 0 the widest blocks run one at a time on a cooperative grid)
 void launch_svd(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, const int64_t* d_work_off, int n,
                 const double* A, double* U, double* S, double* Vt, double* work, cudaStream_t s);
 void launch_truncate(int n_sectors, const int64_t* d_s_begin, const int32_t* d_deg, const double* sv, int64_t total,

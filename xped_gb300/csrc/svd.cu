@@ -25,6 +25,8 @@
 //      Newton steps, s = c t; its angle t comes from FP32 arithmetic on exactly rescaled inputs).
 //   5. sigma_j = |w_j| sorted descending (ties by column), u_j = w_j / sigma_j, v_j = V[:, j]; every pair
 //      sign-normalised (sign rule below).
+// Blocks too large for a cluster's shared memory and at least kFactorN wide take FP64 Jacobi behind a column-pivoted QR
+// instead (svd_factor_kernel).
 // All control is on the device: every stage is launched once, reads the block's convergence state and
 // returns when there is nothing to do, so the host neither waits nor decides.
 //
@@ -66,9 +68,13 @@ constexpr double kFloor64 = 1.0e-30;
 constexpr int kSmemLimit = 220 * 1024;
 // blocks up to kSmallN columns run start to finish in one CTA (svd_small_kernel)
 constexpr int kSmallN = 24;
-// blocks wider than this take the cooperative form (one launch per block) of the FP32 sweeps of pass 0, and of
-// those of pass 1 and the FP64 sweeps
-constexpr int kGridN = 640, kGridN2 = 512;
+// blocks wider than this take the cooperative form (one launch per block) of the FP32 sweeps of pass 1 and of the
+// FP64 sweeps
+constexpr int kGridN = 512;
+// blocks at least this wide whose columns no cluster holds take svd_factor_kernel
+constexpr int kFactorN = 512;
+constexpr int kFactorCols = 4;  // columns of its Jacobi blocks
+constexpr int kFactorSweeps = 80;
 
 template <class T>
 __device__ __forceinline__ T wsum(T v) {
@@ -1521,20 +1527,25 @@ __host__ __device__ __forceinline__ int sweep_ctas(int pass, int64_t mm, int64_t
   return sh.P ? sh.P : most;  // (too large for any: jacobi32_global or block_jacobi on all of them)
 }
 
+// Whether a block takes svd_factor_kernel; `grid_most`: most CTAs per cluster, 0 where no cooperative grid is launched.
+__host__ __device__ __forceinline__ bool factored(int64_t mm, int64_t nn, int grid_most) {
+  return grid_most && nn >= kFactorN && shape32(0, mm, nn, grid_most, kSmemLimit).P == 0;
+}
+
 // FP32 sweeps of the blocks that take lo < CTAs <= hi, one cluster of `hi` CTAs per block; the CTAs that a
 // block does not take leave at once (a cluster barrier waits for the threads that have not exited).  The launch
 // with lo = 0 also decomposes the small blocks, start to finish, beside the others' sweeps.  `widest`: blocks of
-// more columns take the cooperative grid.
+// more columns take the cooperative grid (pass 1).
 __global__ void __launch_bounds__(kThreads)
     svd_sweeps_kernel(const xgb_svd_desc* __restrict__ descs, const int64_t* __restrict__ work_off,
                       const double* __restrict__ A, double* __restrict__ U, double* __restrict__ S,
                       double* __restrict__ Vt, double* __restrict__ work, int* __restrict__ sweep_stats, int pass, int lo,
-                      int most, int widest, int smem_bytes) {
+                      int most, int widest, int grid_most, int smem_bytes) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cg::cluster_group cl = cg::this_cluster();
   const int ctas = int(cl.num_blocks()), sector = int(blockIdx.x) / ctas;
   const Block k = block_of(descs[sector], work_off[sector], A, U, Vt, work);
-  if (k.nn == 0 || k.nn > widest) return;  // uniform across the cluster
+  if (k.nn == 0 || k.nn > widest || factored(k.mm, k.nn, grid_most)) return;  // uniform across the cluster
   int* st6 = sweep_stats ? sweep_stats + 6 * sector : nullptr;
   if (small_block(k.mm, k.nn)) {
     if (pass == 0 && lo == 0 && cl.block_rank() == 0) svd_small(descs[sector], A, U, S, Vt, st6, smem_raw);
@@ -1547,17 +1558,17 @@ __global__ void __launch_bounds__(kThreads)
   fp32_pass<kFormCluster>(cl, c, P, k, pass, reinterpret_cast<float*>(smem_raw), smem_bytes, st6);
 }
 
-// The same for one block wider than kGridN (pass 0) or kGridN2: a cooperative grid of nn / 32 CTAs with grid barriers.
+// Pass 1 of one block wider than kGridN: a cooperative grid of nn / 32 CTAs with grid barriers.
 __global__ void __launch_bounds__(kThreads)
     svd_sweeps_grid_kernel(const xgb_svd_desc* __restrict__ descs, const int64_t* __restrict__ work_off, int sector,
                            const double* __restrict__ A, double* __restrict__ U, double* __restrict__ Vt,
-                           double* __restrict__ work, int* __restrict__ sweep_stats, int pass, int smem_bytes) {
+                           double* __restrict__ work, int* __restrict__ sweep_stats, int smem_bytes) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cg::grid_group gg = cg::this_grid();
   const Block k = block_of(descs[sector], work_off[sector], A, U, Vt, work);
-  if (pass && __ldcg(k.misc + kBig) == 0) return;  // uniform across the grid
+  if (__ldcg(k.misc + kBig) == 0) return;  // uniform across the grid
   const Ctx c = make_ctx(int(blockIdx.x), int(gridDim.x));
-  fp32_pass<kFormGrid>(gg, c, int(gridDim.x), k, pass, reinterpret_cast<float*>(smem_raw), smem_bytes,
+  fp32_pass<kFormGrid>(gg, c, int(gridDim.x), k, 1, reinterpret_cast<float*>(smem_raw), smem_bytes,
                   sweep_stats ? sweep_stats + 6 * sector : nullptr);
 }
 
@@ -1620,11 +1631,11 @@ template <int kMode>
 __global__ void __launch_bounds__(256)
     svd_product_kernel(const xgb_svd_desc* __restrict__ descs, const int64_t* __restrict__ work_off,
                        const double* __restrict__ A, double* __restrict__ U, double* __restrict__ Vt,
-                       double* __restrict__ work, int it) {
+                       double* __restrict__ work, int it, int grid_most) {
   __shared__ double sm[4 * 16 * (kTile + 1)];
   const int sector = blockIdx.y;
   const Block k = block_of(descs[sector], work_off[sector], A, U, Vt, work);
-  if (k.nn == 0 || small_block(k.mm, k.nn)) return;
+  if (k.nn == 0 || small_block(k.mm, k.nn) || factored(k.mm, k.nn, grid_most)) return;
   const int64_t nt = svd_tiles(k.nn), mt = svd_tiles(k.mm);
   int64_t t = blockIdx.x;
   if (t >= (kMode == kProdAV ? mt * nt : kMode == kProdGram ? 2 * nt * nt : mt * nt + nt * nt)) return;
@@ -1660,12 +1671,13 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     svd_update_kernel(const xgb_svd_desc* __restrict__ descs, const int64_t* __restrict__ work_off,
                       const double* __restrict__ A, double* __restrict__ U, double* __restrict__ Vt,
-                      double* __restrict__ work, int it) {
+                      double* __restrict__ work, int it, int grid_most) {
   __shared__ double red[8];
   const int sector = blockIdx.y;
   const Block k = block_of(descs[sector], work_off[sector], A, U, Vt, work);
   const int64_t nn = k.nn;
   if (nn == 0 || small_block(k.mm, nn) || int64_t(blockIdx.x) * 256 >= nn * nn) return;
+  if (factored(k.mm, nn, grid_most)) return;
   if (it > 0 && !iter_on(k.misc, it - 1)) return;
   double gmax = 0;
   for (int64_t j = threadIdx.x; j < nn; j += 256) gmax = fmax(gmax, k.G[j * (nn + 1)]);
@@ -1723,7 +1735,7 @@ __device__ void polish(Group& g, const Ctx& c, const Block& k, int ctas, double*
   }
 }
 
-// The sweeps of `polish` for one block wider than kGridN2, over a cooperative grid.
+// The sweeps of `polish` for one block wider than kGridN, over a cooperative grid.
 __global__ void __launch_bounds__(kThreads)
     svd_polish_grid_kernel(const xgb_svd_desc* __restrict__ descs, const int64_t* __restrict__ work_off, int sector,
                            const double* __restrict__ A, double* __restrict__ U, double* __restrict__ Vt,
@@ -1741,13 +1753,13 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads)
     svd_finish_kernel(const xgb_svd_desc* __restrict__ descs, const int64_t* __restrict__ work_off,
                       const double* __restrict__ A, double* __restrict__ U, double* __restrict__ S,
                       double* __restrict__ Vt, double* __restrict__ work, int* __restrict__ sweep_stats,
-                      int smem_bytes, int grid_min) {
+                      int smem_bytes, int grid_min, int grid_most) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   cg::cluster_group cl = cg::this_cluster();
   const int sector = blockIdx.x / kCluster;
   const xgb_svd_desc d = descs[sector];
   const Block k = block_of(d, work_off[sector], A, U, Vt, work);
-  if (k.nn == 0 || small_block(k.mm, k.nn)) return;  // uniform across the cluster
+  if (k.nn == 0 || small_block(k.mm, k.nn) || factored(k.mm, k.nn, grid_most)) return;  // uniform across the cluster
   const Ctx c = make_ctx(int(cl.block_rank()), kCluster);
   const long long t0 = clock64();
   int* st6 = sweep_stats ? sweep_stats + 6 * sector : nullptr;
@@ -1762,6 +1774,313 @@ __global__ void __cluster_dims__(kCluster, 1, 1) __launch_bounds__(kThreads)
   if (st6 && c.rank == 0 && c.tid == 0) {
     st6[3] = done;
     st6[5] = int((clock64() - t0) >> 10);
+  }
+}
+
+// ---------------------------------------------------------------- wide blocks: QR, then Jacobi on R^T
+// Blocks from kFactorN columns on that no cluster's shared memory holds (beyond 640 columns, or tall): FP64 throughout
+// on a cooperative grid of one CTA per 2 kFactorCols columns (every SM at most), one launch per block.
+//   1. Householder QR with column pivoting, op(A) P = Q R (Businger-Golub: the largest remaining column
+//      norm is pivoted in; the norms are downdated and recomputed under cancellation, the rule of
+//      LAPACK's xLAQP2).  Per step CTA 0 picks the pivot, swaps it into place and forms the reflector,
+//      and then every warp applies it to one trailing column.
+//   2. Block Jacobi on X = R^T (nn x nn): the rows of a column-pivoted R are graded, so the columns of X are close
+//      to orthogonal and converge in 11 to 14 sweeps (the preconditioning of Drmac and Veselic).
+//   3. X V = W with W_j = sigma_j u_j gives R = V Sigma U_X^T, so op(A) = (Q V) Sigma (P U_X)^T: each
+//      warp applies the reflectors to one column [V_j; 0] (no barriers), and P U_X is a row scatter.
+// Bound by the latency of the factor's column steps (two grid barriers each: 50k of 340k kilocycles at 864 columns) and
+// of the sweeps' grid barriers and FP64 dot products.  Measured against FP32 sweeps of op(A) itself with accumulated
+// rotations through L2 and FP64 refinement, which graded spectra (1e-12) take 50 sweeps in (ms):
+//   864 x 864   graded 163, 444   power law 180, 186   Gaussian 167, 124   degenerate pairs 155, 526
+//   1176 x 1176 graded 294, 688   power law 326, 296;   1400 x 520 graded 78, 577;   3000 x 540 graded 104, 1111
+// Projector spectra are graded, and the refinement's bits are no better, so one form for all of them.  Narrower blocks
+// too tall for a cluster stay on the sweeps (3000 x 400 graded 511, without either 1459).
+constexpr double kQrRecompute = 1.4901161193847656e-08;  // sqrt(eps): norm downdates below this are recomputed
+
+// sum over the 512 threads of a CTA, the same bits in every thread; red: kWarps doubles of shared memory
+__device__ double block_sum(double v, double* red, const Ctx& c) {
+  v = wsum(v);
+  __syncthreads();  // red is free (an earlier call's readers are done)
+  if (c.lane == 0) red[c.warp] = v;
+  __syncthreads();
+  double t = 0;
+  for (int w = 0; w < kWarps; ++w) t += red[w];
+  return t;
+}
+
+// Householder QR with column pivoting of H (mm x nn column-major, mm >= nn) in place: R on and above
+// the diagonal, the reflectors v_k = (1, H[k+1:, k]) below it, H_k = I - tau_k v_k v_k^T; piv[k] = the
+// column of the input at position k.  vn1 / vn2: partial column norms and their last exact values.
+template <class Group>
+__device__ void qr_pivoted(Group& gg, const Ctx& c, double* H, int64_t mm, int nn, double* tau, int* piv,
+                           double* vn1, double* vn2, double* red, int* redi) {
+  const unsigned full = 0xffffffffu;
+  for (int j = c.gw; j < nn; j += c.gnw) {
+    const double* h = H + int64_t(j) * mm;
+    double a = 0;
+    for (int64_t i = c.lane; i < mm; i += 32) {
+      const double x = ldg(h + i);
+      a = fma(x, x, a);
+    }
+    a = sqrt(wsum(a));
+    if (c.lane == 0) {
+      stg(vn1 + j, a);
+      stg(vn2 + j, a);
+      __stcg(piv + j, j);
+    }
+  }
+  gg.sync();
+  for (int k = 0; k < nn; ++k) {
+    if (c.rank == 0) {
+      // pivot: the largest remaining norm (the first such column on ties)
+      double best = -1.0;
+      int bi = k;
+      for (int j = k + c.tid; j < nn; j += kThreads) {
+        const double v = ldg(vn1 + j);
+        if (v > best) {
+          best = v;
+          bi = j;
+        }
+      }
+      for (int o = 16; o > 0; o >>= 1) {
+        const double ob = __shfl_xor_sync(full, best, o);
+        const int oi = __shfl_xor_sync(full, bi, o);
+        if (ob > best || (ob == best && oi < bi)) {
+          best = ob;
+          bi = oi;
+        }
+      }
+      __syncthreads();
+      if (c.lane == 0) {
+        red[c.warp] = best;
+        redi[c.warp] = bi;
+      }
+      __syncthreads();
+      best = red[0];
+      bi = redi[0];
+      for (int w = 1; w < kWarps; ++w)
+        if (red[w] > best || (red[w] == best && redi[w] < bi)) {
+          best = red[w];
+          bi = redi[w];
+        }
+      const int p = bi;
+      double* hk = H + int64_t(k) * mm;
+      double* hp = H + int64_t(p) * mm;
+      // swap columns k and p (every row: rows above k hold R's earlier entries), with the sum of squares of
+      // the new column k below row k
+      double ss = 0;
+      for (int64_t i = c.tid; i < mm; i += kThreads) {
+        const double x = ldg(hp + i);
+        if (p != k) {
+          stg(hp + i, ldg(hk + i));
+          stg(hk + i, x);
+        }
+        if (i > k) ss = fma(x, x, ss);
+      }
+      ss = block_sum(ss, red, c);  // its barriers also order the swap before the reads below
+      if (c.tid == 0 && p != k) {
+        const double a1 = ldg(vn1 + k), a2 = ldg(vn2 + k);
+        stg(vn1 + k, ldg(vn1 + p));
+        stg(vn2 + k, ldg(vn2 + p));
+        stg(vn1 + p, a1);
+        stg(vn2 + p, a2);
+        const int q = __ldcg(piv + k);
+        __stcg(piv + k, __ldcg(piv + p));
+        __stcg(piv + p, q);
+      }
+      // reflector: beta = -sign(alpha) |(alpha, x)|, tau = (beta - alpha) / beta, v = x / (alpha - beta)
+      const double alpha = ldg(hk + k);
+      double beta = alpha, t = 0.0, scal = 0.0;
+      if (ss > 0.0) {
+        beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
+        t = (beta - alpha) / beta;
+        scal = 1.0 / (alpha - beta);
+        for (int64_t i = k + 1 + c.tid; i < mm; i += kThreads) stg(hk + i, ldg(hk + i) * scal);
+      }
+      if (c.tid == 0) {
+        stg(hk + k, beta);
+        stg(tau + k, t);
+      }
+    }
+    gg.sync();
+    // apply H_k to the trailing columns (one warp each) and downdate their norms
+    const double tk = ldg(tau + k);
+    const double* v = H + int64_t(k) * mm;
+    for (int j = k + 1 + c.gw; j < nn; j += c.gnw) {
+      double* h = H + int64_t(j) * mm;
+      const double hkj = ldg(h + k);
+      double w = 0.0;
+      if (tk != 0.0) {
+        double a0 = 0, a1 = 0, a2 = 0, a3 = 0;
+        int64_t i = k + 1 + c.lane;
+        for (; i + 96 < mm; i += 128) {
+          a0 = fma(ldg(v + i), ldg(h + i), a0);
+          a1 = fma(ldg(v + i + 32), ldg(h + i + 32), a1);
+          a2 = fma(ldg(v + i + 64), ldg(h + i + 64), a2);
+          a3 = fma(ldg(v + i + 96), ldg(h + i + 96), a3);
+        }
+        for (; i < mm; i += 32) a0 = fma(ldg(v + i), ldg(h + i), a0);
+        w = tk * (hkj + wsum((a0 + a1) + (a2 + a3)));
+        for (int64_t i2 = k + 1 + c.lane; i2 < mm; i2 += 32) stg(h + i2, fma(-w, ldg(v + i2), ldg(h + i2)));
+      }
+      const double rkj = hkj - w;  // R(k, j)
+      if (c.lane == 0) stg(h + k, rkj);
+      const double n1 = ldg(vn1 + j);
+      if (n1 != 0.0) {  // warp-uniform
+        double r = fabs(rkj) / n1;
+        r = fmax(0.0, (1.0 + r) * (1.0 - r));
+        const double q = n1 / ldg(vn2 + j);
+        double n1new;
+        if (r * q * q <= kQrRecompute) {
+          // each lane re-reads the rows it wrote above
+          double a = 0;
+          for (int64_t i2 = k + 1 + c.lane; i2 < mm; i2 += 32) {
+            const double x = ldg(h + i2);
+            a = fma(x, x, a);
+          }
+          n1new = sqrt(wsum(a));
+          if (c.lane == 0) stg(vn2 + j, n1new);
+        } else {
+          n1new = n1 * sqrt(r);
+        }
+        if (c.lane == 0) stg(vn1 + j, n1new);
+      }
+    }
+    gg.sync();
+  }
+}
+
+__global__ void __launch_bounds__(kThreads)
+    svd_factor_kernel(const xgb_svd_desc* __restrict__ descs, const int64_t* __restrict__ work_off, int sector,
+                    const double* __restrict__ A, double* __restrict__ U, double* __restrict__ S,
+                    double* __restrict__ Vt, double* __restrict__ work, int* __restrict__ sweep_stats,
+                    int smem_bytes) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  __shared__ double red[kWarps];
+  __shared__ int redi[kWarps];
+  cg::grid_group gg = cg::this_grid();
+  const xgb_svd_desc d = descs[sector];
+  const bool tr = d.m < d.n;
+  const int64_t mm = tr ? d.n : d.m;
+  const int nn = int(tr ? d.m : d.n);
+  if (nn == 0) return;  // uniform across the grid
+
+  const Ctx c = make_ctx(int(blockIdx.x), int(gridDim.x));
+  // workspace (doubles): H mm*nn | V nn*nn | T1 nn*nn | X nn*nn | n64 nn | misc 8 | Y mm*nn (svd_work_elems
+  // adds Y for blocks this wide); T1: the Jacobi column order (nn ints), then tau, vn1, vn2 (nn each), piv
+  const int64_t nn2 = int64_t(nn) * nn;
+  double* H = work + work_off[sector];
+  double* V64 = H + mm * nn;
+  double* T1 = V64 + nn2;
+  double* X = T1 + nn2;
+  double* n64 = X + nn2;
+  int* flag = reinterpret_cast<int*>(n64 + nn);
+  double* Y = n64 + nn + 8;
+  int* jorder = reinterpret_cast<int*>(T1);
+  double* tau = T1 + nn;
+  double* vn1 = tau + nn;
+  double* vn2 = vn1 + nn;
+  int* piv = reinterpret_cast<int*>(vn2 + nn);
+  auto opA = [&](int64_t i, int64_t j) { return tr ? A[d.a_off + j + i * d.m] : A[d.a_off + i + j * d.m]; };
+  const long long t0 = clock64();
+  for (int j = c.gw; j < nn; j += c.gnw)
+    for (int64_t i = c.lane; i < mm; i += 32) stg(H + int64_t(j) * mm + i, opA(i, j));
+  gg.sync();
+  qr_pivoted(gg, c, H, mm, nn, tau, piv, vn1, vn2, red, redi);
+  // X = R^T (lower triangle), V = I
+  for (int j = c.gw; j < nn; j += c.gnw)
+    for (int i = c.lane; i < nn; i += 32) {
+      stg(X + int64_t(j) * nn + i, i >= j ? ldg(H + int64_t(i) * mm + j) : 0.0);
+      stg(V64 + int64_t(j) * nn + i, i == j ? 1.0 : 0.0);
+    }
+  gg.sync();
+  const long long t1 = clock64();
+  const int nblocks = 2 * int(gridDim.x);
+  const int b = (nn + nblocks - 1) / nblocks;
+  const bool staged = int64_t(2 * b) * (nn + nn + 1) * 8 <= smem_bytes;
+  const int sw = nn > 1 ? block_jacobi<double>(gg, c, X, V64, n64, flag, nn, nn, 1.0e-13, kFloor64, kFactorSweeps,
+                                               reinterpret_cast<double*>(smem_raw), staged, nblocks, jorder)
+                        : 0;
+  const long long t2 = clock64();
+  // sigma_j = |x_j|
+  for (int j = c.gw; j < nn; j += c.gnw) {
+    const double* x = X + int64_t(j) * nn;
+    double a = 0;
+    for (int i = c.lane; i < nn; i += 32) {
+      const double e = ldg(x + i);
+      a = fma(e, e, a);
+    }
+    a = wsum(a);
+    if (c.lane == 0) stg(n64 + j, sqrt(a));
+  }
+  gg.sync();
+  // per Jacobi column j (one warp, no barriers): rank r among the sigmas (descending, ties by column),
+  // Y_j = Q [V_j; 0] (reflectors H_{nn-1} first; lane ln owns rows ln + 32 t throughout), then U, S, V^T of
+  // the block with the sign rule
+  const int64_t kk = nn;
+  for (int j = c.gw; j < nn; j += c.gnw) {
+    const double sj = ldg(n64 + j);
+    int r = 0;
+    for (int i = c.lane; i < nn; i += 32) {
+      const double si = ldg(n64 + i);
+      r += ranks_above(si, sj, i < j);
+    }
+    r = wsum(r);
+    const double inv = sj > 0 ? 1.0 / sj : 0.0;
+    double* y = Y + int64_t(j) * mm;
+    for (int64_t i = c.lane; i < mm; i += 32) stg(y + i, i < nn ? ldg(V64 + int64_t(j) * nn + i) : 0.0);
+    for (int k = nn - 1; k >= 0; --k) {
+      const double tk = ldg(tau + k);
+      if (tk == 0.0) continue;  // uniform
+      const double* v = H + int64_t(k) * mm;
+      double a0 = 0, a1 = 0, yk = 0;
+      int64_t i = c.lane;
+      for (; i + 32 < mm; i += 64) {
+        const double y0 = ldg(y + i), y1 = ldg(y + i + 32);
+        if (i > k) a0 = fma(ldg(v + i), y0, a0);
+        else if (i == k) yk = y0;
+        if (i + 32 > k) a1 = fma(ldg(v + i + 32), y1, a1);
+        else if (i + 32 == k) yk = y1;
+      }
+      for (; i < mm; i += 32) {
+        const double y0 = ldg(y + i);
+        if (i > k) a0 = fma(ldg(v + i), y0, a0);
+        else if (i == k) yk = y0;
+      }
+      yk = __shfl_sync(0xffffffffu, yk, k & 31);
+      const double w = tk * (yk + wsum(a0 + a1));
+      for (int64_t i2 = c.lane; i2 < mm; i2 += 32) {
+        if (i2 == k) stg(y + i2, yk - w);
+        else if (i2 > k) stg(y + i2, fma(-w, ldg(v + i2), ldg(y + i2)));
+      }
+    }
+    // op(A) = Y Sigma (P U_X)^T with U_X = X / sigma: column j of P U_X has X[i, j] / sigma_j at row piv[i]
+    double* ucol = U + d.u_off + int64_t(r) * d.m;
+    double sg;
+    if (!tr) {
+      sg = sign_of<true>(y, mm, 1.0, c.lane);
+      for (int64_t i = c.lane; i < mm; i += 32) ucol[i] = sg * ldg(y + i);
+      for (int i = c.lane; i < nn; i += 32)
+        Vt[d.vt_off + r + int64_t(__ldcg(piv + i)) * kk] = sg * inv * ldg(X + int64_t(j) * nn + i);
+    } else {
+      // U = P U_X (nn rows): scattered, then read back for the sign
+      for (int i = c.lane; i < nn; i += 32) stg(ucol + __ldcg(piv + i), inv * ldg(X + int64_t(j) * nn + i));
+      __syncwarp();
+      sg = sign_of<true>(ucol, nn, 1.0, c.lane);
+      if (sg < 0)
+        for (int i = c.lane; i < nn; i += 32) stg(ucol + i, -ldg(ucol + i));
+      for (int64_t cc = c.lane; cc < mm; cc += 32) Vt[d.vt_off + r + cc * kk] = sg * ldg(y + cc);
+    }
+    if (c.lane == 0) S[d.s_off + r] = sj;
+  }
+  if (sweep_stats && c.rank == 0 && c.tid == 0) {
+    int* st6 = sweep_stats + 6 * sector;
+    st6[0] = 0;
+    st6[1] = sw;
+    st6[2] = int((t1 - t0) >> 10);  // QR cycles / 1024 on CTA 0's SM
+    st6[3] = 0;
+    st6[4] = int((t2 - t1) >> 10);
+    st6[5] = int((clock64() - t2) >> 10);
   }
 }
 
@@ -1783,13 +2102,13 @@ void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int grid
   cfg.numAttrs = 1;
 }
 
-void launch_clusters(int pass, int lo, int ctas, int widest, int n, const xgb_svd_desc* descs, const int64_t* off,
+void launch_clusters(int pass, int lo, int ctas, int widest, int grid_most, int n, const xgb_svd_desc* descs, const int64_t* off,
                      const double* A, double* U, double* S, double* Vt, double* work, int* stats, cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   cluster_config(cfg, attr, n * ctas, ctas, s);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, svd_sweeps_kernel, descs, off, A, U, S, Vt, work, stats, pass, lo,
-                                           g_most_ctas, widest, int(kSmemLimit));
+                                           g_most_ctas, widest, grid_most, int(kSmemLimit));
   if (e != cudaSuccess) throw std::runtime_error(std::string("svd sweeps launch: ") + cudaGetErrorString(e));
   count_launch();
 }
@@ -1801,7 +2120,7 @@ void launch_grid(const void* kernel, int ctas, void** args, cudaStream_t s) {
   count_launch();
 }
 
-// All stages of a batch, in stream order; allocates nothing.  grid: blocks wider than kGridN may use
+// All stages of a batch, in stream order; allocates nothing.  grid: wide blocks may use
 // cooperative launches (a side lane shares the SMs with the other lane's kernels, and a cooperative grid's
 // CTAs wait on one another, so there every block stays on clusters, which take any width).
 void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, const int64_t* d_off, int n,
@@ -1812,6 +2131,7 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
     for (const void* f : {reinterpret_cast<const void*>(svd_sweeps_kernel),
                           reinterpret_cast<const void*>(svd_sweeps_grid_kernel),
                           reinterpret_cast<const void*>(svd_polish_grid_kernel),
+                          reinterpret_cast<const void*>(svd_factor_kernel),
                           reinterpret_cast<const void*>(svd_finish_kernel),
                           reinterpret_cast<const void*>(svd_small_kernel)})
       cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemLimit);
@@ -1827,8 +2147,9 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
   int64_t small_bytes = 0;
   int narrow[2] = {0, 0}, broad[2] = {0, 0};  // CTAs of the two sweep launches of each pass
   int64_t av = 0, gram = 0, apply = 0, upd = 0;
-  std::vector<int> wide[2];  // blocks whose sweeps of a pass take the cooperative grid
-  const int widest[2] = {grid ? kGridN : INT32_MAX, grid ? kGridN2 : INT32_MAX};
+  std::vector<int> factor, wide;  // blocks of svd_factor_kernel; those whose pass 1 and polish take the cooperative grid
+  const int widest[2] = {INT32_MAX, grid ? kGridN : INT32_MAX};
+  const int grid_most = grid ? g_most_ctas : 0;
   for (int i = 0; i < n; ++i) {
     const int64_t mm = std::max(h_descs[i].m, h_descs[i].n), nn = std::min(h_descs[i].m, h_descs[i].n);
     if (nn == 0) continue;
@@ -1836,9 +2157,13 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
       small_bytes = std::max<int64_t>(small_bytes, 8 * (2 * (mm | 1) * nn + 4 * (nn | 1) * nn));
       continue;
     }
+    if (factored(mm, nn, grid_most)) {
+      factor.push_back(i);
+      continue;
+    }
     for (int pass = 0; pass < 2; ++pass) {
       const int ctas = sweep_ctas(pass, mm, nn, g_most_ctas);
-      if (nn > widest[pass]) wide[pass].push_back(i);
+      if (nn > widest[pass]) wide.push_back(i);
       else if (ctas <= kNarrow) narrow[pass] = std::max(narrow[pass], ctas);
       else broad[pass] = std::max(broad[pass], ctas);
     }
@@ -1852,52 +2177,60 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
     svd_small_kernel<<<n, kThreads, size_t(small_bytes), s>>>(d_descs, A, U, S, Vt, stats);
     count_launch();
   }
-  if (!av) return;
   int smem = kSmemLimit;
+  for (int sector : factor) {
+    const int64_t nn = std::min(h_descs[sector].m, h_descs[sector].n);
+    const int ctas = int(std::min<int64_t>(num_sms(), (nn + 2 * kFactorCols - 1) / (2 * kFactorCols)));
+    void* args[] = {&d_descs, &d_off, &sector, const_cast<double**>(&A), &U, &S, &Vt, &work, &stats, &smem};
+    launch_grid(reinterpret_cast<const void*>(svd_factor_kernel), ctas, args, s);
+  }
+  if (!av) return;
   auto sweeps = [&](int pass) {
-    for (int sector : wide[pass]) {
-      const int64_t nn = std::min(h_descs[sector].m, h_descs[sector].n);
-      const int ctas = int(std::min<int64_t>(num_sms(), (nn + 2 * kWarps - 1) / (2 * kWarps)));
-      void* args[] = {&d_descs, &d_off, &sector, const_cast<double**>(&A), &U, &Vt, &work, &stats, &pass, &smem};
-      launch_grid(reinterpret_cast<const void*>(svd_sweeps_grid_kernel), ctas, args, s);
-    }
+    if (pass)
+      for (int sector : wide) {
+        const int64_t nn = std::min(h_descs[sector].m, h_descs[sector].n);
+        const int ctas = int(std::min<int64_t>(num_sms(), (nn + 2 * kWarps - 1) / (2 * kWarps)));
+        void* args[] = {&d_descs, &d_off, &sector, const_cast<double**>(&A), &U, &Vt, &work, &stats, &smem};
+        launch_grid(reinterpret_cast<const void*>(svd_sweeps_grid_kernel), ctas, args, s);
+      }
     if (broad[pass])
-      launch_clusters(pass, kNarrow, broad[pass], widest[pass], n, d_descs, d_off, A, U, S, Vt, work, stats, s);
+      launch_clusters(pass, kNarrow, broad[pass], widest[pass], grid_most, n, d_descs, d_off, A, U, S, Vt, work, stats, s);
     if (narrow[pass])
-      launch_clusters(pass, 0, narrow[pass], widest[pass], n, d_descs, d_off, A, U, S, Vt, work, stats, s);
+      launch_clusters(pass, 0, narrow[pass], widest[pass], grid_most, n, d_descs, d_off, A, U, S, Vt, work, stats, s);
   };
   sweeps(0);
   const unsigned ny = unsigned(n);
-  svd_product_kernel<kProdAV><<<dim3(unsigned(av), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, 0);
+  svd_product_kernel<kProdAV><<<dim3(unsigned(av), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, 0, grid_most);
   count_launch();
   for (int it = 0; it < kIters; ++it) {
-    svd_product_kernel<kProdGram><<<dim3(unsigned(gram), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, it);
-    svd_update_kernel<<<dim3(unsigned(upd), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, it);
+    svd_product_kernel<kProdGram><<<dim3(unsigned(gram), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, it, grid_most);
+    svd_update_kernel<<<dim3(unsigned(upd), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, it, grid_most);
     count_launch(2);
     if (it == kPass2) sweeps(1);
-    svd_product_kernel<kProdApply><<<dim3(unsigned(apply), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, it);
+    svd_product_kernel<kProdApply><<<dim3(unsigned(apply), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, it, grid_most);
     count_launch();
   }
-  for (int sector : wide[1]) {
+  for (int sector : wide) {
     const int64_t nn = std::min(h_descs[sector].m, h_descs[sector].n);
     const int ctas = int(std::min<int64_t>(num_sms(), (nn + 7) / 8));
     void* args[] = {&d_descs, &d_off, &sector, const_cast<double**>(&A), &U, &Vt, &work, &stats, &smem};
     launch_grid(reinterpret_cast<const void*>(svd_polish_grid_kernel), ctas, args, s);
   }
   svd_finish_kernel<<<n * kCluster, kThreads, kSmemLimit, s>>>(d_descs, d_off, A, U, S, Vt, work, stats, smem,
-                                                               wide[1].empty() ? INT32_MAX : kGridN2 + 1);
+                                                               wide.empty() ? INT32_MAX : kGridN + 1,
+                                                               grid_most);
   count_launch();
 }
 
 }  // namespace
 
 size_t svd_work_elems(int64_t m, int64_t n) {
-  // W, V, G, E, norms and the state words (Block above) take the first mm nn + 3 nn^2 + nn + 10; the size that
-  // callers were told, and the no-alloc entry's capacity that follows from it, stay as they were published
+  // W, V, G, E, norms and the state words (Block above) take the first mm nn + 3 nn^2 + nn + 10
   const int64_t mm = std::max(m, n), nn = std::min(m, n);
   const int64_t doubles = mm * nn + 3 * nn * nn + nn + 8;
   const int64_t floats = mm * nn + nn * nn + nn;
-  return size_t(doubles + std::max((floats + 1) / 2 + 2, nn >= 512 ? mm * nn : 0));
+  // svd_factor_kernel keeps Q's columns (mm x nn) behind them
+  return size_t(doubles + std::max((floats + 1) / 2 + 2, nn >= kFactorN ? mm * nn : 0));
 }
 
 void launch_svd(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, const int64_t* d_work_off, int n,
