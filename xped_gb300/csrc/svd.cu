@@ -1032,15 +1032,18 @@ __device__ void finish_svd(Group& cl, const Ctx& c, const xgb_svd_desc& d, bool 
 }
 
 // ---------------------------------------------------------------- state of one block
-// Workspace of a block wider than kSmallN (doubles): W0 mm*nn | V0 nn*nn | G nn*nn | E nn*nn | n64 nn | misc.
-// The second W / V pair of the refinement is the block's own U / V^T output, and the FP32 columns live in
-// whichever pair does not hold the current W and V.
+// Workspace of a block wider than kSmallN (doubles): W0 mm*nn | V0 nn*nn | G nn*nn | E nn*nn | n64 nn | misc 10 | the
+// FP32 columns W32 (mm*nn floats) of a pass 0 that no cluster holds, from a 32-byte sector on (columns across sectors:
+// 3000 x 400 graded 761 ms instead of 511); their rotations V32 lie in E.
+// The second W / V pair of the refinement is the block's own U / V^T output, written only once A has been read for
+// the last time (W = op(A) V): an output may overlap its block of A.
 struct Block {
   int64_t mm, lda;
   int nn;
   bool tr;
   const double* A;
   double *W0, *V0, *G, *E, *n64, *W1, *V1;
+  float* W32;
   int* misc;  // 0: Jacobi flag, 2-3: largest |entry| (bits), per iteration kUnconv and kZmax (float bits), kBig
 };
 constexpr int kPass2 = 1;  // the iteration after whose test unresolved blocks go through FP32 sweeps again
@@ -1063,6 +1066,9 @@ __device__ __forceinline__ Block block_of(const xgb_svd_desc& d, int64_t off, co
   k.E = k.G + nn2;
   k.n64 = k.E + nn2;
   k.misc = reinterpret_cast<int*>(k.n64 + k.nn);
+  // (one column takes no sweeps, and its workspace has no room to spare)
+  const uintptr_t unit = k.nn > 1 ? 32 : 8;
+  k.W32 = reinterpret_cast<float*>((reinterpret_cast<uintptr_t>(k.misc + kState) + unit - 1) / unit * unit);
   k.W1 = k.tr ? Vt + d.vt_off : U + d.u_off;
   k.V1 = k.tr ? U + d.u_off : Vt + d.vt_off;
   return k;
@@ -1135,8 +1141,8 @@ __device__ void fp32_pass(Group& g, const Ctx& c, int P, const Block& k, int pas
   // pass 1 comes after one update: W and V lie in W1 and V1, W0 and V0 are free
   static_assert(kPass2 == 1, "W and V after one update");
   const double* src = k.W1;
-  float* W32 = reinterpret_cast<float*>(pass ? k.W0 : k.W1);
-  float* V32 = reinterpret_cast<float*>(pass ? k.V0 : k.V1);
+  float* W32 = pass ? reinterpret_cast<float*>(k.W0) : k.W32;
+  float* V32 = reinterpret_cast<float*>(pass ? k.V0 : k.E);
   int* perm = reinterpret_cast<int*>(k.G);
   float* n32 = reinterpret_cast<float*>(k.G) + nn;
   if (pass == 0) {
@@ -2225,7 +2231,8 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
 }  // namespace
 
 size_t svd_work_elems(int64_t m, int64_t n) {
-  // W, V, G, E, norms and the state words (Block above) take the first mm nn + 3 nn^2 + nn + 10
+  // Block above: W, V, G, E, norms and the state words take mm nn + 3 nn^2 + nn + 10, the FP32 columns up to
+  // mm nn / 2 + 3 (alignment) behind them
   const int64_t mm = std::max(m, n), nn = std::min(m, n);
   const int64_t doubles = mm * nn + 3 * nn * nn + nn + 8;
   const int64_t floats = mm * nn + nn * nn + nn;
