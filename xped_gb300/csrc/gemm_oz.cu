@@ -617,7 +617,7 @@ __global__ void __launch_bounds__(256) oz_splitk_reduce_kernel(const xgb_gemm_de
   *c = beta != 0.0 ? fma(alpha, acc, beta * *c) : alpha == 1.0 ? acc : alpha * acc;
 }
 
-std::once_flag g_oz_attr;
+PerDevice g_oz_attr;
 
 }  // namespace
 
@@ -722,7 +722,7 @@ void launch_oz_gemm(const xgb_gemm_desc* d_descs, const OzGroup* d_groups, const
                     const unsigned char* bpack, const unsigned long long* rowmax, double* C, double alpha, double beta,
                     cudaStream_t s) {
   if (n_tiles <= 0) return;
-  std::call_once(g_oz_attr, [] {
+  g_oz_attr.once([] {
     cudaFuncSetAttribute(oz_gemm_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kOzSmem);
   });
   double* ws = slots > 0 ? static_cast<double*>(dev_alloc(sizeof(double) * size_t(slots) * OM * ON)) : nullptr;

@@ -421,7 +421,8 @@ __global__ void __launch_bounds__(kTcThreads, 1)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemAlloc));
 }
 
-std::once_flag g_tc_attr, g_tc_err_once;
+PerDevice g_tc_attr;
+std::once_flag g_tc_err_once;
 int* g_tc_err = nullptr;
 
 }  // namespace
@@ -456,7 +457,7 @@ void launch_gemm_tc(const xgb_gemm_desc* d_descs, const TcGroup* d_groups, const
                     const GemmTile* d_tiles, int n_tiles, const double* A, const double* B, float* apack,
                     float* bpack, double* C, double alpha, double beta, cudaStream_t s, int form) {
   if (n_tiles <= 0) return;
-  std::call_once(g_tc_attr, [] {
+  g_tc_attr.once([] {
     cudaFuncSetAttribute(gemm_tc_kernel<0>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
     cudaFuncSetAttribute(gemm_tc_kernel<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemBytes);
   });

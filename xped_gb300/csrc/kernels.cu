@@ -729,8 +729,8 @@ __global__ void __launch_bounds__(kTruncThreads) truncate_kernel(int n_sectors, 
 void launch_truncate(int n_sectors, const int64_t* d_s_begin, const int32_t* d_deg, const double* s, int64_t total,
                      int64_t max_keep, double eps, int preserve, int32_t* keep, double* out2, cudaStream_t st) {
   if (total > INT32_MAX / 4) throw std::runtime_error("truncate: too many singular values");
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice attr;
+  attr.once([] {
     cudaFuncSetAttribute(truncate_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kTruncSmem) * 24);
   });
   const bool in_smem = total <= kTruncSmem;

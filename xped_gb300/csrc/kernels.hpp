@@ -12,6 +12,7 @@
 #include <vector>
 
 #include "../../include/xgb.h"
+#include "per_device.hpp"
 
 namespace xgb {
 

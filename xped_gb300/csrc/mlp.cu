@@ -202,10 +202,10 @@ __global__ void mlp_reduce_adam_kernel(float* __restrict__ p, float* __restrict_
   p[i] -= lr * (m1 / c1) / (sqrtf(v1 / c2) + eps);
 }
 
-std::once_flag g_attr_set;
+PerDevice g_attr_set;
 
 void set_attrs() {
-  std::call_once(g_attr_set, [] {
+  g_attr_set.once([] {
     const int bytes = kSmemFloats * int(sizeof(float));
     cudaFuncSetAttribute(mlp_forward_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     cudaFuncSetAttribute(mlp_grad_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);

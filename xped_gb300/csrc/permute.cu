@@ -305,9 +305,12 @@ void launch_form(const PlaneTask* d_tasks, const int64_t* d_start, int n_tasks, 
   const unsigned blocks = unsigned(std::min<int64_t>((n_planes + batch - 1) / batch, int64_t(1) << 20));
   constexpr int bytes = kTranspose ? kWarps * kTileElems * int(sizeof(double)) : 0;
   if constexpr (kTranspose) {
-    static const cudaError_t set = cudaFuncSetAttribute(permute_planes_kernel<G, kTranspose, kSingle, SI>,
-                                                        cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
-    if (set != cudaSuccess) throw std::runtime_error("permute: shared memory not granted");
+    static PerDevice attr;
+    attr.once([] {
+      if (cudaFuncSetAttribute(permute_planes_kernel<G, kTranspose, kSingle, SI>,
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) != cudaSuccess)
+        throw std::runtime_error("permute: shared memory not granted");
+    });
   }
   permute_planes_kernel<G, kTranspose, kSingle, SI>
       <<<blocks, kThreads, bytes, s>>>(d_tasks, d_start, n_tasks, n_planes, batch, d_sources, src, dst);

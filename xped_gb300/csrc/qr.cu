@@ -278,8 +278,8 @@ size_t qr_work_elems(int64_t m, int64_t n) { return size_t(m * n + std::min(m, n
 void launch_qr(const xgb_qr_desc* d_descs, const xgb_qr_desc* h_descs, const int64_t* d_work_off, int n,
                const double* A, double* Q, double* R, double* work, cudaStream_t s) {
   if (n <= 0) return;
-  static std::once_flag attr;
-  std::call_once(attr, [] {
+  static PerDevice attr;
+  attr.once([] {
     cudaFuncSetAttribute(qr_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemLimit));
     cudaFuncSetAttribute(qr_form_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemLimit));
   });

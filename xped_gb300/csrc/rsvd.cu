@@ -797,7 +797,7 @@ __global__ void __launch_bounds__(32 * kTrinvCols) trinv_kernel(const CholDesc* 
 void launch_chol_inv(const CholDesc* d_descs, int n, int64_t max_l, double* G, double* Rinv, double rel_shift,
                      int* bad, cudaStream_t s) {
   if (n <= 0 || max_l <= 0) return;
-  static std::once_flag attr;
+  static PerDevice attr;
   // Cholesky alone: one l x (l | 1) matrix in shared memory up to l = 167 (< 227 KB)
   constexpr int kCapChol = 167;
   // Cholesky and inverse in one CTA (blocks wider than the register-resident inverse allows):
@@ -805,7 +805,7 @@ void launch_chol_inv(const CholDesc* d_descs, int n, int64_t max_l, double* G, d
   constexpr int kCapBoth = 119;
   constexpr int kBytesChol = kCapChol * (kCapChol | 1) * int(sizeof(double));
   constexpr int kBytesBoth = 2 * kCapBoth * (kCapBoth | 1) * int(sizeof(double));
-  std::call_once(attr, [] {
+  attr.once([] {
     cudaFuncSetAttribute(chol_inv_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytesChol);
     cudaFuncSetAttribute(chol_inv_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, kBytesBoth);
   });
@@ -826,8 +826,8 @@ void launch_chol_inv(const CholDesc* d_descs, int n, int64_t max_l, double* G, d
   if (max_l <= kCholCluster) {
     const int cluster = max_l <= 4 * kPan ? 4 : 8;
     const int bytes = chol_cluster_elems(int(max_l), cluster) * int(sizeof(double));
-    static std::once_flag cattr;
-    std::call_once(cattr, [] {
+    static PerDevice cattr;
+    cattr.once([] {
       cudaFuncSetAttribute(chol_cluster_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                            chol_cluster_elems(kCholCluster, 8) * int(sizeof(double)));
     });

@@ -2094,7 +2094,7 @@ int* g_stats_dev = nullptr;
 int g_stats_cap = 0;
 int g_stats_n = 0;
 
-int g_most_ctas = 8;  // most CTAs per cluster (set once)
+int g_most_ctas[PerDevice::kMost];  // most CTAs per cluster, by device (set with its kernels' attributes)
 
 void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int grid, int ctas, cudaStream_t s) {
   cfg.gridDim = dim3(unsigned(grid));
@@ -2108,13 +2108,14 @@ void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int grid
   cfg.numAttrs = 1;
 }
 
-void launch_clusters(int pass, int lo, int ctas, int widest, int grid_most, int n, const xgb_svd_desc* descs, const int64_t* off,
-                     const double* A, double* U, double* S, double* Vt, double* work, int* stats, cudaStream_t s) {
+void launch_clusters(int pass, int lo, int ctas, int most, int widest, int grid_most, int n, const xgb_svd_desc* descs,
+                     const int64_t* off, const double* A, double* U, double* S, double* Vt, double* work, int* stats,
+                     cudaStream_t s) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   cluster_config(cfg, attr, n * ctas, ctas, s);
   const cudaError_t e = cudaLaunchKernelEx(&cfg, svd_sweeps_kernel, descs, off, A, U, S, Vt, work, stats, pass, lo,
-                                           g_most_ctas, widest, grid_most, int(kSmemLimit));
+                                           most, widest, grid_most, int(kSmemLimit));
   if (e != cudaSuccess) throw std::runtime_error(std::string("svd sweeps launch: ") + cudaGetErrorString(e));
   count_launch();
 }
@@ -2132,8 +2133,8 @@ void launch_grid(const void* kernel, int ctas, void** args, cudaStream_t s) {
 void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, const int64_t* d_off, int n,
                   const double* A, double* U, double* S, double* Vt, double* work, int* stats, bool grid,
                   cudaStream_t s) {
-  static std::once_flag configured;
-  std::call_once(configured, [] {
+  static PerDevice configured;
+  configured.once([] {
     for (const void* f : {reinterpret_cast<const void*>(svd_sweeps_kernel),
                           reinterpret_cast<const void*>(svd_sweeps_grid_kernel),
                           reinterpret_cast<const void*>(svd_polish_grid_kernel),
@@ -2148,14 +2149,15 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
     cluster_config(cfg, attr, kMostCtas, kMostCtas, nullptr);
     int fit = 0;
     if (cudaOccupancyMaxActiveClusters(&fit, svd_sweeps_kernel, &cfg) != cudaSuccess) (void)cudaGetLastError();
-    g_most_ctas = fit > 0 ? kMostCtas : 8;
+    g_most_ctas[PerDevice::current()] = fit > 0 ? kMostCtas : 8;
   });
+  const int most = g_most_ctas[PerDevice::current()];
   int64_t small_bytes = 0;
   int narrow[2] = {0, 0}, broad[2] = {0, 0};  // CTAs of the two sweep launches of each pass
   int64_t av = 0, gram = 0, apply = 0, upd = 0;
   std::vector<int> factor, wide;  // blocks of svd_factor_kernel; those whose pass 1 and polish take the cooperative grid
   const int widest[2] = {INT32_MAX, grid ? kGridN : INT32_MAX};
-  const int grid_most = grid ? g_most_ctas : 0;
+  const int grid_most = grid ? most : 0;
   for (int i = 0; i < n; ++i) {
     const int64_t mm = std::max(h_descs[i].m, h_descs[i].n), nn = std::min(h_descs[i].m, h_descs[i].n);
     if (nn == 0) continue;
@@ -2168,7 +2170,7 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
       continue;
     }
     for (int pass = 0; pass < 2; ++pass) {
-      const int ctas = sweep_ctas(pass, mm, nn, g_most_ctas);
+      const int ctas = sweep_ctas(pass, mm, nn, most);
       if (nn > widest[pass]) wide.push_back(i);
       else if (ctas <= kNarrow) narrow[pass] = std::max(narrow[pass], ctas);
       else broad[pass] = std::max(broad[pass], ctas);
@@ -2200,9 +2202,11 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
         launch_grid(reinterpret_cast<const void*>(svd_sweeps_grid_kernel), ctas, args, s);
       }
     if (broad[pass])
-      launch_clusters(pass, kNarrow, broad[pass], widest[pass], grid_most, n, d_descs, d_off, A, U, S, Vt, work, stats, s);
+      launch_clusters(pass, kNarrow, broad[pass], most, widest[pass], grid_most, n, d_descs, d_off, A, U, S, Vt, work,
+                      stats, s);
     if (narrow[pass])
-      launch_clusters(pass, 0, narrow[pass], widest[pass], grid_most, n, d_descs, d_off, A, U, S, Vt, work, stats, s);
+      launch_clusters(pass, 0, narrow[pass], most, widest[pass], grid_most, n, d_descs, d_off, A, U, S, Vt, work,
+                      stats, s);
   };
   sweeps(0);
   const unsigned ny = unsigned(n);
