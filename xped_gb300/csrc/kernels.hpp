@@ -70,6 +70,12 @@ struct AllocScope {
   AllocScope& operator=(const AllocScope&) = delete;
 };
 void count_launch(int n = 1);
+// launch(first, count) over n descriptors in pieces that a grid's second extent holds
+template <class F>
+void in_grid_rows(int n, F&& launch) {
+  constexpr int kMost = 65535;
+  for (int first = 0; first < n; first += kMost) launch(first, unsigned(n - first < kMost ? n - first : kMost));
+}
 int num_sms();
 
 // device scratch for small results (absmax, truncation outputs)

@@ -314,9 +314,11 @@ void launch_qr(const xgb_qr_desc* d_descs, const xgb_qr_desc* h_descs, const int
     if (e != cudaSuccess) throw std::runtime_error(std::string("qr launch: ") + cudaGetErrorString(e));
     count_launch();
     if (q_cols > 0) {
-      qr_form_q_kernel<<<dim3(unsigned((q_cols + kQCols - 1) / kQCols), unsigned(n)), 32 * kQCols, size_t(q_bytes), s>>>(
-          d_descs, d_work_off, Q, work);
-      count_launch();
+      in_grid_rows(n, [&](int first, unsigned count) {
+        qr_form_q_kernel<<<dim3(unsigned((q_cols + kQCols - 1) / kQCols), count), 32 * kQCols, size_t(q_bytes), s>>>(
+            d_descs + first, d_work_off + first, Q, work);
+        count_launch();
+      });
     }
   }
   if (large) {

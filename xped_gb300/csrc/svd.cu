@@ -2209,16 +2209,18 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
                       stats, s);
   };
   sweeps(0);
-  const unsigned ny = unsigned(n);
-  svd_product_kernel<kProdAV><<<dim3(unsigned(av), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, 0, grid_most);
-  count_launch();
+  auto rows = [&](auto* kernel, int64_t x, int it) {
+    in_grid_rows(n, [&](int first, unsigned count) {
+      kernel<<<dim3(unsigned(x), count), 256, 0, s>>>(d_descs + first, d_off + first, A, U, Vt, work, it, grid_most);
+      count_launch();
+    });
+  };
+  rows(svd_product_kernel<kProdAV>, av, 0);
   for (int it = 0; it < kIters; ++it) {
-    svd_product_kernel<kProdGram><<<dim3(unsigned(gram), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, it, grid_most);
-    svd_update_kernel<<<dim3(unsigned(upd), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, it, grid_most);
-    count_launch(2);
+    rows(svd_product_kernel<kProdGram>, gram, it);
+    rows(svd_update_kernel, upd, it);
     if (it == kPass2) sweeps(1);
-    svd_product_kernel<kProdApply><<<dim3(unsigned(apply), ny), 256, 0, s>>>(d_descs, d_off, A, U, Vt, work, it, grid_most);
-    count_launch();
+    rows(svd_product_kernel<kProdApply>, apply, it);
   }
   for (int sector : wide) {
     const int64_t nn = std::min(h_descs[sector].m, h_descs[sector].n);
