@@ -7,7 +7,8 @@
 // step is that warp's chain (a dot product, an update, a norm, a square root and a division: GB300's dependent
 // FP64 operations take ~64 cycles, a division ~430, a square root ~675), one cluster barrier and the copy of
 // the reflector to the other CTAs, ~10k cycles together with 300 rows.  Reflectors stay unscaled (v = x with
-// v_j = 1 / scal), which takes a pass over the column off that chain.  qr_form_q_kernel: column c of Q is
+// v_j = 1 / scal), which takes a pass over the column off that chain, unless x is far from one: then a power of two
+// brings it there, so that its products with columns of any other scale stay in range.  qr_form_q_kernel: column c of Q is
 // H_0 .. H_c e_c, independent of the others: one warp a column, four (one per SM sub-partition) a CTA, over
 // all SMs.  One CTA per block (the kernel below, kept for blocks that no cluster's shared memory holds) was
 // bound by a single SM's FP64 pipe: five blocks of 120 x 40 to 308 x 128 took 7.4 ms there and take
@@ -33,6 +34,7 @@ constexpr int kWarps = kThreads / 32;
 constexpr int kMostCtas = 8;  // portable cluster size (16 gained 1 %: the chain bounds a step, not the update)
 constexpr int64_t kSmemLimit = 220 * 1024;
 constexpr int kQCols = 4;  // columns of Q per CTA
+constexpr int kUnscaled = 32;  // largest |exponent| of a reflector that stays as it is
 
 __device__ __forceinline__ double warp_sum(double v) {
 #pragma unroll
@@ -95,7 +97,14 @@ __global__ void __launch_bounds__(kThreads)
     if (ss > 0.0) {
       beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
       t = (beta - alpha) / beta;
-      sc = 1.0 / (alpha - beta);
+      const int e = int((__double_as_longlong(beta) >> 52) & 0x7ff) - 1023;
+      if (abs(e) <= kUnscaled || e > 1023) {  // (1024: infinite or NaN)
+        sc = 1.0 / (alpha - beta);
+      } else {
+        const double p = __longlong_as_double((long long)(1023 - e) << 52);  // 2^-e: |e| stays below 540
+        sc = 1.0 / ((alpha - beta) * p);
+        for (int i = j + 1 + lane; i < m; i += 32) x[i] *= p;
+      }
     }
     __syncwarp();
     if (lane == 0) {
