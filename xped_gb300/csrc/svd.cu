@@ -1097,6 +1097,10 @@ __device__ __forceinline__ float z_limit(int it) {
 // this fraction of the largest wait for the second iteration.
 __device__ __forceinline__ double z_gap(int it, double gmax) { return it == 0 ? 1.0e-9 * gmax : 0.0; }
 
+// The power of two by which the Gram entries enter z_pair: their products with one another stay in range for blocks
+// down to 1e-140 and up to 1e150 (unscaled ones left it at 1e77).
+__device__ __forceinline__ double z_scale(double gmax) { return pow2(-min(exponent_of(gmax), 1000)); }
+
 // First-order update of the pair (p, q), and whether it misses the tolerance (1) or is unresolved (2: far
 // from orthogonal and not a small rotation).
 __device__ __forceinline__ int z_pair(double g, double gp, double gq, double e, double floor, float lim, double gap,
@@ -1397,9 +1401,9 @@ __device__ void svd_small(const xgb_svd_desc& d, const double* __restrict__ A, d
     __syncthreads();
     double gmax = 0;
     for (int j = 0; j < nn; ++j) gmax = fmax(gmax, G[j * (ldv + 1)]);
-    const double floor = kFloor64 * gmax;
+    const double sc = z_scale(gmax), floor = kFloor64 * (sc * gmax);
     const float lim = z_limit(it);
-    const double gap = z_gap(it, gmax);
+    const double gap = z_gap(it, sc * gmax);
     float zmax = 0.f;
     for (int e = tid; e < nn * nn; e += kThreads) {
       const int p = e % nn, q = e / nn;
@@ -1411,7 +1415,7 @@ __device__ void svd_small(const xgb_svd_desc& d, const double* __restrict__ A, d
         continue;
       }
       double zpq, zqp;
-      const int s = z_pair(G[p + q * ldv], G[p * (ldv + 1)], G[q * (ldv + 1)], E[p + q * ldv], floor, lim,
+      const int s = z_pair(sc * G[p + q * ldv], sc * G[p * (ldv + 1)], sc * G[q * (ldv + 1)], E[p + q * ldv], floor, lim,
                            gap, zpq, zqp);
       if (s) atomicAdd(&unconv, 1);
       if (s == 2) atomicAdd(&unresolved, 1);
@@ -1692,9 +1696,9 @@ __global__ void __launch_bounds__(256)
   if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = gmax;
   __syncthreads();
   for (int w = 0; w < 8; ++w) gmax = fmax(gmax, red[w]);
-  const double floor = kFloor64 * gmax;
+  const double sc = z_scale(gmax), floor = kFloor64 * (sc * gmax);
   const float lim = z_limit(it);
-  const double gap = z_gap(it, gmax);
+  const double gap = z_gap(it, sc * gmax);
   int unconv = 0, unresolved = 0;
   float zmax = 0.f;
   for (int64_t e = int64_t(blockIdx.x) * 256 + threadIdx.x; e < nn * nn; e += int64_t(gridDim.x) * 256) {
@@ -1707,7 +1711,7 @@ __global__ void __launch_bounds__(256)
       continue;
     }
     double zpq, zqp;
-    const int s = z_pair(k.G[e], k.G[p * (nn + 1)], k.G[q * (nn + 1)], k.E[e], floor, lim, gap, zpq, zqp);
+    const int s = z_pair(sc * k.G[e], sc * k.G[p * (nn + 1)], sc * k.G[q * (nn + 1)], k.E[e], floor, lim, gap, zpq, zqp);
     unconv += s != 0;
     unresolved += s == 2;
     k.E[e] = zpq;
