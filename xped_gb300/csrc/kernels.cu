@@ -847,20 +847,37 @@ void launch_diag_apply(const xgb_copy2d_desc* d_descs, int n, int64_t max_k, int
 }
 
 // A Tensor<2,3> with a diagonal Tensor<1,1> on each of its first four legs: y = (((x wL) wT) wR) wB entry by entry, one
-// warp per 256 entries of a fusion-tree pair's sub-block.  Each weight costs one multiplication where contracting it
+// warp per 256 entries of a fusion-tree pair's sub-block (found in the prefix sums of the pairs' chunks, so that the
+// tables do not grow with the degeneracies).  Each weight costs one multiplication where contracting it
 // takes a permute of the tensor to the leg, a product with the weight's blocks and a permute back (13 launches of small
 // kernels instead of one; a D = 6 simple-update step 6.2 ms instead of 4.0).  Bound by launch and load latency for such
 // tensors, by HBM for large ones.
 __global__ void __launch_bounds__(256) leg_weights_kernel(const LegWeightTask* __restrict__ tasks, int n,
+                                                          int64_t chunks, const int64_t* __restrict__ start,
                                                           LegWeights w, const double* __restrict__ x,
                                                           double* __restrict__ y) {
-  const int t = blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (t >= n) return;
-  const LegWeightTask& k = tasks[t];
+  constexpr int kHeld = 512;
+  __shared__ int64_t start_s[kHeld];
+  const bool held = n <= kHeld;
+  if (held)
+    for (int i = threadIdx.x; i < n; i += blockDim.x) start_s[i] = start[i];
+  __syncthreads();
+  const int64_t c = int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5);
+  if (c >= chunks) return;
+  const int64_t* at = held ? start_s : start;
+  int a = 0, b = n - 1;
+  while (a < b) {
+    const int mid = (a + b + 1) >> 1;
+    if (at[mid] <= c) a = mid;
+    else b = mid - 1;
+  }
+  const LegWeightTask& k = tasks[a];
+  const int64_t first = (c - at[a]) * kLegWeightChunk;
+  const int64_t last = first + kLegWeightChunk < k.entries ? first + kLegWeightChunk : k.entries;
   const int lane = threadIdx.x & 31;
   auto entries = [&](auto index) {  // 32-bit divisions where the sub-block's entries fit
     using Index = decltype(index);
-    for (int64_t e = k.first + lane; e < k.last; e += 32) {
+    for (int64_t e = first + lane; e < last; e += 32) {
       Index r = Index(e);
       int64_t src = k.src, dst = k.dst;
       int i[5];
@@ -878,14 +895,14 @@ __global__ void __launch_bounds__(256) leg_weights_kernel(const LegWeightTask* _
       y[dst] = v;
     }
   };
-  if (k.last <= INT32_MAX) entries(uint32_t(0));
+  if (k.entries <= INT32_MAX) entries(uint32_t(0));
   else entries(uint64_t(0));
 }
 
-void launch_leg_weights(const LegWeightTask* d_tasks, int n, const LegWeights& w, const double* x, double* y,
-                        cudaStream_t s) {
-  if (n <= 0) return;
-  leg_weights_kernel<<<(n + 7) / 8, 256, 0, s>>>(d_tasks, n, w, x, y);
+void launch_leg_weights(const LegWeightTask* d_tasks, const int64_t* d_start, int n, int64_t chunks, const LegWeights& w,
+                        const double* x, double* y, cudaStream_t s) {
+  if (n <= 0 || chunks <= 0) return;
+  leg_weights_kernel<<<unsigned((chunks + 7) / 8), 256, 0, s>>>(d_tasks, n, chunks, d_start, w, x, y);
   count_launch();
 }
 

@@ -149,16 +149,18 @@ void launch_copy2d(const xgb_copy2d_desc* d_descs, int n, int64_t max_elems, con
 void launch_diag_from_vec(const xgb_copy2d_desc* d_descs, int n, int64_t max_k, int fn, const double* src, double* dst,
                           cudaStream_t s);
 void launch_diag_apply(const xgb_copy2d_desc* d_descs, int n, int64_t max_k, int fn, double* x, cudaStream_t s);
-// diagonal weights on the first four legs of a Tensor<2,3>: entries [first, last) of a sub-block
+// diagonal weights on the first four legs of a Tensor<2,3>: one sub-block, in chunks of kLegWeightChunk entries
+constexpr int64_t kLegWeightChunk = 256;
 struct LegWeightTask {
-  int64_t src, dst, first, last;
+  int64_t src, dst, entries;
   int64_t src_stride[5], dst_stride[5];
   int64_t weight[4], weight_step[4];  // first diagonal entry of the leg's charge, and the step to the next
   int32_t dims[5];
 };
 struct LegWeights { const double* data[4]; };
-void launch_leg_weights(const LegWeightTask* d_tasks, int n, const LegWeights& w, const double* x, double* y,
-                        cudaStream_t s);
+// d_start: chunks before each task, and their total
+void launch_leg_weights(const LegWeightTask* d_tasks, const int64_t* d_start, int n, int64_t chunks, const LegWeights& w,
+                        const double* x, double* y, cudaStream_t s);
 
 // split-precision (3xTF32) tensor-core grouped GEMM (gemm_tc.cu): operands packed into
 // 16 KB hi/lo chunks (128 rows x 32 K, canonical MMA layout), 128 x 128 output tiles

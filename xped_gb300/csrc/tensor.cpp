@@ -208,7 +208,9 @@ struct WeightPlan {
   MetaPtr out;
   bool needs_zero = false;
   int n_tasks = 0;
+  int64_t n_chunks = 0;
   LegWeightTask* d_tasks = nullptr;
+  int64_t* d_start = nullptr;
   double bytes = 0;
 };
 std::mutex g_plan_mu;
@@ -1248,6 +1250,7 @@ std::shared_ptr<WeightPlan> build_weight_plan(const TensorMeta& m, const std::ar
   plan->out = make_meta(m.sym, {w[0]->dom[0], w[1]->dom[0]}, {w[2]->cod[0], w[3]->cod[0], m.cod[2]});
   const TensorMeta& o = *plan->out;
   std::vector<LegWeightTask> tasks;
+  std::vector<int64_t> start{0};
   int64_t written = 0;
   for (size_t si = 0; si < m.sectors.size(); ++si) {
     const int q = m.sectors[si], oq = o.index(q);
@@ -1274,17 +1277,18 @@ std::shared_ptr<WeightPlan> build_weight_plan(const TensorMeta& m, const std::ar
         k.dst = o.offset[oq] + o.cdom->left_offset(f1) + o.ccod->left_offset(f2) * o.rows[oq];
         sub_strides(f1, f2, m.rows[si], k.src_stride);
         sub_strides(f1, f2, o.rows[oq], k.dst_stride);
-        for (k.first = 0; k.first < n; k.first += 256) {
-          k.last = std::min<int64_t>(n, k.first + 256);
-          tasks.push_back(k);
-        }
+        k.entries = n;
+        tasks.push_back(k);
+        start.push_back(start.back() + (n + kLegWeightChunk - 1) / kLegWeightChunk);
         written += n;
       }
   }
   plan->n_tasks = int(tasks.size());
+  plan->n_chunks = start.back();
   plan->needs_zero = written != o.size;
   plan->bytes = 16.0 * double(written);
   plan->d_tasks = plan->mem.table(tasks);
+  plan->d_start = plan->mem.table(start);
   return plan;
 }
 }  // namespace
@@ -1312,8 +1316,8 @@ Tensor apply_weights(const Tensor& A, const Tensor& wL, const Tensor& wT, const 
   }
   Tensor out = plan->needs_zero ? zeros(plan->out) : empty_like_meta(plan->out);
   prof_begin(K_DIAG, stream());
-  launch_leg_weights(plan->d_tasks, plan->n_tasks, {{w[0].data(), w[1].data(), w[2].data(), w[3].data()}}, t.data(),
-                     out.data(), stream());
+  launch_leg_weights(plan->d_tasks, plan->d_start, plan->n_tasks, plan->n_chunks,
+                     {{w[0].data(), w[1].data(), w[2].data(), w[3].data()}}, t.data(), out.data(), stream());
   prof_end(K_DIAG, stream(), plan->bytes);
   return out;
 }
