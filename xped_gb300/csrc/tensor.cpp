@@ -1254,7 +1254,7 @@ std::shared_ptr<WeightPlan> build_weight_plan(const TensorMeta& m, const std::ar
   int64_t written = 0;
   for (size_t si = 0; si < m.sectors.size(); ++si) {
     const int q = m.sectors[si], oq = o.index(q);
-    if (oq < 0) throw std::runtime_error("weights: output sector missing");
+    if (oq < 0) continue;  // reached by charges that a weight does not carry alone
     for (const auto& f1 : m.cdom->trees[m.cdom->index(q)])
       for (const auto& f2 : m.ccod->trees[m.ccod->index(q)]) {
         LegWeightTask k{};
