@@ -1385,17 +1385,34 @@ __device__ void svd_small(const xgb_svd_desc& d, const double* __restrict__ A, d
   double *W = Wb, *Wn = Wa, *V = Va, *Vn = Vb;
   float zprev = 1.0f;
   int it = 0;
+  // Gram entries: a thread each, or, in tall blocks of few columns, a warp each.  FP64 warp instructions of an SM quarter:
+  // mm for every 128 entries, or (mm / 32 + 10) for every 4 (5000 x 1: 516 us with one thread over all rows, 121 so).
+  const int entries = nn * (nn + 1) / 2;
+  const bool tall = mm >= 256 && 4 * ((entries + 127) / 128) * mm > entries * (mm / 32 + 10);
+  auto pair_of = [](int e, int& p, int& q) {
+    q = int((sqrtf(8.0f * float(e) + 1.0f) - 1.0f) * 0.5f);
+    while ((q + 1) * (q + 2) / 2 <= e) ++q;
+    while (q * (q + 1) / 2 > e) --q;
+    p = e - q * (q + 1) / 2;
+  };
   for (; it < kIters; ++it) {
-    for (int e = tid; e < nn * (nn + 1) / 2; e += kThreads) {
-      int q = int((sqrtf(8.0f * float(e) + 1.0f) - 1.0f) * 0.5f);
-      while ((q + 1) * (q + 2) / 2 <= e) ++q;
-      while (q * (q + 1) / 2 > e) --q;
-      const int p = e - q * (q + 1) / 2;
+    for (int e = tid; e < entries; e += kThreads) {
+      int p, q;
+      pair_of(e, p, q);
       double g = 0, v = 0;
-      for (int i = 0; i < mm; ++i) g = fma(W[i + p * ldw], W[i + q * ldw], g);
+      if (!tall)
+        for (int i = 0; i < mm; ++i) g = fma(W[i + p * ldw], W[i + q * ldw], g);
       for (int i = 0; i < nn; ++i) v = fma(V[i + p * ldv], V[i + q * ldv], v);
-      G[p + q * ldv] = g;
+      if (!tall) G[p + q * ldv] = g;
       E[p + q * ldv] = v;
+    }
+    for (int e = warp; tall && e < entries; e += kWarps) {
+      int p, q;
+      pair_of(e, p, q);
+      double g = 0;
+      for (int i = lane; i < mm; i += 32) g = fma(W[i + p * ldw], W[i + q * ldw], g);
+      g = wsum(g);
+      if (lane == 0) G[p + q * ldv] = g;
     }
     if (tid == 0) unconv = unresolved = zbits = 0;
     __syncthreads();
