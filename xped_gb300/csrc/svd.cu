@@ -1034,7 +1034,7 @@ __device__ void finish_svd(Group& cl, const Ctx& c, const xgb_svd_desc& d, bool 
 // ---------------------------------------------------------------- state of one block
 // Workspace of a block wider than kSmallN (doubles): W0 mm*nn | V0 nn*nn | G nn*nn | E nn*nn | n64 nn | misc 10 | the
 // FP32 columns W32 (mm*nn floats) of a pass 0 that no cluster holds, from a 32-byte sector on (columns across sectors:
-// 3000 x 400 graded 761 ms instead of 511); their rotations V32 lie in E.
+// 3000 x 400 graded 761 ms instead of 511); their rotations V32 lie in E.  Later W32 is room for partial Gram sums.
 // The second W / V pair of the refinement is the block's own U / V^T output, written only once A has been read for
 // the last time (W = op(A) V): an output may overlap its block of A.
 struct Block {
@@ -1551,7 +1551,17 @@ __global__ void __launch_bounds__(kThreads)
 // CTAs of a block's FP32 sweeps on a cluster of at most `most`
 __host__ __device__ __forceinline__ int sweep_ctas(int pass, int64_t mm, int64_t nn, int most) {
   const Shape32 sh = shape32(pass, mm, nn, most, kSmemLimit);
-  return sh.P ? sh.P : most;  // (too large for any: jacobi32_global or block_jacobi on all of them)
+  if (sh.P) return sh.P;
+  // too large for any: jacobi32_global or block_jacobi on all of them, but no more than give each of their 2P column
+  // blocks a column (with 16 CTAs eight columns met in 31 rounds of one pair instead of seven of four: 1000000 x 8
+  // 780 ms instead of 322), unless two single columns fit shared memory where two blocks do not (20000 x 30 graded 41
+  // ms on 16 CTAs, 92 on 8)
+  auto staged = [&](int P) { return 8 * ((nn + 2 * P - 1) / (2 * P)) * (mm + nn + 1) <= kSmemLimit; };
+  int P = 1;
+  while (2 * P <= most && 4 * P <= nn) P *= 2;
+  if (staged(most))
+    while (!staged(P)) P *= 2;
+  return P;
 }
 
 // Whether a block takes svd_factor_kernel; `grid_most`: most CTAs per cluster, 0 where no cooperative grid is launched.
@@ -1650,6 +1660,19 @@ __device__ __forceinline__ void tile_product(const double* __restrict__ A, int64
 
 __host__ __device__ __forceinline__ int64_t svd_tiles(int64_t x) { return (x + kTile - 1) / kTile; }
 
+// Row ranges that the tiles of W^T W are cut into: a thin block has few tiles, and one CTA over all rows of each kept the
+// other SMs waiting (1000000 x 2: 255 ms, of which about 200 for three Gram products; 42 cut).  Four CTAs per SM, at least 512
+// rows each, and partial sums (from W32 on, free by then) that fit mm nn / 2 doubles.  Below 4096 rows the rest of an
+// iteration is as long.
+__host__ __device__ __forceinline__ int64_t gram_splits(int64_t mm, int64_t nn) {
+  if (mm < 4096) return 1;
+  const int64_t nt = svd_tiles(nn);
+  int64_t s = 608 / (nt * (nt + 1) / 2);
+  if (s > mm / 512) s = mm / 512;
+  if (s > mm / (2 * nn)) s = mm / (2 * nn);
+  return s > 1 ? s : 1;
+}
+
 enum { kProdAV = 0, kProdGram = 1, kProdApply = 2 };
 
 // W = op(A) V (kProdAV), G = W^T W and E = V^T V on and above the diagonal (kProdGram), or W (I + Z) and
@@ -1665,7 +1688,8 @@ __global__ void __launch_bounds__(256)
   if (k.nn == 0 || small_block(k.mm, k.nn) || factored(k.mm, k.nn, grid_most)) return;
   const int64_t nt = svd_tiles(k.nn), mt = svd_tiles(k.mm);
   int64_t t = blockIdx.x;
-  if (t >= (kMode == kProdAV ? mt * nt : kMode == kProdGram ? 2 * nt * nt : mt * nt + nt * nt)) return;
+  const int64_t splits = kMode == kProdGram ? gram_splits(k.mm, k.nn) : 1;
+  if (t >= (kMode == kProdAV ? mt * nt : kMode == kProdGram ? (splits + 1) * nt * nt : mt * nt + nt * nt)) return;
   auto run = [&](const double* a, int64_t lda, bool ta, const double* b, int64_t ldb, double* c, int64_t ldc, int64_t M,
                  int64_t K, int64_t tm, int64_t tn) {
     tile_product(a, lda, ta, b, ldb, c, ldc, M, k.nn, K, tm, tn, sm);
@@ -1679,11 +1703,16 @@ __global__ void __launch_bounds__(256)
   const double* W = cur ? k.W1 : k.W0;
   const double* V = cur ? k.V1 : k.V0;
   if (kMode == kProdGram) {
-    const bool e = t >= nt * nt;
-    if (e) t -= nt * nt;
+    const int64_t part = t / (nt * nt);  // a row range of G, or (the last one) E
+    t -= part * nt * nt;
     if (t % nt > t / nt) return;
-    if (e) run(V, k.nn, true, V, k.nn, k.E, k.nn, k.nn, k.nn, t % nt, t / nt);
-    else run(W, k.mm, true, W, k.mm, k.G, k.nn, k.nn, k.mm, t % nt, t / nt);
+    if (part == splits) {
+      run(V, k.nn, true, V, k.nn, k.E, k.nn, k.nn, k.nn, t % nt, t / nt);
+      return;
+    }
+    const int64_t rows = (k.mm + splits - 1) / splits, r0 = part * rows, here = k.mm - r0 < rows ? k.mm - r0 : rows;
+    double* g = splits > 1 ? reinterpret_cast<double*>(k.W32) + part * k.nn * k.nn : k.G;
+    run(W + r0, k.mm, true, W + r0, k.mm, g, k.nn, k.nn, here, t % nt, t / nt);
     return;
   }
   if (t < mt * nt) {
@@ -1692,6 +1721,24 @@ __global__ void __launch_bounds__(256)
     t -= mt * nt;
     run(V, k.nn, false, k.E, k.nn, cur ? k.V0 : k.V1, k.nn, k.nn, k.nn, t % nt, t / nt);
   }
+}
+
+// G of the blocks whose Gram product was cut: its row ranges' sums, added in order.
+__global__ void __launch_bounds__(256)
+    svd_gram_sum_kernel(const xgb_svd_desc* __restrict__ descs, const int64_t* __restrict__ work_off,
+                        const double* __restrict__ A, double* __restrict__ U, double* __restrict__ Vt,
+                        double* __restrict__ work, int it, int grid_most) {
+  const int sector = blockIdx.y;
+  const Block k = block_of(descs[sector], work_off[sector], A, U, Vt, work);
+  if (k.nn == 0 || small_block(k.mm, k.nn) || factored(k.mm, k.nn, grid_most)) return;
+  const int64_t splits = gram_splits(k.mm, k.nn), nn2 = int64_t(k.nn) * k.nn, e = int64_t(blockIdx.x) * 256 + threadIdx.x;
+  if (splits == 1 || e >= nn2 || e % k.nn > e / k.nn) return;
+  if (it > 0 && !iter_on(k.misc, it - 1)) return;
+  const double* part = reinterpret_cast<const double*>(k.W32) + e;
+  double g = part[0];
+#pragma unroll 8
+  for (int64_t s = 1; s < splits; ++s) g += part[s * nn2];
+  k.G[e] = g;
 }
 
 // E <- I + Z from G and E, and the block's convergence state of this iteration.
@@ -2175,7 +2222,7 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
   const int most = g_most_ctas[PerDevice::current()];
   int64_t small_bytes = 0;
   int narrow[2] = {0, 0}, broad[2] = {0, 0};  // CTAs of the two sweep launches of each pass
-  int64_t av = 0, gram = 0, apply = 0, upd = 0;
+  int64_t av = 0, gram = 0, cut = 0, apply = 0, upd = 0;
   std::vector<int> factor, wide;  // blocks of svd_factor_kernel; those whose pass 1 and polish take the cooperative grid
   const int widest[2] = {INT32_MAX, grid ? kGridN : INT32_MAX};
   const int grid_most = grid ? most : 0;
@@ -2198,7 +2245,9 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
     }
     const int64_t nt = svd_tiles(nn), mt = svd_tiles(mm);
     av = std::max(av, mt * nt);
-    gram = std::max(gram, 2 * nt * nt);
+    const int64_t splits = gram_splits(mm, nn);
+    gram = std::max(gram, (splits + 1) * nt * nt);
+    if (splits > 1) cut = std::max(cut, (nn * nn + 255) / 256);
     apply = std::max(apply, mt * nt + nt * nt);
     upd = std::max(upd, std::min<int64_t>((nn * nn + 255) / 256, 1024));
   }
@@ -2239,6 +2288,7 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
   rows(svd_product_kernel<kProdAV>, av, 0);
   for (int it = 0; it < kIters; ++it) {
     rows(svd_product_kernel<kProdGram>, gram, it);
+    if (cut) rows(svd_gram_sum_kernel, cut, it);
     rows(svd_update_kernel, upd, it);
     if (it == kPass2) sweeps(1);
     rows(svd_product_kernel<kProdApply>, apply, it);
