@@ -347,6 +347,12 @@ void launch_permute(const PlaneTask* d_tasks, const int64_t* d_start, int n_task
 
 namespace {
 
+// Planes of the output's two fast legs smaller than this take the longest of the other legs in place of the second: a
+// plane costs its decoding, some 100 instructions, whatever it holds.  Measured (us, second leg / longest leg): [2, 5 M, 3]
+// -> (0,2,1) 1680 / 203, twenty of [3, 200, 2, 200] -> (0,2,1,3) 56 / 38, a hundred of [2^5, 1000] -> (0,2,1,4,3,5) 62 /
+// 51; planes of 36 ([6, 6, 200, 200] -> (0,1,3,2)) 42 either way.
+constexpr int64_t kSmallPlane = 32;
+
 // lanes x (of g) along a leg of extent n, r = g / x along one of extent m: few left over, runs not too short, that is
 // the largest share of busy lanes, n m / (g ceil(n / x) ceil(m / r)), times x / (x + 8).  For each r only the largest x
 // can be the best: ten candidates of 32.
@@ -445,7 +451,10 @@ PlanePlan plan_planes(const xgb_perm_task* tasks, int n_tasks, const xgb_perm_co
       }
       return span <= INT32_MAX;
     };
-    const int b = sh.n < 2 ? -1 : plan.form.transpose && sh.fast > 0 ? sh.fast : 1;
+    int b = sh.n < 2 ? -1 : plan.form.transpose && sh.fast > 0 ? sh.fast : 1;
+    if (b == 1 && sh.dim[0] * sh.dim[1] < kSmallPlane)
+      for (int i = 2; i < sh.n; ++i)
+        if (sh.dim[i] > sh.dim[b]) b = i;
     PlaneTask& p = plan.tasks.emplace_back();
     p.dst_base = k.dst_base;
     p.na = sh.n > 0 ? int32_t(sh.dim[0]) : 1;
