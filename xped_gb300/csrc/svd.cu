@@ -1673,10 +1673,12 @@ __host__ __device__ __forceinline__ int64_t gram_splits(int64_t mm, int64_t nn) 
   return s > 1 ? s : 1;
 }
 
-enum { kProdAV = 0, kProdGram = 1, kProdApply = 2 };
+enum { kProdAV, kProdGram, kProdGramUncut, kProdCut, kProdApply };
 
-// W = op(A) V (kProdAV), G = W^T W and E = V^T V on and above the diagonal (kProdGram), or W (I + Z) and
-// V (I + Z) (kProdApply, I + Z in E): one launch over all blocks, blockIdx.y = block.
+// W = op(A) V (kProdAV), G = W^T W and E = V^T V on and above the diagonal (kProdGram), or W (I + Z) and V (I + Z)
+// (kProdApply, I + Z in E): one launch over all blocks, blockIdx.y = block.  Batches with blocks whose Gram product is
+// cut take kProdCut for those and kProdGramUncut for the rest of G and E: in one kernel they cost every batch 19
+// registers, 1.2 % of a plain CTM step.
 template <int kMode>
 __global__ void __launch_bounds__(256)
     svd_product_kernel(const xgb_svd_desc* __restrict__ descs, const int64_t* __restrict__ work_off,
@@ -1688,8 +1690,11 @@ __global__ void __launch_bounds__(256)
   if (k.nn == 0 || small_block(k.mm, k.nn) || factored(k.mm, k.nn, grid_most)) return;
   const int64_t nt = svd_tiles(k.nn), mt = svd_tiles(k.mm);
   int64_t t = blockIdx.x;
-  const int64_t splits = kMode == kProdGram ? gram_splits(k.mm, k.nn) : 1;
-  if (t >= (kMode == kProdAV ? mt * nt : kMode == kProdGram ? (splits + 1) * nt * nt : mt * nt + nt * nt)) return;
+  const int64_t splits = kMode == kProdCut ? gram_splits(k.mm, k.nn) : 1;
+  if (kMode == kProdCut && splits == 1) return;
+  constexpr bool kGram = kMode == kProdGram || kMode == kProdGramUncut;
+  if (t >= (kMode == kProdAV ? mt * nt : kGram ? 2 * nt * nt : kMode == kProdCut ? splits * nt * nt : mt * nt + nt * nt))
+    return;
   auto run = [&](const double* a, int64_t lda, bool ta, const double* b, int64_t ldb, double* c, int64_t ldc, int64_t M,
                  int64_t K, int64_t tm, int64_t tn) {
     tile_product(a, lda, ta, b, ldb, c, ldc, M, k.nn, K, tm, tn, sm);
@@ -1698,21 +1703,25 @@ __global__ void __launch_bounds__(256)
     run(k.A, k.lda, k.tr, k.V0, k.nn, k.W0, k.mm, k.mm, k.nn, t % mt, t / mt);
     return;
   }
-  if (kMode == kProdGram ? (it > 0 && !iter_on(k.misc, it - 1)) : !iter_on(k.misc, it)) return;
+  if (kMode != kProdApply ? (it > 0 && !iter_on(k.misc, it - 1)) : !iter_on(k.misc, it)) return;
   const int cur = iters_done(k.misc, it) & 1;
   const double* W = cur ? k.W1 : k.W0;
   const double* V = cur ? k.V1 : k.V0;
-  if (kMode == kProdGram) {
-    const int64_t part = t / (nt * nt);  // a row range of G, or (the last one) E
+  if (kGram) {
+    const bool e = t >= nt * nt;
+    if (e) t -= nt * nt;
+    if (t % nt > t / nt) return;
+    if (e) run(V, k.nn, true, V, k.nn, k.E, k.nn, k.nn, k.nn, t % nt, t / nt);
+    else if (kMode == kProdGram || gram_splits(k.mm, k.nn) == 1)
+      run(W, k.mm, true, W, k.mm, k.G, k.nn, k.nn, k.mm, t % nt, t / nt);
+    return;
+  }
+  if (kMode == kProdCut) {
+    const int64_t part = t / (nt * nt), rows = (k.mm + splits - 1) / splits, r0 = part * rows;
     t -= part * nt * nt;
     if (t % nt > t / nt) return;
-    if (part == splits) {
-      run(V, k.nn, true, V, k.nn, k.E, k.nn, k.nn, k.nn, t % nt, t / nt);
-      return;
-    }
-    const int64_t rows = (k.mm + splits - 1) / splits, r0 = part * rows, here = k.mm - r0 < rows ? k.mm - r0 : rows;
-    double* g = splits > 1 ? reinterpret_cast<double*>(k.W32) + part * k.nn * k.nn : k.G;
-    run(W + r0, k.mm, true, W + r0, k.mm, g, k.nn, k.nn, here, t % nt, t / nt);
+    run(W + r0, k.mm, true, W + r0, k.mm, reinterpret_cast<double*>(k.W32) + part * k.nn * k.nn, k.nn, k.nn,
+        k.mm - r0 < rows ? k.mm - r0 : rows, t % nt, t / nt);
     return;
   }
   if (t < mt * nt) {
@@ -2222,7 +2231,7 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
   const int most = g_most_ctas[PerDevice::current()];
   int64_t small_bytes = 0;
   int narrow[2] = {0, 0}, broad[2] = {0, 0};  // CTAs of the two sweep launches of each pass
-  int64_t av = 0, gram = 0, cut = 0, apply = 0, upd = 0;
+  int64_t av = 0, gram = 0, cut = 0, sum = 0, apply = 0, upd = 0;
   std::vector<int> factor, wide;  // blocks of svd_factor_kernel; those whose pass 1 and polish take the cooperative grid
   const int widest[2] = {INT32_MAX, grid ? kGridN : INT32_MAX};
   const int grid_most = grid ? most : 0;
@@ -2246,8 +2255,11 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
     const int64_t nt = svd_tiles(nn), mt = svd_tiles(mm);
     av = std::max(av, mt * nt);
     const int64_t splits = gram_splits(mm, nn);
-    gram = std::max(gram, (splits + 1) * nt * nt);
-    if (splits > 1) cut = std::max(cut, (nn * nn + 255) / 256);
+    gram = std::max(gram, 2 * nt * nt);
+    if (splits > 1) {
+      cut = std::max(cut, splits * nt * nt);
+      sum = std::max(sum, (nn * nn + 255) / 256);
+    }
     apply = std::max(apply, mt * nt + nt * nt);
     upd = std::max(upd, std::min<int64_t>((nn * nn + 255) / 256, 1024));
   }
@@ -2287,8 +2299,13 @@ void svd_pipeline(const xgb_svd_desc* d_descs, const xgb_svd_desc* h_descs, cons
   };
   rows(svd_product_kernel<kProdAV>, av, 0);
   for (int it = 0; it < kIters; ++it) {
-    rows(svd_product_kernel<kProdGram>, gram, it);
-    if (cut) rows(svd_gram_sum_kernel, cut, it);
+    if (cut) {
+      rows(svd_product_kernel<kProdGramUncut>, gram, it);
+      rows(svd_product_kernel<kProdCut>, cut, it);
+      rows(svd_gram_sum_kernel, sum, it);
+    } else {
+      rows(svd_product_kernel<kProdGram>, gram, it);
+    }
     rows(svd_update_kernel, upd, it);
     if (it == kPass2) sweeps(1);
     rows(svd_product_kernel<kProdApply>, apply, it);
