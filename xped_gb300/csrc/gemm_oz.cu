@@ -72,6 +72,7 @@ constexpr int kDrainCols = ON / (kOzDrainWarps / 4);  // columns of a drain warp
 constexpr long long kOzSpin = 1ll << 26;
 constexpr int kReduceThreads = 256;
 constexpr int kPackRows = 32;                       // rows of a slicing cluster
+constexpr int kPackCluster = 8;                     // its CTAs at most
 constexpr uint32_t kSboBytes = 128;                 // next 8-row group
 // A: seven separate 128-row pieces.  B: the seven 64-row pieces stacked into one 448-row operand (row
 // group g of piece s is row group 8 s + g), so that pieces t .. t + c - 1 form one N = 64 c operand
@@ -229,7 +230,11 @@ __device__ __forceinline__ void store_slice(unsigned char* at, int stride, const
 // 14 bytes written per entry for large operands, by the reads' latency for small ones.
 // Measured (nine blocks of 100 to 1729 squared, both operands): 233 us as a maximum kernel (with atomics) and a slicing
 // kernel with 64-bit digit arithmetic, 114 now.
-__global__ void __launch_bounds__(256) oz_pack_kernel(const xgb_gemm_desc* __restrict__ descs,
+// A list of few rows and a long k (a full contraction) has no CTAs for all SMs in clusters of eight: kMax and kSlice do the
+// two halves in launches of their own, over any number of CTAs per task, with the maxima in `rowmax` (cleared before).
+enum PackForm { kWhole, kMax, kSlice };
+template <PackForm kForm>
+__global__ void __launch_bounds__(256) oz_pack_kernel(int ctas, const xgb_gemm_desc* __restrict__ descs,
                                                        const OzGroup* __restrict__ groups,
                                                        const TcPackTask* __restrict__ tasks,
                                                        const double* __restrict__ A, const double* __restrict__ B,
@@ -238,7 +243,8 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const xgb_gemm_desc* __res
                                                        unsigned char* __restrict__ bpack) {
   __shared__ unsigned long long part[256], own[kPackRows];
   cg::cluster_group cluster = cg::this_cluster();
-  const int P = int(cluster.num_blocks()), me = int(cluster.block_rank());
+  const int P = kForm == kWhole ? int(cluster.num_blocks()) : ctas;
+  const int me = kForm == kWhole ? int(cluster.block_rank()) : int(blockIdx.x % unsigned(P));
   const TcPackTask t = tasks[blockIdx.x / unsigned(P)];
   const xgb_gemm_desc d = descs[t.g];
   const OzGroup gr = groups[t.g];
@@ -273,8 +279,9 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const xgb_gemm_desc* __res
 #pragma unroll
     for (int j = 0; j < 8; ++j) x[j] = live && k + j < d.k ? __ldg(at + j * step) : 0.0;
   };
+  unsigned long long* rmax = rowmax + (isB ? gr.b_rowmax : gr.a_rowmax) + row;
   unsigned long long m = 0;
-  for (int g = first; g < last; g += nq) {
+  for (int g = first; kForm != kSlice && g < last; g += nq) {
     double x[8];
     load8(g, x);
 #pragma unroll
@@ -283,22 +290,31 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const xgb_gemm_desc* __res
       m = m > b ? m : b;
     }
   }
-  part[threadIdx.x] = m;
-  __syncthreads();
-  if (int(threadIdx.x) < tr) {
-    for (int p = 1; p < nq; ++p) m = m > part[p * tr + r] ? m : part[p * tr + r];
-    own[r] = m;
-  }
-  cluster.sync();
-  if (int(threadIdx.x) < tr) {
-    for (int p = 0; p < P; ++p) {
-      const unsigned long long o = cluster.map_shared_rank(own, p)[r];
-      m = m > o ? m : o;
+  if constexpr (kForm == kSlice) {
+    if (int(threadIdx.x) < tr) part[r] = live ? *rmax : 0ull;
+    __syncthreads();
+  } else {
+    part[threadIdx.x] = m;
+    __syncthreads();
+    if (int(threadIdx.x) < tr) {
+      for (int p = 1; p < nq; ++p) m = m > part[p * tr + r] ? m : part[p * tr + r];
+      own[r] = m;
     }
-    part[r] = m;
-    if (me == 0 && live) rowmax[(isB ? gr.b_rowmax : gr.a_rowmax) + row] = m;
+    if constexpr (kForm == kMax) {
+      if (int(threadIdx.x) < tr && live && m) atomicMax(rmax, m);
+      return;
+    }
+    cluster.sync();
+    if (int(threadIdx.x) < tr) {
+      for (int p = 0; p < P; ++p) {
+        const unsigned long long o = cluster.map_shared_rank(own, p)[r];
+        m = m > o ? m : o;
+      }
+      part[r] = m;
+      if (me == 0 && live) *rmax = m;
+    }
+    cluster.sync();  // `own` of every CTA has been read
   }
-  cluster.sync();  // `own` of every CTA has been read
   const int e = row_scale(part[r]);
   // block of one (tile, K slice): kPieces pieces of tr x OK BF16, each in canonical layout
   const int piece_bytes = isB ? kBPieceBytes : kAPieceBytes;
@@ -319,6 +335,16 @@ __global__ void __launch_bounds__(256) oz_pack_kernel(const xgb_gemm_desc* __res
     store_slice<1>(base + int64_t(g / (OK / 8)) * (kPieces * piece_bytes) + (g % (OK / 8)) * lbo, piece_stride, lo,
                    hi, sign);
   }
+}
+
+// the maxima of each task's rows to zero
+__global__ void oz_clear_kernel(const xgb_gemm_desc* __restrict__ descs, const OzGroup* __restrict__ groups,
+                                const TcPackTask* __restrict__ tasks, unsigned long long* __restrict__ rowmax) {
+  const TcPackTask t = tasks[blockIdx.x];
+  const OzGroup gr = groups[t.g];
+  const bool sb = (t.which != 0) != (gr.swap != 0);
+  const int64_t row = int64_t(t.tile) * kPackRows + threadIdx.x;
+  if (row < (sb ? descs[t.g].n : descs[t.g].m)) rowmax[(t.which ? gr.b_rowmax : gr.a_rowmax) + row] = 0;
 }
 
 // ----------------------------------------------------------------------------- gemm
@@ -650,11 +676,19 @@ OzPlanHost build_oz_plan(const xgb_gemm_desc* descs, int n, bool allow_swap) {
     p.a_bytes += int64_t(gr.a_tiles) * gr.slices * kPieces * kAPieceBytes;
     p.b_bytes += int64_t(gr.b_tiles) * gr.slices * kPieces * kBPieceBytes;
     // clusters that slice the operands: at most 128 k values per CTA, eight CTAs
-    while (p.pack_cluster < 8 && gr.slices * OK > 128 * p.pack_cluster) p.pack_cluster *= 2;
+    while (p.pack_cluster < kPackCluster && gr.slices * OK > 128 * p.pack_cluster) p.pack_cluster *= 2;
     for (int32_t t = 0; t < gr.a_tiles * (OM / kPackRows); ++t) p.tasks_a.push_back({g, t, 0, 0});
     for (int32_t t = 0; t < gr.b_tiles * (ON / kPackRows); ++t) p.tasks_b.push_back({g, t, 0, 1});
     p.groups.push_back(gr);
   }
+  // few tasks over a long k: the slicing in launches of its own over four CTAs per SM, at least 512 k values each (the
+  // whole product, us: 4 x 4 x 100000 581 in clusters of eight, 213 so; 1 x 1 x 10000 90 and 76; at k = 2000 the launches
+  // cost more than the CTAs gain)
+  const int64_t sms = num_sms() > 0 ? num_sms() : 152, n_tasks = int64_t(p.tasks_a.size() + p.tasks_b.size());
+  int64_t kmax = 0;
+  for (const auto& gr : p.groups) kmax = std::max<int64_t>(kmax, int64_t(gr.slices) * OK);
+  if (n_tasks * kPackCluster < sms && kmax >= 1024 * kPackCluster)
+    p.pack_cluster = int(std::min(kmax / 512, (4 * sms + n_tasks - 1) / n_tasks));
   // output tiles and their K ranges.  One CTA runs per SM (its stages and TMEM fill one), so the K
   // slices of all tiles are cut into ranges of at most `cap` slices (at least kMinSplit), the largest
   // tiles split the most: cap starts at total / SMs and grows until the CTAs fit one wave (a second,
@@ -665,7 +699,6 @@ OzPlanHost build_oz_plan(const xgb_gemm_desc* descs, int n, bool allow_swap) {
     work += int64_t(gr.a_tiles) * gr.b_tiles * gr.slices;
     smax = std::max<int64_t>(smax, gr.slices);
   }
-  const int64_t sms = num_sms() > 0 ? num_sms() : 152;
   auto ctas = [&](int64_t cp) {
     int64_t c = 0;
     for (const auto& gr : p.groups) c += int64_t(gr.a_tiles) * gr.b_tiles * std::max<int64_t>(1, (gr.slices + cp - 1) / cp);
@@ -703,6 +736,14 @@ void launch_oz_pack(const xgb_gemm_desc* d_descs, const OzGroup* d_groups, const
                     int cluster, const double* A, const double* B, unsigned long long* rowmax, unsigned char* apack,
                     unsigned char* bpack, cudaStream_t s) {
   if (n_tasks <= 0) return;
+  if (cluster > kPackCluster) {
+    const unsigned grid = unsigned(n_tasks) * unsigned(cluster);
+    oz_clear_kernel<<<n_tasks, kPackRows, 0, s>>>(d_descs, d_groups, d_tasks, rowmax);
+    oz_pack_kernel<kMax><<<grid, 256, 0, s>>>(cluster, d_descs, d_groups, d_tasks, A, B, rowmax, apack, bpack);
+    oz_pack_kernel<kSlice><<<grid, 256, 0, s>>>(cluster, d_descs, d_groups, d_tasks, A, B, rowmax, apack, bpack);
+    count_launch(3);
+    return;
+  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = dim3(unsigned(n_tasks) * unsigned(cluster));
   cfg.blockDim = dim3(256);
@@ -712,7 +753,8 @@ void launch_oz_pack(const xgb_gemm_desc* d_descs, const OzGroup* d_groups, const
   at.val.clusterDim = {unsigned(cluster), 1, 1};
   cfg.attrs = &at;
   cfg.numAttrs = 1;
-  const cudaError_t e = cudaLaunchKernelEx(&cfg, oz_pack_kernel, d_descs, d_groups, d_tasks, A, B, rowmax, apack, bpack);
+  const cudaError_t e =
+      cudaLaunchKernelEx(&cfg, oz_pack_kernel<kWhole>, 0, d_descs, d_groups, d_tasks, A, B, rowmax, apack, bpack);
   if (e != cudaSuccess) throw std::runtime_error(std::string("slicing launch: ") + cudaGetErrorString(e));
   count_launch();
 }

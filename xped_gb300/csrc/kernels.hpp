@@ -202,7 +202,7 @@ struct OzPlanHost {
   std::vector<OzGroup> groups;
   std::vector<TcPackTask> tasks;            // tasks_a then tasks_b
   std::vector<TcPackTask> tasks_a, tasks_b;  // the op(A) and op(B) tiles alone
-  int pack_cluster = 1;                      // CTAs per task
+  int pack_cluster = 1;                      // CTAs per task: a cluster, or (more than 8) separate ones in two launches
   std::vector<GemmTile> tiles;               // k0 / k1 in K slices; slot >= 0: split-K partial
   std::vector<SplitReduce> red;              // fixed-order sums of the split tiles
   int32_t slots = 0;                         // partial tiles (workspace slots x 128 x 64 doubles)
@@ -212,7 +212,7 @@ struct OzPlanHost {
 // allow_swap: groups with few rows and many columns may be computed transposed (not for callers that
 // keep one operand's slices across products, whose roles must stay fixed)
 OzPlanHost build_oz_plan(const xgb_gemm_desc* descs, int n, bool allow_swap = true);
-// the row scales and slices of the given tiles (pack_cluster CTAs each)
+// the row scales and slices of the given tiles (cluster: the plan's pack_cluster)
 void launch_oz_pack(const xgb_gemm_desc* d_descs, const OzGroup* d_groups, const TcPackTask* d_tasks, int n_tasks,
                     int cluster, const double* A, const double* B, unsigned long long* rowmax, unsigned char* apack,
                     unsigned char* bpack, cudaStream_t s);
