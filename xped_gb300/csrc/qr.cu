@@ -97,12 +97,11 @@ __global__ void __launch_bounds__(kThreads)
     if (ss > 0.0) {
       beta = -copysign(sqrt(fma(alpha, alpha, ss)), alpha);
       t = (beta - alpha) / beta;
-      const int e = int((__double_as_longlong(beta) >> 52) & 0x7ff) - 1023;
-      if (abs(e) <= kUnscaled || e > 1023) {  // (1024: infinite or NaN)
-        sc = 1.0 / (alpha - beta);
-      } else {
-        const double p = __longlong_as_double((long long)(1023 - e) << 52);  // 2^-e: |e| stays below 540
-        sc = 1.0 / ((alpha - beta) * p);
+      sc = 1.0 / (alpha - beta);
+      const int e = ((__double2hiint(beta) >> 20) & 0x7ff) - 1023;
+      if (abs(e) > kUnscaled && e <= 1023) {  // (1024: infinite or NaN; else |e| stays below 540)
+        const double p = __hiloint2double((1023 - e) << 20, 0);  // 2^-e
+        sc *= __hiloint2double((1023 + e) << 20, 0);
         for (int i = j + 1 + lane; i < m; i += 32) x[i] *= p;
       }
     }
