@@ -1088,12 +1088,13 @@ def roofline(prof, steps, fp64_peak=None):
     # DRAM bytes per launch of the dominant kernel from one ncu capture (profiles/): the chosen
     # step's working sets are L2-resident
     traffic = {"gemm_tc": (7.025e9, "ncu capture, SU(2) Tensor<2,2> product (6.613 GB read + 0.412 GB written)"),
-               "gemm_f64tc": (68.27e6, "ncu one-pass capture of the 76 oz_gemm_kernel launches of one chosen U(1) D=6 "
-                                       "chi=128 step (bench.py --profile-step): 67.44 MB read + 0.83 MB written per "
+               "gemm_f64tc": (44.85e6, "ncu one-pass capture of the 146 oz_gemm_kernel launches of one chosen U(1) D=6 "
+                                       "chi=128 step (bench.py --profile-step): 44.52 MB read + 0.33 MB written per "
                                        "launch, average (the packed slices of the sector blocks)"),
                "gemm_f64": (14.10e6, "ncu one-pass capture of 348 consecutive gemm_simt_kernel launches of the "
-                                     "chosen U(1) D=6 chi=128 run (dram read + write per launch, average; the "
-                                     "operands are L2-resident after their first touch)")}
+                                     "chosen U(1) D=6 chi=128 run with 64-wide tiles (dram read + write per launch, "
+                                     "average); the 202 launches of a step with the present tiles: 7.15 MB read + "
+                                     "0.32 MB written (the operands are L2-resident after their first touch)")}
     out["traffic"] = traffic[dom][0] if dom in traffic else None
     if dom in traffic:
         out["traffic_source"] = traffic[dom][1]

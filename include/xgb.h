@@ -176,9 +176,11 @@ typedef struct xgb_svd_desc {
   int64_t vt_off;         /* V^T block k x n, ld = k */
 } xgb_svd_desc;
 
-/* Thin SVD of every block (FP64, one-sided Jacobi).  Singular vectors are
-   sign-normalised: the entry of largest magnitude of each u_j is positive.
-   `work` must hold xgb_svd_workspace_bytes(...) bytes. */
+/* Thin SVD of every block to FP64 accuracy (one-sided Jacobi).  Singular vectors are
+   sign-normalised: each u_j has a positive product with a fixed generic vector
+   (its entry of largest magnitude is positive where that product vanishes).
+   `work` must hold xgb_svd_workspace_bytes(...) bytes.  A block's U or Vt may
+   overlap the same block of A; work may not. */
 size_t xgb_svd_workspace_bytes(int n, const xgb_svd_desc* descs);
 int xgb_batched_svd(int n, const xgb_svd_desc* descs, const double* A, double* U, double* S, double* Vt, void* work,
                     void* stream);

@@ -266,8 +266,8 @@ void prof_end(int kind, cudaStream_t s, double work) {
 // Grouped GEMM on the CUDA cores: C_g = alpha*op(A_g)op(B_g) + beta*C_g.  One
 // CTA per TILE x TILE output tile of one group; 256 threads, each owning a
 // (TILE/16)^2 micro-tile.  T = double is the FP64 form, bound by GB300's narrow
-// FP64 pipe (two multiply-adds per clock and SM): it reaches 1.0 of that rate on
-// nine blocks 36 to 616 wide (1010 us; 1399 us when edge tiles were multiplied
+// FP64 pipe (two multiply-adds per clock and SM): it reaches 0.96 of that rate on
+// nine blocks 36 to 616 wide (1013 us; 1399 us when edge tiles were multiplied
 // whole and the tiles were 64 wide).  T = float is the FP32 form (operands
 // rounded to FP32 as they are staged, FP32 accumulation, alpha/beta and the
 // store in FP64).

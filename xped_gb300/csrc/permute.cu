@@ -18,7 +18,7 @@
 // Bound by HBM where the tensor is large, by the number of warp instructions for sums over short legs, and for the
 // smallest by the dependent loads of one batch (6.5 us under the profiler).  Measured, before -> now (U(1), 5 sectors,
 // legs up to 60, 2.8 GB moved): (0,2,1,3) 803 -> 540 us, (2,3,0,1) 3440 -> 438, (2,0,3,1) 1475 -> 499; SU(2) 2.6 M
-// elements: (2,0,3,1) with 270 sources of 158 sub-blocks 48 -> 35 us, (1,0,3,2) 27 -> 17.
+// elements: (2,0,3,1) with 270 sources of 158 sub-blocks 48 -> 41 us on inputs out of cache (35 repeated).
 #include <cuda_runtime.h>
 
 #include <algorithm>

@@ -5,7 +5,7 @@
 // shared memory (column j on CTA j mod P), one warp a trailing column.  The warp that holds column j + 1
 // applies reflector j to it first and forms reflector j + 1 at once, beside the other columns' update, so a
 // step is that warp's chain (a dot product, an update, a norm, a square root and a division: GB300's dependent
-// FP64 operations take ~64 cycles, a division ~430, a square root ~675), one cluster barrier and the copy of
+// FP64 operations take 65 cycles, a division 560, a square root 595), one cluster barrier and the copy of
 // the reflector to the other CTAs, ~10k cycles together with 300 rows.  Reflectors stay unscaled (v = x with
 // v_j = 1 / scal), which takes a pass over the column off that chain, unless x is far from one: then a power of two
 // brings it there, so that its products with columns of any other scale stay in range.  qr_form_q_kernel: column c of Q is

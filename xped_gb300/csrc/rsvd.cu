@@ -270,7 +270,7 @@ __device__ void chol_inv_body(const CholDesc& d, double* __restrict__ Gg, double
   //   rest of column j + 1 and scales it with the pivot's reciprocal (two-warp barrier in between),
   //   warps 2.. apply column j to the trailing columns j + 2 .. l - 1,
   // and one barrier ends the iteration.  The pivot chain - on GB300 a dependent FP64 operation takes
-  // ~64 cycles, sqrt ~675 and a division ~430, so the pivot is r = rsqrt(d) (~430) with L_jj = d r and
+  // 65 cycles, sqrt 595 and a division 560, so the pivot is r = rsqrt(d) (380) with L_jj = d r and
   // 1 / L_jj = r - runs beside the trailing update instead of between two barriers.  Every element sees
   // the same FMAs in the same order as in the unblocked column algorithm.
   const unsigned full_warp = 0xffffffffu;
@@ -401,7 +401,7 @@ __global__ void __launch_bounds__(1024) chol_inv_kernel(const CholDesc* __restri
 // pivot between its multiply-add and the scaling), applies column j to the columns behind and row j - 1 of X to the
 // rows behind while warp 1 finishes row j of X; one barrier ends it.  The other warps take a row each, lanes along its
 // columns of X and L: no index is divided.  What bounds it is the chain of warp 0 (on GB300 a dependent FP64 operation
-// takes ~64 cycles and rsqrt ~430, so about 700 cycles a column).  So the warps that share warp 0's quarter of the SM
+// takes 65 cycles and rsqrt 380, so about 700 cycles a column).  So the warps that share warp 0's quarter of the SM
 // stay out of the updates, and the pivot test is on the bits (a comparison is an FP64 instruction).
 // Measured (two blocks, widths about 16 / 32 / 48, factor and inverse): 63 / 85 / 158 us with one warp per block and a
 // second kernel for the inverse, 25 / 29 / 44 now.
