@@ -42,13 +42,22 @@ __device__ __forceinline__ double warp_sum(double v) {
   return v;
 }
 
-// CTAs of a block's cluster: one per 16 columns (a warp each), more when the columns need more shared memory; 0: no
-// cluster holds them (a CTA's columns and its copy of the current reflector; kQCols columns of Q).
-__host__ __device__ __forceinline__ int qr_ctas(int64_t m, int64_t n) {
+// Columns per CTA that a batch's blocks aim at (spread_of): blocks whose chain is at least `from` long, and the others.
+struct Spread {
+  int64_t from;
+  int wide, rest;
+};
+// a block's chain of reflectors, in rows
+__host__ __device__ __forceinline__ int64_t qr_chain(int64_t m, int64_t n) { return (m < n ? m : n) * (m + 256); }
+
+// CTAs of a block's cluster: one per 16 columns (a warp each) or fewer in crowded batches, more when the columns need more
+// shared memory; 0: no cluster holds them (a CTA's columns and its copy of the current reflector; kQCols columns of Q).
+__host__ __device__ __forceinline__ int qr_ctas(int64_t m, int64_t n, const Spread& sp) {
   if (8 * m * kQCols > kSmemLimit) return 0;
+  const int per = qr_chain(m, n) >= sp.from ? sp.wide : sp.rest;
   for (int p = 1; p <= kMostCtas; p *= 2) {
     const int64_t cols = (n + p - 1) / p;
-    if ((cols <= kWarps || p == kMostCtas) && 8 * m * (cols + 1) <= kSmemLimit) return p;
+    if ((cols <= per || p == kMostCtas) && 8 * m * (cols + 1) <= kSmemLimit) return p;
   }
   return 0;
 }
@@ -69,15 +78,70 @@ __device__ __forceinline__ double column_dot(const double* x, const double* y, i
   return warp_sum(a0 + a1);
 }
 
+// Reflector j (v below row j, tau t, scale sc) applied to N columns of a warp, `next` apart, with the bits of one column at a
+// time.  What a crowded SM waits for is FP64 instructions: N sums share the steps of a butterfly (six additions for four
+// columns instead of twenty), and the lanes of each column's part compute its factors at once.  300 blocks of 30 x 500
+// 4.03 ms one column at a time, 2.62 so; one of 20 x 4000 1.21 and 0.59.
+template <int N>
+__device__ __forceinline__ void apply_reflector(const double* v, double* c, int64_t next, int j, int m, double t, double sc,
+                                                int lane) {
+  double a0[N] = {}, a1[N] = {};
+  int i = j + 1 + lane;
+  for (; i + 32 < m; i += 64) {
+    const double x = v[i], y = v[i + 32];
+#pragma unroll
+    for (int k = 0; k < N; ++k) {
+      a0[k] = fma(x, c[i + k * next], a0[k]);
+      a1[k] = fma(y, c[i + 32 + k * next], a1[k]);
+    }
+  }
+  if (i < m) {
+    const double x = v[i];
+#pragma unroll
+    for (int k = 0; k < N; ++k) a0[k] = fma(x, c[i + k * next], a0[k]);
+  }
+#pragma unroll
+  for (int k = 0; k < N; ++k) a0[k] += a1[k];
+  int o = 16;
+#pragma unroll
+  for (int half = N / 2; half > 0; half /= 2, o /= 2) {  // lanes with bit o keep the upper half of the columns
+    const bool up = lane & o;
+#pragma unroll
+    for (int k = 0; k < half; ++k) {
+      const double keep = up ? a0[k + half] : a0[k], send = up ? a0[k] : a0[k + half];
+      a0[k] = keep + __shfl_xor_sync(0xffffffffu, send, o);
+    }
+  }
+#pragma unroll
+  for (; o > 0; o /= 2) a0[0] += __shfl_xor_sync(0xffffffffu, a0[0], o);
+  constexpr int kPart = 32 / N;  // lanes of a column
+  double* cj = c + j + (lane / kPart) * next;
+  const double w = t * (*cj + sc * a0[0]), ws = -w * sc;
+  __syncwarp();
+  if (lane % kPart == 0) *cj -= w;
+  double f[N];
+#pragma unroll
+  for (int k = 0; k < N; ++k) f[k] = __shfl_sync(0xffffffffu, ws, k * kPart);
+#pragma unroll 4
+  for (i = j + 1 + lane; i < m; i += 32) {
+    const double x = v[i];
+#pragma unroll
+    for (int k = 0; k < N; ++k) c[i + k * next] = fma(f[k], x, c[i + k * next]);
+  }
+  __syncwarp();
+}
+
+// kGroups: some CTA holds more columns than warps (the branch alone costs a step of the others 2 %)
+template <bool kGroups>
 __global__ void __launch_bounds__(kThreads)
     qr_factor_kernel(const xgb_qr_desc* __restrict__ descs, const int64_t* __restrict__ work_off,
-                     const double* __restrict__ A, double* __restrict__ R, double* __restrict__ work) {
+                     const double* __restrict__ A, double* __restrict__ R, double* __restrict__ work, Spread sp) {
   extern __shared__ __align__(16) double qr_sm[];
   __shared__ double tau_s[2], scal_s[2];  // of the reflector that this CTA formed last, by parity of its column
   cg::cluster_group cl = cg::this_cluster();
   const int ctas = int(cl.num_blocks()), block = int(blockIdx.x) / ctas, rank = int(cl.block_rank());
   const xgb_qr_desc d = descs[block];
-  const int P = qr_ctas(d.m, d.n);
+  const int P = qr_ctas(d.m, d.n, sp);
   if (P == 0 || rank >= P) return;  // (a cluster barrier waits for the threads that have not exited)
   const int m = int(d.m), n = int(d.n), kk = m < n ? m : n;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -138,6 +202,16 @@ __global__ void __launch_bounds__(kThreads)
     const int lowest = j + 1 <= rank ? 0 : (j + 1 - rank + P - 1) / P;
     for (int u = lowest + warp; u < own; u += kWarps) {
       double* c = cols + u * m;
+      if (kGroups && t != 0.0 && u + kWarps < own && rank + u * P != j + 1) {  // four or two columns of this warp
+        if (u + 3 * kWarps < own) {
+          apply_reflector<4>(v, c, int64_t(kWarps) * m, j, m, t, sc, lane);
+          u += 3 * kWarps;
+        } else {
+          apply_reflector<2>(v, c, int64_t(kWarps) * m, j, m, t, sc, lane);
+          u += kWarps;
+        }
+        continue;
+      }
       if (t != 0.0) {
         const double w = t * (c[j] + sc * column_dot(v, c, j + 1, m, lane)), ws = -w * sc;
         __syncwarp();
@@ -163,10 +237,10 @@ __global__ void __launch_bounds__(kThreads)
 
 __global__ void __launch_bounds__(32 * kQCols)
     qr_form_q_kernel(const xgb_qr_desc* __restrict__ descs, const int64_t* __restrict__ work_off,
-                     double* __restrict__ Q, const double* __restrict__ work) {
+                     double* __restrict__ Q, const double* __restrict__ work, Spread sp) {
   extern __shared__ __align__(16) double qr_sm[];
   const xgb_qr_desc d = descs[blockIdx.y];
-  if (qr_ctas(d.m, d.n) == 0) return;
+  if (qr_ctas(d.m, d.n, sp) == 0) return;
   const int m = int(d.m), kk = int(d.m < d.n ? d.m : d.n);
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t c = d.q_cols - 1 - (int64_t(blockIdx.x) * kQCols + warp);  // the longest products first
@@ -199,9 +273,10 @@ __global__ void __launch_bounds__(32 * kQCols)
 // One CTA per block, the columns in global memory: blocks that no cluster's shared memory holds.
 __global__ void __launch_bounds__(256) qr_kernel(const xgb_qr_desc* __restrict__ descs, const int64_t* __restrict__ work_off,
                                                  const double* __restrict__ A, double* __restrict__ Q,
-                                                 double* __restrict__ R, double* __restrict__ work) {
+                                                 double* __restrict__ R, double* __restrict__ work,
+                                                 Spread sp) {
   const xgb_qr_desc d = descs[blockIdx.x];
-  if (qr_ctas(d.m, d.n) != 0) return;
+  if (qr_ctas(d.m, d.n, sp) != 0) return;
   const int64_t m = d.m, n = d.n, kk = m < n ? m : n;
   double* W = work + work_off[blockIdx.x];  // m x n working copy (Householder vectors below diagonal)
   double* tau = W + m * n;                  // kk
@@ -279,6 +354,29 @@ __global__ void __launch_bounds__(256) qr_kernel(const xgb_qr_desc* __restrict__
   }
 }
 
+// 16 columns a CTA keep a block's chain shortest; where the clusters of a batch are more CTAs than the SMs take at once they
+// only share the FP64 pipes, and pay for their barriers.  So from 5/4 CTAs per SM on, blocks take fewer: first those with
+// less than half of the longest chain, then all.  Measured (us, 16 / 32 / 64 columns): 38 of 60 x 60 409 / 429 / 465, 75 of
+// them 698 / 509 / 544, 300 1951 / 1455 / 1169 (one CTA per block in global memory 1346); 20 of 120 x 120 (160 CTAs) 908
+// / 955 / 1154, 75 2560 / 2375 / 1767; 300 of 300 x 60 3024 / 2360 / 2290.
+Spread spread_of(const xgb_qr_desc* d, int n) {
+  int64_t longest = 0, cols = kWarps;
+  for (int i = 0; i < n; ++i) {
+    longest = std::max(longest, qr_chain(d[i].m, d[i].n));
+    cols = std::max(cols, std::min<int64_t>(d[i].n, INT32_MAX / 2));
+  }
+  Spread sp{(longest + 1) / 2, kWarps, kWarps};
+  auto crowded = [&](bool all) {
+    int64_t room = 5 * int64_t(num_sms() > 0 ? num_sms() : 152) / 4;
+    for (int i = 0; i < n && room >= 0; ++i)
+      if (all || qr_chain(d[i].m, d[i].n) >= sp.from) room -= qr_ctas(d[i].m, d[i].n, sp);
+    return room < 0;
+  };
+  while (sp.rest < cols && crowded(true)) sp.rest *= 2;
+  while (sp.wide < cols && crowded(false)) sp.wide *= 2;
+  return sp;
+}
+
 }  // namespace
 
 size_t qr_work_elems(int64_t m, int64_t n) { return size_t(m * n + std::min(m, n) + m * m); }
@@ -288,20 +386,23 @@ void launch_qr(const xgb_qr_desc* d_descs, const xgb_qr_desc* h_descs, const int
   if (n <= 0) return;
   static PerDevice attr;
   attr.once([] {
-    cudaFuncSetAttribute(qr_factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemLimit));
+    cudaFuncSetAttribute(qr_factor_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemLimit));
+    cudaFuncSetAttribute(qr_factor_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemLimit));
     cudaFuncSetAttribute(qr_form_q_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemLimit));
   });
+  const Spread sp = spread_of(h_descs, n);
   int ctas = 0;
   int64_t bytes = 0, q_bytes = 0, q_cols = 0;
-  bool large = false;
+  bool large = false, groups = false;
   for (int i = 0; i < n; ++i) {
     const xgb_qr_desc& d = h_descs[i];
-    const int p = qr_ctas(d.m, d.n);
+    const int p = qr_ctas(d.m, d.n, sp);
     if (p == 0) {
       large = true;
       continue;
     }
     ctas = std::max(ctas, p);
+    groups = groups || d.n > int64_t(p) * kWarps;
     bytes = std::max(bytes, 8 * d.m * ((d.n + p - 1) / p + 1));
     q_bytes = std::max(q_bytes, 8 * d.m * kQCols);
     q_cols = std::max(q_cols, d.q_cols);
@@ -318,19 +419,20 @@ void launch_qr(const xgb_qr_desc* d_descs, const xgb_qr_desc* h_descs, const int
     a[0].val.clusterDim.y = a[0].val.clusterDim.z = 1;
     cfg.attrs = a;
     cfg.numAttrs = 1;
-    const cudaError_t e = cudaLaunchKernelEx(&cfg, qr_factor_kernel, d_descs, d_work_off, A, R, work);
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, groups ? qr_factor_kernel<true> : qr_factor_kernel<false>, d_descs,
+                                             d_work_off, A, R, work, sp);
     if (e != cudaSuccess) throw std::runtime_error(std::string("qr launch: ") + cudaGetErrorString(e));
     count_launch();
     if (q_cols > 0) {
       in_grid_rows(n, [&](int first, unsigned count) {
         qr_form_q_kernel<<<dim3(unsigned((q_cols + kQCols - 1) / kQCols), count), 32 * kQCols, size_t(q_bytes), s>>>(
-            d_descs + first, d_work_off + first, Q, work);
+            d_descs + first, d_work_off + first, Q, work, sp);
         count_launch();
       });
     }
   }
   if (large) {
-    qr_kernel<<<n, 256, 0, s>>>(d_descs, d_work_off, A, Q, R, work);
+    qr_kernel<<<n, 256, 0, s>>>(d_descs, d_work_off, A, Q, R, work, sp);
     count_launch();
   }
 }
