@@ -62,3 +62,20 @@ def test_crowded_batches(name):
             seen[m, n] += 1
             own_q, own_r = batched_qr([x])[0]
             assert np.array_equal(q, own_q) and np.array_equal(r, own_r), (m, n)
+
+
+@pytest.mark.parametrize("shapes", [[(1, 1)], [(8, 4)] * 9, [(4, 4), (9, 3), (2, 4), (1, 4), (2, 1)],
+                                    [(3128, 4), (4693, 1), (3, 2)], [(3129, 4)], [(4694, 1)]], ids=str)
+def test_batches_of_one_launch(shapes):
+    """Q formed beside R (blocks of at most four columns that fit) or, in a batch with a wider block, by its own kernel."""
+    rng = np.random.default_rng(len(shapes))
+    mats = [rng.standard_normal(s) for s in shapes]
+    if len(mats) > 2:
+        mats[1][:, 0] = 0.0
+    wider = rng.standard_normal((20, 17))
+    for x, (q, r), (q2, r2) in zip(mats, batched_qr(mats), batched_qr(mats + [wider])):
+        m, n = x.shape
+        k, tol = min(m, n), 50 * max(m, n) * EPS
+        assert np.abs(q.T @ q - np.eye(k)).max() <= tol, (m, n)
+        assert np.linalg.norm(q @ r - x) <= tol * np.linalg.norm(x), (m, n)
+        assert np.array_equal(q, q2) and np.array_equal(r, r2), (m, n)

@@ -131,11 +131,35 @@ __device__ __forceinline__ void apply_reflector(const double* v, double* c, int6
   __syncwarp();
 }
 
-// kGroups: some CTA holds more columns than warps (the branch alone costs a step of the others 2 %)
+// Column c of Q = H_0 .. H_c e_c by one warp, in shared memory (y), from the reflectors W (m rows each).
+__device__ __forceinline__ void form_q(double* q, int64_t c, int m, int kk, const double* W, const double* tau,
+                                       const double* scal, double* y, int lane) {
+  if (c >= kk) {
+    for (int i = lane; i < m; i += 32) q[i] = 0.0;
+    return;
+  }
+  for (int i = lane; i < m; i += 32) y[i] = i == c ? 1.0 : 0.0;
+  __syncwarp();
+  for (int k = int(c); k >= 0; --k) {
+    const double t = tau[k], sc = scal[k];
+    if (t == 0.0) continue;
+    const double* v = W + int64_t(k) * m;
+    const double w = t * (y[k] + sc * column_dot(v, y, k + 1, m, lane)), ws = -w * sc;
+    __syncwarp();
+    if (lane == 0) y[k] -= w;
+#pragma unroll 4
+    for (int i = k + 1 + lane; i < m; i += 32) y[i] = fma(ws, v[i], y[i]);
+    __syncwarp();
+  }
+  for (int i = lane; i < m; i += 32) q[i] = y[i];
+}
+
+// kGroups: some CTA holds more columns than warps (the branch alone costs a step of the others 2 %).  whole: Q as well.
 template <bool kGroups>
 __global__ void __launch_bounds__(kThreads)
     qr_factor_kernel(const xgb_qr_desc* __restrict__ descs, const int64_t* __restrict__ work_off,
-                     const double* __restrict__ A, double* __restrict__ R, double* __restrict__ work, Spread sp) {
+                     const double* __restrict__ A, double* __restrict__ Q, double* __restrict__ R,
+                     double* __restrict__ work, Spread sp, bool whole) {
   extern __shared__ __align__(16) double qr_sm[];
   __shared__ double tau_s[2], scal_s[2];  // of the reflector that this CTA formed last, by parity of its column
   cg::cluster_group cl = cg::this_cluster();
@@ -230,9 +254,11 @@ __global__ void __launch_bounds__(kThreads)
     const int c = rank + u * P;
     for (int64_t i = lane; i < d.r_rows; i += 32)
       R[d.r_off + i + int64_t(c) * d.r_rows] = i < kk && i <= c ? cols[u * m + i] : 0.0;
-    if (c < kk)
+    if (c < kk && !whole)
       for (int i = c + 1 + lane; i < m; i += 32) W[i + int64_t(c) * m] = cols[u * m + i];
   }
+  if (whole && warp < d.q_cols)  // (P = 1)
+    form_q(Q + d.q_off + int64_t(warp) * m, warp, m, kk, cols, tau, scal, cols + (n + warp) * m, lane);
 }
 
 __global__ void __launch_bounds__(32 * kQCols)
@@ -245,29 +271,9 @@ __global__ void __launch_bounds__(32 * kQCols)
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t c = d.q_cols - 1 - (int64_t(blockIdx.x) * kQCols + warp);  // the longest products first
   if (c < 0) return;
-  double* q = Q + d.q_off + c * m;
-  if (c >= kk) {
-    for (int i = lane; i < m; i += 32) q[i] = 0.0;
-    return;
-  }
   const double* W = work + work_off[blockIdx.y];
   const double* tau = W + d.m * d.n;
-  const double* scal = tau + kk;
-  double* y = qr_sm + warp * m;
-  for (int i = lane; i < m; i += 32) y[i] = i == c ? 1.0 : 0.0;
-  __syncwarp();
-  for (int k = int(c); k >= 0; --k) {
-    const double t = tau[k], sc = scal[k];
-    if (t == 0.0) continue;
-    const double* v = W + int64_t(k) * m;
-    const double w = t * (y[k] + sc * column_dot(v, y, k + 1, m, lane)), ws = -w * sc;
-    __syncwarp();
-    if (lane == 0) y[k] -= w;
-#pragma unroll 4
-    for (int i = k + 1 + lane; i < m; i += 32) y[i] = fma(ws, v[i], y[i]);
-    __syncwarp();
-  }
-  for (int i = lane; i < m; i += 32) q[i] = y[i];
+  form_q(Q + d.q_off + c * m, c, m, kk, W, tau, tau + kk, qr_sm + warp * m, lane);
 }
 
 // One CTA per block, the columns in global memory: blocks that no cluster's shared memory holds.
@@ -354,6 +360,12 @@ __global__ void __launch_bounds__(256) qr_kernel(const xgb_qr_desc* __restrict__
   }
 }
 
+// Blocks of so few columns that their CTA forms Q as fast as qr_form_q_kernel does (one warp per SM sub-partition): a batch of
+// them is one launch (one block of 1 x 1: 22.8 -> 19.1 us).
+bool whole_block(const xgb_qr_desc& d) {
+  return d.n <= kQCols && d.q_cols <= kQCols && 8 * d.m * (d.n + 1 + kQCols) <= kSmemLimit;
+}
+
 // 16 columns a CTA keep a block's chain shortest; where the clusters of a batch are more CTAs than the SMs take at once they
 // only share the FP64 pipes, and pay for their barriers.  So from 5/4 CTAs per SM on, blocks take fewer: first those with
 // less than half of the longest chain, then all.  Measured (us, 16 / 32 / 64 columns): 38 of 60 x 60 409 / 429 / 465, 75 of
@@ -392,8 +404,8 @@ void launch_qr(const xgb_qr_desc* d_descs, const xgb_qr_desc* h_descs, const int
   });
   const Spread sp = spread_of(h_descs, n);
   int ctas = 0;
-  int64_t bytes = 0, q_bytes = 0, q_cols = 0;
-  bool large = false, groups = false;
+  int64_t bytes = 0, whole_bytes = 0, q_bytes = 0, q_cols = 0;
+  bool large = false, groups = false, whole = true;
   for (int i = 0; i < n; ++i) {
     const xgb_qr_desc& d = h_descs[i];
     const int p = qr_ctas(d.m, d.n, sp);
@@ -402,12 +414,15 @@ void launch_qr(const xgb_qr_desc* d_descs, const xgb_qr_desc* h_descs, const int
       continue;
     }
     ctas = std::max(ctas, p);
+    whole = whole && whole_block(d);
+    whole_bytes = std::max(whole_bytes, 8 * d.m * (d.n + 1 + kQCols));
     groups = groups || d.n > int64_t(p) * kWarps;
     bytes = std::max(bytes, 8 * d.m * ((d.n + p - 1) / p + 1));
     q_bytes = std::max(q_bytes, 8 * d.m * kQCols);
     q_cols = std::max(q_cols, d.q_cols);
   }
   if (ctas) {
+    if (whole) bytes = whole_bytes;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(unsigned(n * ctas));
     cfg.blockDim = dim3(kThreads);
@@ -420,10 +435,10 @@ void launch_qr(const xgb_qr_desc* d_descs, const xgb_qr_desc* h_descs, const int
     cfg.attrs = a;
     cfg.numAttrs = 1;
     const cudaError_t e = cudaLaunchKernelEx(&cfg, groups ? qr_factor_kernel<true> : qr_factor_kernel<false>, d_descs,
-                                             d_work_off, A, R, work, sp);
+                                             d_work_off, A, Q, R, work, sp, whole);
     if (e != cudaSuccess) throw std::runtime_error(std::string("qr launch: ") + cudaGetErrorString(e));
     count_launch();
-    if (q_cols > 0) {
+    if (q_cols > 0 && !whole) {
       in_grid_rows(n, [&](int first, unsigned count) {
         qr_form_q_kernel<<<dim3(unsigned((q_cols + kQCols - 1) / kQCols), count), 32 * kQCols, size_t(q_bytes), s>>>(
             d_descs + first, d_work_off + first, Q, work, sp);
