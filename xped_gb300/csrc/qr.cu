@@ -1,8 +1,9 @@
 // Batched Householder QR in FP64 with LAPACK's dlarfg sign convention (beta = -sign(alpha) ||x||), so Q
 // and R agree with dgeqrf / dorgqr (Tensor::tQR, src/Core/Tensor.cpp:757-780).
 //
-// Two launches per batch.  qr_factor_kernel: one cluster per block with the block's columns in its CTAs'
-// shared memory (column j on CTA j mod P), one warp a trailing column.  The warp that holds column j + 1
+// Two launches per batch (one where no block has more than four columns).  qr_factor_kernel: one cluster per block with the
+// block's columns in its CTAs' shared memory (column j on CTA j mod P, fewer CTAs in crowded batches), a warp one to four
+// trailing columns at a time.  The warp that holds column j + 1
 // applies reflector j to it first and forms reflector j + 1 at once, beside the other columns' update, so a
 // step is that warp's chain (a dot product, an update, a norm, a square root and a division: GB300's dependent
 // FP64 operations take 65 cycles, a division 560, a square root 595), one cluster barrier and the copy of
